@@ -568,6 +568,14 @@ int poyd_to_bf16(const float *x, void *y, int64_t n, void *stream);
 int poyd_mlp_forward(const void *X, int32_t M, const void *W1t, const float *b1,
                      const void *W2t, const float *b2, const void *W3t, const float *b3,
                      const void *w4, const float *b4, float *y, void *stream);
+/* The same with the weights as the parameters hold them ([in][out] bf16,
+ * 4-byte aligned); X is bf16, or fp32 (rounded to bf16) when x_fp32, 16-byte
+ * aligned.  H1, H2 [M][256] and H3 [M][128] (bf16, 16-byte aligned), where
+ * given, receive the hidden layers' activations for poyd_mlp_backward. */
+int poyd_mlp_forward_rows(const void *X, int32_t x_fp32, int32_t M, const void *W1,
+                          const float *b1, const void *W2, const float *b2, const void *W3,
+                          const float *b3, const void *w4, const float *b4, void *H1, void *H2,
+                          void *H3, float *y, void *stream);
 
 /* ---------------------------------------------------------------------
  * Measurement helpers (no counterpart in the reference, which has no

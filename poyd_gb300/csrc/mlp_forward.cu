@@ -1,0 +1,429 @@
+// Forward pass of the 32-256-256-128-1 join-proposal MLP, fused into one
+// launch on the tcgen05 tensor cores: inference over a pass's candidates and,
+// with the activations written out, the training forward.
+//
+// A CTA keeps all three weight matrices in shared memory (208 KB, staged once)
+// and runs 128-row tiles through the layers.  Per tile:
+//   * layer 1: A = the tile's bf16 inputs in shared memory, D in TMEM columns
+//     0-255 (region 0);
+//   * the epilogue reads a row's sums with tcgen05.ld (one thread per row and
+//     half of the columns), adds the bias, applies ReLU, rounds to bf16 and
+//     writes the packed values back with tcgen05.st over columns it has read:
+//     the next layer's A operand never leaves TMEM, which is what leaves the
+//     shared memory to the weights;
+//   * layer 2: A from region 0, D in region 1; layer 3: A from region 1, D in
+//     region 0; then the 128 -> 1 head from registers.
+// Measured: 984,102 rows from fp32 in 0.29 ms (0.72 PFLOP/s) where the
+// mma.sync kernel with its weights in L2 took 1.21 ms, the input's conversion
+// and the weights' transposes 33 us more.  What bounds it: the chain of a
+// tile's products and epilogues, which share the one set of TMEM columns.
+//
+// Every layer accumulates k in ascending chunks of 16 from zero and the head
+// sums as k_head_forward does (lane-strided, then the xor butterfly's tree).
+//
+// B and the layer 1 A operand are K-major without swizzle: 8 x 16-byte core
+// matrices, K-adjacent ones 128 bytes apart, 8-row groups 128 * K / 8 + 16
+// bytes apart (the 16 bytes spread the staging stores over the banks).
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <cstdint>
+#include "poyd_internal.h"
+
+namespace poyd {
+namespace {
+
+constexpr int kMRows = 128, kMThreads = 256;
+constexpr int kMIn = 32, kMH1 = 256, kMH2 = 256, kMH3 = 128;
+__host__ __device__ constexpr int m_sbo(int k) { return k / 8 * 128 + 16; }
+constexpr uint32_t kMW1 = 0;
+constexpr uint32_t kMW2 = kMW1 + kMH1 / 8 * m_sbo(kMIn);
+constexpr uint32_t kMW3 = kMW2 + kMH2 / 8 * m_sbo(kMH1);
+constexpr uint32_t kMX = kMW3 + kMH3 / 8 * m_sbo(kMH2);
+constexpr uint32_t kMBias = kMX + kMRows / 8 * m_sbo(kMIn);  // b1, b2, b3, w4 (fp32)
+constexpr uint32_t kMBar = kMBias + 4 * (kMH1 + kMH2 + 2 * kMH3);
+constexpr uint32_t kMSmem = kMBar + 32 + 128;  // + alignment slack
+static_assert(kMSmem <= 227 * 1024, "weights, inputs and biases fit one CTA");
+constexpr int kMWaitMax = 1 << 22;  // mbarrier polls before a wait gives up
+
+struct MlpFwdArgs {
+  const void *X;
+  int x32;      // X is fp32 (converted here), else bf16
+  int trans;    // weights are [out][in] rows, else [in][out]
+  int M;
+  const uint16_t *W[3];
+  const float *b[3];
+  const uint16_t *w4;
+  const float *b4;
+  uint16_t *H[3];  // activations [M][256], [M][256], [M][128], or null
+  float *y;
+};
+
+__device__ __forceinline__ uint64_t m_desc(uint32_t addr, uint32_t sbo) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(128 >> 4) << 16 |
+         (uint64_t)(sbo >> 4) << 32 | 1ull << 46;
+}
+// kind::f16: fp32 accumulator, bf16 A and B, both K-major
+__host__ __device__ constexpr uint32_t m_idesc(int n) {
+  return 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(n >> 3) << 17 | (uint32_t)(kMRows >> 4) << 24;
+}
+
+__device__ __forceinline__ void m_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t acc) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void m_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t acc) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d),
+      "r"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void m_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool m_wait(uint32_t bar, uint32_t parity) {
+  for (int i = 0; i < kMWaitMax; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void m_ld32(uint32_t (&r)[32], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void m_st16(uint32_t addr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void m_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void m_after() {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t m_relu2(float lo, float hi) {
+  lo = lo > 0.f ? lo : 0.f;
+  hi = hi > 0.f ? hi : 0.f;
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+
+// Stages a K x N weight matrix as the K-major B operand at `dst`.
+__device__ __forceinline__ void m_stage_w(uint8_t *dst, const uint16_t *W, int K, int N,
+                                          int trans) {
+  const int sbo = m_sbo(K);
+  const bool al = ((uintptr_t)W & 15) == 0;
+  if (trans) {  // [n][k]: a core matrix row is 16 contiguous bytes
+    for (int e = threadIdx.x; e < N * (K / 8); e += kMThreads) {
+      const int n = (e & 7) | e / K << 3, kc = e / 8 % (K / 8);
+      const uint32_t *s = reinterpret_cast<const uint32_t *>(W + (int64_t)n * K + kc * 8);
+      const uint4 v = al ? *reinterpret_cast<const uint4 *>(s) : make_uint4(s[0], s[1], s[2], s[3]);
+      *reinterpret_cast<uint4 *>(dst + (n >> 3) * sbo + kc * 128 + (n & 7) * 16) = v;
+    }
+    return;
+  }
+  // [k][n]: two k rows of eight columns per thread, paired into words
+  const int n8s = N / 8;
+  for (int e = threadIdx.x; e < K / 2 * n8s; e += kMThreads) {
+    const int lo = e & 31, hi = e >> 5;
+    const int n8 = hi % (n8s / 8) * 8 + (lo >> 2), k = 2 * (hi / (n8s / 8) * 4 + (lo & 3));
+    const uint16_t *s0 = W + (int64_t)k * N + n8 * 8, *s1 = s0 + N;
+    uint32_t a[4], b[4];
+    if (al) {
+      const uint4 u = *reinterpret_cast<const uint4 *>(s0), v = *reinterpret_cast<const uint4 *>(s1);
+      a[0] = u.x, a[1] = u.y, a[2] = u.z, a[3] = u.w;
+      b[0] = v.x, b[1] = v.y, b[2] = v.z, b[3] = v.w;
+    } else {
+      for (int q = 0; q < 4; ++q) {
+        a[q] = s0[2 * q] | (uint32_t)s0[2 * q + 1] << 16;
+        b[q] = s1[2 * q] | (uint32_t)s1[2 * q + 1] << 16;
+      }
+    }
+    uint8_t *o = dst + n8 * sbo + (k >> 3) * 128 + (k & 7) * 2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      *reinterpret_cast<uint32_t *>(o + (2 * q) * 16) = __byte_perm(a[q], b[q], 0x5410);
+      *reinterpret_cast<uint32_t *>(o + (2 * q + 1) * 16) = __byte_perm(a[q], b[q], 0x7632);
+    }
+  }
+}
+
+// Eight inputs (one core matrix row) of row m, zero past M.
+__device__ __forceinline__ uint4 m_load_x(const MlpFwdArgs &A, int64_t m, int kc) {
+  if (m >= A.M) return make_uint4(0, 0, 0, 0);
+  if (!A.x32) return *reinterpret_cast<const uint4 *>((const uint16_t *)A.X + m * kMIn + kc * 8);
+  const float4 *p = reinterpret_cast<const float4 *>((const float *)A.X + m * kMIn + kc * 8);
+  const float4 u = p[0], v = p[1];
+  uint4 r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.x) : "f"(u.y), "f"(u.x));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.y) : "f"(u.w), "f"(u.z));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.z) : "f"(v.y), "f"(v.x));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.w) : "f"(v.w), "f"(v.z));
+  return r;
+}
+
+// One hidden layer's epilogue for this thread's row and half of 256 columns:
+// the sums at `reg` become the next layer's packed A operand in place (and,
+// when H is given, row-major activations).
+__device__ __forceinline__ void m_epilogue(uint32_t reg, const float *bias, uint16_t *h) {
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    uint32_t r[32], p[16];
+    m_ld32(r, reg + 32 * c);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const float2 bb = *reinterpret_cast<const float2 *>(bias + 32 * c + 2 * q);
+      p[q] = m_relu2(__uint_as_float(r[2 * q]) + bb.x, __uint_as_float(r[2 * q + 1]) + bb.y);
+    }
+    m_st16(reg + 16 * c, p);
+    if (h) {
+      uint4 *o = reinterpret_cast<uint4 *>(h + 32 * c);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[q] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+    }
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_constant__ MlpFwdArgs A) {
+  extern __shared__ unsigned char mlp_raw[];
+  uint8_t *sm = mlp_raw + ((128 - ((uint32_t)__cvta_generic_to_shared(mlp_raw) & 127)) & 127);
+  const uint32_t sb = (uint32_t)__cvta_generic_to_shared(sm);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int half = warp >> 2;                       // columns 128 half ..
+  const int row = (warp & 3) * 32 + lane;           // this thread's TMEM lane
+  float *bias = reinterpret_cast<float *>(sm + kMBias);
+  const uint32_t bar = sb + kMBar;
+  uint32_t *slot = reinterpret_cast<uint32_t *>(sm + kMBar + 16);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sb + kMBar + 16)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  m_stage_w(sm + kMW1, A.W[0], kMIn, kMH1, A.trans);
+  m_stage_w(sm + kMW2, A.W[1], kMH1, kMH2, A.trans);
+  m_stage_w(sm + kMW3, A.W[2], kMH2, kMH3, A.trans);
+  for (int i = tid; i < kMH1 + kMH2 + 2 * kMH3; i += kMThreads)
+    bias[i] = i < 256 ? A.b[0][i] : i < 512 ? A.b[1][i - 256] : i < 640 ? A.b[2][i - 512]
+              : __uint_as_float((uint32_t)A.w4[i - 640] << 16);
+  const int tiles = (A.M + kMRows - 1) / kMRows;
+  // a thread's two core matrix rows of an input tile
+  auto put_x = [&](int e, uint4 v) {
+    const int r = (e & 7) | e >> 5 << 3, kc = e >> 3 & 3;
+    *reinterpret_cast<uint4 *>(sm + kMX + (r >> 3) * m_sbo(kMIn) + kc * 128 + (r & 7) * 16) = v;
+  };
+  auto get_x = [&](int t, int e) {
+    return m_load_x(A, (int64_t)t * kMRows + ((e & 7) | e >> 5 << 3), e >> 3 & 3);
+  };
+  int t = blockIdx.x;
+  if (t < tiles) {
+    put_x(tid, get_x(t, tid));
+    put_x(tid + kMThreads, get_x(t, tid + kMThreads));
+  }
+  m_before();
+  __syncthreads();
+  m_after();
+  const uint32_t tm = *slot;
+  const uint32_t lane_base = (uint32_t)(warp & 3) << 21;  // TMEM lane 32 (warp % 4) in bits 16-
+  const uint32_t mine = tm + lane_base + 128 * half;
+  uint32_t parity = 0;
+  bool dead = false;
+  // all threads: wait for the committed products (bounded)
+  auto wait_mma = [&]() {
+    const bool ok = m_wait(bar, parity);
+    parity ^= 1;
+    dead = __syncthreads_or(!ok);
+    m_after();
+  };
+  for (; t < tiles && !dead; t += gridDim.x) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // staged operands
+    m_before();
+    __syncthreads();
+    if (tid == 0) {
+      m_after();
+      for (int k = 0; k < kMIn / 16; ++k)
+        m_mma_ss(tm, m_desc(sb + kMX + 256 * k, m_sbo(kMIn)), m_desc(sb + kMW1 + 256 * k, m_sbo(kMIn)),
+                 m_idesc(kMH1), k);
+      m_commit(bar);
+    }
+    // the next tile's inputs travel while this one computes
+    const int tn = t + gridDim.x;
+    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+    if (tn < tiles) {
+      x0 = get_x(tn, tid);
+      x1 = get_x(tn, tid + kMThreads);
+    }
+    wait_mma();
+    if (dead) break;
+    put_x(tid, x0);
+    put_x(tid + kMThreads, x1);
+    const int64_t m = (int64_t)t * kMRows + row;
+    const bool in = m < A.M;
+    m_epilogue(mine, bias + 128 * half, in && A.H[0] ? A.H[0] + m * kMH1 + 128 * half : nullptr);
+    m_before();
+    __syncthreads();
+    if (tid == 0) {
+      m_after();
+      for (int k = 0; k < kMH1 / 16; ++k)  // A: columns 8 k of each half's 64
+        m_mma_ts(tm + 256, tm + 8 * k + (k >= 8 ? 64 : 0), m_desc(sb + kMW2 + 256 * k, m_sbo(kMH1)),
+                 m_idesc(kMH2), k);
+      m_commit(bar);
+    }
+    wait_mma();
+    if (dead) break;
+    m_epilogue(mine + 256, bias + 256 + 128 * half,
+               in && A.H[1] ? A.H[1] + m * kMH2 + 128 * half : nullptr);
+    m_before();
+    __syncthreads();
+    if (tid == 0) {
+      m_after();
+      for (int k = 0; k < kMH2 / 16; ++k)
+        m_mma_ts(tm, tm + 256 + 8 * k + (k >= 8 ? 64 : 0),
+                 m_desc(sb + kMW3 + 256 * k, m_sbo(kMH2)), m_idesc(kMH3), k);
+      m_commit(bar);
+    }
+    wait_mma();
+    if (dead) break;
+    if (half == 0) {
+      // the third layer's epilogue and the head: s[l] sums columns l, l + 32,
+      // l + 64, l + 96, then the butterfly's tree over l
+      float s[32];
+#pragma unroll
+      for (int l = 0; l < 32; ++l) s[l] = 0.f;
+      uint16_t *h = in && A.H[2] ? A.H[2] + m * kMH3 : nullptr;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t r[32], p[16];
+        m_ld32(r, mine + 32 * c);
+        const float *b3 = bias + 512 + 32 * c, *w4 = bias + 640 + 32 * c;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const float2 bb = *reinterpret_cast<const float2 *>(b3 + 2 * q);
+          const float2 ww = *reinterpret_cast<const float2 *>(w4 + 2 * q);
+          p[q] = m_relu2(__uint_as_float(r[2 * q]) + bb.x, __uint_as_float(r[2 * q + 1]) + bb.y);
+          s[2 * q] = fmaf(__uint_as_float(p[q] << 16), ww.x, s[2 * q]);
+          s[2 * q + 1] = fmaf(__uint_as_float(p[q] & 0xFFFF0000u), ww.y, s[2 * q + 1]);
+        }
+        if (h) {
+          uint4 *o = reinterpret_cast<uint4 *>(h + 32 * c);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            o[q] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int l = 0; l < o; ++l) s[l] += s[l + o];
+      if (in) A.y[m] = s[0] + A.b4[0];
+    }
+  }
+  if (dead)  // a product never completed: no prediction may pass for one
+    for (; t < tiles; t += gridDim.x) {
+      const int64_t m = (int64_t)t * kMRows + row;
+      if (half == 0 && m < A.M) A.y[m] = __int_as_float(0x7FFFFFFF);
+    }
+  m_before();
+  __syncthreads();
+  if (warp == 0) {
+    m_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm) : "memory");
+  }
+}
+
+int mlp_forward(const MlpFwdArgs &A, cudaStream_t st) {
+  if (A.M < 0) return fail(POYD_EINVAL, "negative size");
+  if (A.M == 0) return POYD_OK;
+  for (int i = 0; i < 3; ++i)
+    if (!A.W[i] || !A.b[i] || ((uintptr_t)A.W[i] & 3) || ((uintptr_t)A.H[i] & 15))
+      return fail(POYD_EINVAL, "MLP forward: null or misaligned layer %d", i + 1);
+  if (!A.X || !A.w4 || !A.b4 || !A.y) return fail(POYD_EINVAL, "MLP forward: null argument");
+  if ((uintptr_t)A.X & 15) return fail(POYD_EINVAL, "MLP forward: X must be 16-byte aligned");
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kMSmem);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_mlp_forward)");
+  const int tiles = (A.M + kMRows - 1) / kMRows;
+  {
+    ProfScope ps("mlp_forward", st);
+    k_mlp_forward<<<tiles < sms ? tiles : sms, kMThreads, kMSmem, st>>>(A);
+  }
+  const cudaError_t l = cudaGetLastError();
+  return l != cudaSuccess ? cuda_fail(l, "k_mlp_forward") : POYD_OK;
+}
+
+}  // namespace
+}  // namespace poyd
+
+using namespace poyd;
+
+extern "C" int poyd_mlp_forward(const void *X, int32_t M, const void *W1t, const float *b1,
+                                const void *W2t, const float *b2, const void *W3t,
+                                const float *b3, const void *w4, const float *b4, float *y,
+                                void *stream) {
+  MlpFwdArgs A = {};
+  A.X = X;
+  A.trans = 1;
+  A.M = M;
+  const void *W[3] = {W1t, W2t, W3t};
+  const float *b[3] = {b1, b2, b3};
+  for (int i = 0; i < 3; ++i) A.W[i] = (const uint16_t *)W[i], A.b[i] = b[i];
+  A.w4 = (const uint16_t *)w4;
+  A.b4 = b4;
+  A.y = y;
+  return mlp_forward(A, (cudaStream_t)stream);
+}
+
+extern "C" int poyd_mlp_forward_rows(const void *X, int32_t x_fp32, int32_t M, const void *W1,
+                                     const float *b1, const void *W2, const float *b2,
+                                     const void *W3, const float *b3, const void *w4,
+                                     const float *b4, void *H1, void *H2, void *H3, float *y,
+                                     void *stream) {
+  MlpFwdArgs A = {};
+  A.X = X;
+  A.x32 = x_fp32;
+  A.M = M;
+  const void *W[3] = {W1, W2, W3};
+  const float *b[3] = {b1, b2, b3};
+  void *H[3] = {H1, H2, H3};
+  for (int i = 0; i < 3; ++i)
+    A.W[i] = (const uint16_t *)W[i], A.b[i] = b[i], A.H[i] = (uint16_t *)H[i];
+  A.w4 = (const uint16_t *)w4;
+  A.b4 = b4;
+  A.y = y;
+  return mlp_forward(A, (cudaStream_t)stream);
+}

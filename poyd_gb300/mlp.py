@@ -25,7 +25,13 @@ def _lib():
     L.poyd_mlp_head_backward.argtypes = [vp, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp]
     L.poyd_adam_step.argtypes = [vp, vp, vp, vp, vp, i64, f32, f32, f32, f32, i32, vp]
     L.poyd_to_bf16.argtypes = [vp, vp, i64, vp]
+    L.poyd_mlp_forward_rows.argtypes = [vp, i32, i32] + [vp] * 13
     return L
+
+
+def _aligned(t):
+    """t, or a copy when its rows do not start on 16 bytes (the kernels' loads)."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def _p(t):
@@ -64,24 +70,22 @@ class MLP:
         native.check(self.L.poyd_gemm_bf16(_p(A), lda, tA, _p(B), ldb, tB, M, N, K, _p(bias),
                                            int(relu), _p(c32), _p(c16), ldc, int(acc), _st()))
 
+    def _forward(self, X, fp32, H, y):
+        W, b = self.W16, self.b
+        native.check(self.L.poyd_mlp_forward_rows(
+            X.data_ptr(), fp32, X.shape[0], W[0].data_ptr(), b[0].data_ptr(), W[1].data_ptr(),
+            b[1].data_ptr(), W[2].data_ptr(), b[2].data_ptr(), W[3].data_ptr(), b[3].data_ptr(),
+            *[h.data_ptr() if h is not None else None for h in H], y.data_ptr(), _st()))
+
     def forward(self, X16: torch.Tensor):
         """X16 [B, 32] bf16 -> predictions [B] fp32 (activations kept)."""
         B = X16.shape[0]
         self.X16 = X16
-        self.H = []
-        a = X16
-        for i in range(3):
-            K, N = DIMS[i], DIMS[i + 1]
-            h = torch.empty((B, N), dtype=torch.bfloat16, device=self.dev)
-            self._gemm(a, 0, K, self.W16[i], 0, N, B, N, K, bias=self.b[i], relu=True, c16=h,
-                       ldc=N)
-            self.H.append(h)
-            a = h
-        y = torch.empty(B, dtype=torch.float32, device=self.dev)
-        native.check(self.L.poyd_mlp_head_forward(_p(a), _p(self.W16[3]), _p(self.b[3]), B,
-                                                  DIMS[3], _p(y), _st()))
-        self.y = y
-        return y
+        self.H = [torch.empty((B, DIMS[i + 1]), dtype=torch.bfloat16, device=self.dev)
+                  for i in range(3)]
+        self.y = torch.empty(B, dtype=torch.float32, device=self.dev)
+        self._forward(_aligned(X16), 0, self.H, self.y)
+        return self.y
 
     def backward(self, target: torch.Tensor):
         """Gradients of mean squared error; returns (loss, gW list, gb list)."""
@@ -137,13 +141,12 @@ class MLP:
 
     def predict(self, X: torch.Tensor) -> torch.Tensor:
         """Predictions for the rows of X (fp32 [n, 32]) in one fused launch
-        (``poyd_mlp_forward``), equal to ``forward``'s."""
-        X16 = X.to(torch.bfloat16).contiguous()
-        y = torch.empty(X16.shape[0], dtype=torch.float32, device=self.dev)
-        if X16.shape[0] == 0:
+        (``poyd_mlp_forward_rows``), equal to ``forward``'s."""
+        y = torch.empty(X.shape[0], dtype=torch.float32, device=self.dev)
+        if X.shape[0] == 0:
             return y
-        Wt = [w.t().contiguous() for w in self.W16[:3]]
-        native.check(self.L.poyd_mlp_forward(_p(X16), X16.shape[0], _p(Wt[0]), _p(self.b[0]),
-                                             _p(Wt[1]), _p(self.b[1]), _p(Wt[2]), _p(self.b[2]),
-                                             _p(self.W16[3]), _p(self.b[3]), _p(y), _st()))
+        if X.dtype == torch.float32 and X.is_contiguous() and X.device == y.device:
+            self._forward(_aligned(X), 1, (None, None, None), y)  # rounded to bf16 on the way in
+        else:
+            self._forward(_aligned(X.to(torch.bfloat16).contiguous()), 0, (None, None, None), y)
         return y
