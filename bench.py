@@ -1027,14 +1027,15 @@ def run_kernels(args):
     prop.fit(X, y, epochs=steps, batch=4096)
     torch.cuda.synchronize()
     wall = time.perf_counter() - t0
-    gms, gn = native.profile_read("mlp_gemm", clear=False)
+    parts = [native.profile_read(k, clear=False) for k in ("mlp_forward", "mlp_chain", "mlp_grads")]
+    gms, gn = sum(p[0] for p in parts), sum(p[1] for p in parts)
     native.profile_read(clear=True)
     native.lib().poyd_profile_enable(0)
     dims = (learned.NFEAT, 256, 256, 128)
     fwd = sum(2 * dims[i] * dims[i + 1] for i in range(3))  # per sample, GEMM layers
     flops = steps * (1 << 16) * (3 * fwd - 2 * dims[0] * dims[1])  # fwd, dW, dH (no dX)
     tf = flops / (gms * 1e-3) / 1e12 if gms else None
-    out["mlp_gemm"] = {"kernel": "k_gemm_bf16 (mma.sync m16n8k16)", "samples_per_s":
+    out["mlp_gemm"] = {"kernel": "k_mlp_forward (tcgen05), k_mlp_chain, k_mlp_grads", "samples_per_s":
                        steps * (1 << 16) / wall, "gemm_ms": gms, "gemm_launches": gn,
                        "tflop_s": tf, "peak_tflop_s": bf16, "frac": tf / bf16 if tf else None}
     return {"workload": "kernels: Fitch / Sankoff rows larger than L2, closest, MLP GEMMs",

@@ -576,6 +576,19 @@ int poyd_mlp_forward_rows(const void *X, int32_t x_fp32, int32_t M, const void *
                           const float *b1, const void *W2, const float *b2, const void *W3,
                           const float *b3, const void *w4, const float *b4, void *H1, void *H2,
                           void *H3, float *y, void *stream);
+/* Every gradient of the mean squared error of predictions y: gW, gb are host
+ * arrays of 4 device pointers (W1 [32][256], W2 [256][256], W3 [256][128],
+ * w4 [128]; b1 .. b4, fp32), loss [1].  dZ: device scratch of M * 640 bf16
+ * values, 16-byte aligned. */
+int poyd_mlp_backward(const void *X, int32_t M, const void *H1, const void *H2, const void *H3,
+                      const void *W2, const void *W3, const void *w4, const float *y,
+                      const float *target, void *dZ, float *const *gW, float *const *gb,
+                      float *loss, void *stream);
+/* poyd_adam_step over n <= 16 tensors in one launch: host arrays of device
+ * pointers (w16 entries may be NULL) and element counts. */
+int poyd_adam_step_all(int32_t n, float *const *w, void *const *w16, const float *const *g,
+                       float *const *m, float *const *v, const int64_t *sizes, float lr, float b1,
+                       float b2, float eps, int32_t step, void *stream);
 
 /* ---------------------------------------------------------------------
  * Measurement helpers (no counterpart in the reference, which has no

@@ -149,21 +149,6 @@ __global__ void k_head_backward(const __nv_bfloat16 *H, const __nv_bfloat16 *w, 
   }
 }
 
-// Adam on fp32 master weights, refreshing the bf16 copy.
-__global__ void k_adam(float *w, __nv_bfloat16 *w16, const float *g, float *mo, float *ve,
-                       int64_t n, float lr, float b1, float b2, float eps, float c1, float c2) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float m = b1 * mo[i] + (1.f - b1) * gi;
-  const float v = b2 * ve[i] + (1.f - b2) * gi * gi;
-  mo[i] = m;
-  ve[i] = v;
-  const float upd = lr * (m / c1) / (sqrtf(v / c2) + eps);
-  w[i] -= upd;
-  if (w16) w16[i] = __float2bfloat16_rn(w[i]);
-}
-
 __global__ void k_to_bf16(const float *x, __nv_bfloat16 *y, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = __float2bfloat16_rn(x[i]);
@@ -236,19 +221,6 @@ extern "C" int poyd_mlp_head_backward(const void *H, const void *w, const float 
   k_head_backward<<<nblk((int64_t)M * K, 256) < 1024 ? nblk((int64_t)M * K, 256) : 1024, 256, 0,
                     st>>>((const __nv_bfloat16 *)H, (const __nv_bfloat16 *)w, y, target, M, K,
                           (__nv_bfloat16 *)dZ, dw, db, loss);
-  MLP_LAUNCH_CHECK();
-  return POYD_OK;
-}
-
-extern "C" int poyd_adam_step(float *w, void *w16, const float *g, float *m, float *v, int64_t n,
-                              float lr, float b1, float b2, float eps, int32_t step,
-                              void *stream) {
-  if (n <= 0) return POYD_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  ProfScope ps("mlp_adam", st);
-  k_adam<<<nblk(n, 256), 256, 0, st>>>(w, (__nv_bfloat16 *)w16, g, m, v, n, lr, b1, b2, eps, c1,
-                                       c2);
   MLP_LAUNCH_CHECK();
   return POYD_OK;
 }

@@ -152,13 +152,15 @@ __device__ __forceinline__ void m_stage_w(uint8_t *dst, const uint16_t *W, int K
   }
   // [k][n]: two k rows of eight columns per thread, paired into words
   const int n8s = N / 8;
+#pragma unroll 4
   for (int e = threadIdx.x; e < K / 2 * n8s; e += kMThreads) {
     const int lo = e & 31, hi = e >> 5;
     const int n8 = hi % (n8s / 8) * 8 + (lo >> 2), k = 2 * (hi / (n8s / 8) * 4 + (lo & 3));
     const uint16_t *s0 = W + (int64_t)k * N + n8 * 8, *s1 = s0 + N;
     uint32_t a[4], b[4];
     if (al) {
-      const uint4 u = *reinterpret_cast<const uint4 *>(s0), v = *reinterpret_cast<const uint4 *>(s1);
+      const uint4 u = __ldg(reinterpret_cast<const uint4 *>(s0));
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(s1));
       a[0] = u.x, a[1] = u.y, a[2] = u.z, a[3] = u.w;
       b[0] = v.x, b[1] = v.y, b[2] = v.z, b[3] = v.w;
     } else {

@@ -26,6 +26,8 @@ def _lib():
     L.poyd_adam_step.argtypes = [vp, vp, vp, vp, vp, i64, f32, f32, f32, f32, i32, vp]
     L.poyd_to_bf16.argtypes = [vp, vp, i64, vp]
     L.poyd_mlp_forward_rows.argtypes = [vp, i32, i32] + [vp] * 13
+    L.poyd_mlp_backward.argtypes = [vp, i32] + [vp] * 13
+    L.poyd_adam_step_all.argtypes = [i32] + [vp] * 6 + [f32, f32, f32, f32, i32, vp]
     return L
 
 
@@ -34,8 +36,8 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+def _ptrs(ts):
+    return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
 def _st():
@@ -65,11 +67,6 @@ class MLP:
     def state(self):
         return {"W": [w.cpu().numpy() for w in self.W], "b": [b.cpu().numpy() for b in self.b]}
 
-    def _gemm(self, A, tA, lda, B, tB, ldb, M, N, K, bias=None, relu=False, c32=None, c16=None,
-              ldc=None, acc=False):
-        native.check(self.L.poyd_gemm_bf16(_p(A), lda, tA, _p(B), ldb, tB, M, N, K, _p(bias),
-                                           int(relu), _p(c32), _p(c16), ldc, int(acc), _st()))
-
     def _forward(self, X, fp32, H, y):
         W, b = self.W16, self.b
         native.check(self.L.poyd_mlp_forward_rows(
@@ -92,36 +89,23 @@ class MLP:
         B = self.X16.shape[0]
         gW = [torch.empty_like(w) for w in self.W]
         gb = [torch.empty_like(b) for b in self.b]
-        loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
-        dZ = torch.empty((B, DIMS[3]), dtype=torch.bfloat16, device=self.dev)
-        native.check(self.L.poyd_mlp_head_backward(_p(self.H[2]), _p(self.W16[3]), _p(self.y),
-                                                   _p(target), B, DIMS[3], _p(dZ),
-                                                   _p(gW[3]), _p(gb[3]), _p(loss), _st()))
-        for i in (2, 1, 0):
-            K, N = DIMS[i], DIMS[i + 1]
-            a_in = self.X16 if i == 0 else self.H[i - 1]
-            # dW_i = a_in^T dZ  ([K, N], reduction over the batch)
-            self._gemm(a_in, 1, K, dZ, 0, N, K, N, B, c32=gW[i], ldc=N)
-            native.check(self.L.poyd_colsum_bf16(_p(dZ), B, N, _p(gb[i]), _st()))
-            if i > 0:
-                dH = torch.empty((B, K), dtype=torch.bfloat16, device=self.dev)
-                # dH = dZ W_i^T  ([B, K])
-                self._gemm(dZ, 0, N, self.W16[i], 1, N, B, K, N, c16=dH, ldc=K)
-                dZn = torch.empty_like(dH)
-                native.check(self.L.poyd_relu_grad_bf16(_p(dH), _p(self.H[i - 1]), _p(dZn),
-                                                        dH.numel(), _st()))
-                dZ = dZn
+        loss = torch.empty(1, dtype=torch.float32, device=self.dev)
+        dZ = torch.empty(B * sum(DIMS[1:4]), dtype=torch.bfloat16, device=self.dev)
+        X = _aligned(self.X16)
+        native.check(self.L.poyd_mlp_backward(
+            X.data_ptr(), B, *[h.data_ptr() for h in self.H], self.W16[1].data_ptr(),
+            self.W16[2].data_ptr(), self.W16[3].data_ptr(), self.y.data_ptr(), target.data_ptr(),
+            dZ.data_ptr(), _ptrs(gW), _ptrs(gb), loss.data_ptr(), _st()))
         return loss, gW, gb
 
     def step(self, gW, gb, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.steps += 1
-        for i in range(4):
-            native.check(self.L.poyd_adam_step(_p(self.W[i]), _p(self.W16[i]), _p(gW[i]),
-                                               _p(self.mW[i]), _p(self.vW[i]), self.W[i].numel(),
-                                               lr, b1, b2, eps, self.steps, _st()))
-            native.check(self.L.poyd_adam_step(_p(self.b[i]), None, _p(gb[i]), _p(self.mb[i]),
-                                               _p(self.vb[i]), self.b[i].numel(), lr, b1, b2, eps,
-                                               self.steps, _st()))
+        w = self.W + self.b
+        w16 = (C.c_void_p * 8)(*[x.data_ptr() for x in self.W16], None, None, None, None)
+        sizes = (C.c_int64 * 8)(*[x.numel() for x in w])
+        native.check(self.L.poyd_adam_step_all(
+            8, _ptrs(w), w16, _ptrs(list(gW) + list(gb)), _ptrs(self.mW + self.mb),
+            _ptrs(self.vW + self.vb), sizes, lr, b1, b2, eps, self.steps, _st()))
 
     def fit(self, X: torch.Tensor, y: torch.Tensor, epochs=3, batch=4096, lr=1e-3, seed=0):
         """Mini-batch Adam on (X fp32 [n, 32], y fp32 [n]); returns losses."""

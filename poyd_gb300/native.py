@@ -66,7 +66,7 @@ class PoydTuneResult(C.Structure):
 # tests check the header's declarations against this list and that the
 # library exports each of them.
 EXPORTED = (
-    "poyd_adam_step", "poyd_autotune_batch", "poyd_autotune_clear", "poyd_autotune_get",
+    "poyd_adam_step", "poyd_adam_step_all", "poyd_autotune_batch", "poyd_autotune_clear", "poyd_autotune_get",
     "poyd_autotune_set", "poyd_algn_align_2d", "poyd_algn_align_affine_3", "poyd_algn_ancestor_2",
     "poyd_algn_backtrack_2d", "poyd_algn_cost_affine_3", "poyd_algn_median_2_no_gaps",
     "poyd_algn_median_2_with_gaps", "poyd_algn_simple_2", "poyd_algn_verify_2",
@@ -77,7 +77,7 @@ EXPORTED = (
     "poyd_int_pipe_rate", "poyd_last_error", "poyd_launch_count", "poyd_matrix_create",
     "poyd_matrix_free", "poyd_median_2_no_gaps_batch", "poyd_median_2_with_gaps_batch",
     "poyd_median_levels",
-    "poyd_mlp_forward", "poyd_mlp_forward_rows", "poyd_mlp_head_backward", "poyd_mlp_head_forward", "poyd_nonadd16_distance_batch",
+    "poyd_mlp_backward", "poyd_mlp_forward", "poyd_mlp_forward_rows", "poyd_mlp_head_backward", "poyd_mlp_head_forward", "poyd_nonadd16_distance_batch",
     "poyd_nonadd16_median_3_batch", "poyd_nonadd16_median_batch",
     "poyd_nonadd32_distance_batch", "poyd_nonadd32_median_3_batch",
     "poyd_nonadd32_median_batch", "poyd_nonadd8_distance_batch", "poyd_nonadd8_median_3_batch",
