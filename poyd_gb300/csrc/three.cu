@@ -7,7 +7,9 @@
 // of Ukkonen's algorithm over 16 column states, with check-pointing
 // (ukk.checkp.c).  Its cost is the optimum of a fixed cost model
 // (alignmentCost, ukkCommon.c:345-391), which does not depend on how the
-// optimum is searched.  Here each triple is one dynamic program over the
+// optimum is searched.  Without gap openings (go = 0) the 16 states share
+// one optimum per cell and three_linear.cu takes the batch; with them, here,
+// each triple is one dynamic program over the
 // full (la x lb x lc) cube and the 16 states, swept by hyperplanes
 // h = i + j + k (a cell depends only on the three hyperplanes before it):
 //   * one block per triple (a cluster of 2-8 blocks for small batches),
@@ -36,7 +38,7 @@
 #include <cstring>
 #include <vector>
 
-#include "poyd_internal.h"
+#include "three_kernels.cuh"
 
 #define CK3(call)                                         \
   do {                                                    \
@@ -46,72 +48,13 @@
 
 namespace poyd {
 
-constexpr int kP3States = 16;
 constexpr int kP3Threads = 256;
 constexpr int kP3Inf = 1 << 30;      // x16 domain
 constexpr int kP3MaxLen = 4096;
 
-// Powell's column states (ukkCommon.c:206-262): per sequence match (M),
-// delete (D) or insert (I), at least one M and at most one I, numbered in
-// increasing order of x0 + 3 x1 + 9 x2 (M 0, D 1, I 2), MMM first.  A
-// state without I consumes a character of each M sequence; a state with I
-// consumes one of the I sequence only.  ngo[s][t] counts the gap openings
-// of a step from s to t (ukkCommon.c:263-290): the sequences in D or I in
-// t that were not in that same state in s.
-struct P3States {
-  int code[kP3States], adv[kP3States], ins[kP3States], ndel[kP3States];
-  int ngo[kP3States][kP3States];
-};
-
-__host__ __device__ constexpr P3States p3_states() {
-  P3States S{};
-  int n = 0;
-  for (int c = 0; c < 27; ++c) {
-    const int x0 = c % 3, x1 = c / 3 % 3, x2 = c / 9 % 3;
-    const int nm = (x0 == 0) + (x1 == 0) + (x2 == 0);
-    const int ni = (x0 == 2) + (x1 == 2) + (x2 == 2);
-    if (nm == 0 || ni > 1) continue;
-    S.code[n] = c;
-    S.ins[n] = ni;
-    S.ndel[n] = 3 - nm - ni;
-    S.adv[n] = ni ? ((x0 == 2) | (x1 == 2) << 1 | (x2 == 2) << 2)
-                  : ((x0 == 0) | (x1 == 0) << 1 | (x2 == 0) << 2);
-    ++n;
-  }
-  for (int s = 0; s < kP3States; ++s)
-    for (int t = 0; t < kP3States; ++t) {
-      int k = 0, cs = S.code[s], ct = S.code[t];
-      for (int q = 0; q < 3; ++q, cs /= 3, ct /= 3)
-        if (ct % 3 != 0 && ct % 3 != cs % 3) ++k;
-      S.ngo[s][t] = k;
-    }
-  return S;
-}
-
 // The same tables for indices known only at run time (traceback, table
 // setup): constant memory rather than a local copy.
 __constant__ P3States c_p3 = p3_states();
-
-struct P3Args {
-  int n, mode;            // mode 1: readjust_3d's early returns and changed flags
-  const uint8_t *seq;
-  const int64_t *off[4];  // a, b, c; m (mode 1)
-  const int32_t *len[4];
-  int32_t *cost;
-  uint8_t *out;
-  const int64_t *out_off;
-  int32_t *out_len;
-  int32_t *changed;
-  const int32_t *order;
-  int32_t *counter;
-  int32_t *err;
-  int32_t *ring;
-  int64_t ring_stride;    // int32 per block
-  uint64_t *dir;
-  int64_t dir_stride;     // words per block
-  int mm, go, ge, gap, has_med, smax;
-  uint8_t med[128];       // Three_D.median of (x, y, z) over A C G T gap, 25 x + 5 y + z
-};
 
 // Offset of the (j + k = s) row in an i-slice of the choice cube:
 // the sum over s' < s of the row lengths min(nb, s') - max(0, s' - nc) + 1.
@@ -125,11 +68,6 @@ __device__ __forceinline__ int64_t p3_soff(int s, int nb, int nc) {
   }
   return f;
 }
-
-__device__ __forceinline__ int p3_code(int x) {  // copySequence: lowest of A C G T
-  return (x & 1) ? 1 : (x & 2) ? 2 : (x & 4) ? 4 : (x & 8) ? 8 : 0;
-}
-__device__ __forceinline__ int p3_ix(int x) { return __ffs(x) - 1; }  // 1 2 4 8 16 -> 0..4
 
 // One cell (a, b, c) of hyperplane h: its 16 values (x16, into the ring)
 // and its 64-bit choice word (returned).
@@ -192,12 +130,8 @@ __device__ __forceinline__ uint64_t p3_cell(int32_t *ring, int64_t pl, int nb, i
 // are read from a constant infinite cell, so the 14 loads of a cell issue
 // before any of its arithmetic.
 constexpr unsigned kP3Inf2 = 0xC000C000u;
-// min per half (measured: the fused add-min with a zero addend in its
-// place executes 365 instructions per cell instead of 331; sharing one
-// 16-way minimum among the next states of a step when go = 0 let the
-// loads interleave with the arithmetic again and ran 1.5x slower)
 __device__ __forceinline__ unsigned p3_min2(unsigned a, unsigned b) { return __vminu2(a, b); }
-template <bool GO0, bool CL>
+template <bool CL>
 __device__ __forceinline__ uint64_t p3_cell16(const uint16_t *const *src, uint16_t *dst,
                                               const unsigned *gg, const uint4 ca,
                                               const uint4 cb) {
@@ -222,9 +156,7 @@ __device__ __forceinline__ uint64_t p3_cell16(const uint16_t *const *src, uint16
       if (S.adv[t] != d) continue;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        best[t] = GO0 ? p3_min2(w[q], best[t])
-                      : __viaddmin_u16x2(w[q], gg[4 * S.ngo[2 * q][t] + S.ngo[2 * q + 1][t]],
-                                         best[t]);
+        best[t] = __viaddmin_u16x2(w[q], gg[4 * S.ngo[2 * q][t] + S.ngo[2 * q + 1][t]], best[t]);
     }
   }
   const unsigned col2[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
@@ -265,7 +197,7 @@ __device__ __forceinline__ unsigned p3_col2(int k, int x0, int x1, int x2, int m
 // ends each hyperplane; block 0 of the cluster takes the jobs, writes the
 // early-return outputs and walks the choices back.  Every branch depends
 // only on data all blocks read alike, so all blocks reach every barrier.
-template <bool PACKED, bool GO0, bool CL>
+template <bool PACKED, bool CL>
 __global__ void __launch_bounds__(kP3Threads) k_p3(const __grid_constant__ P3Args A) {
   namespace cg = cooperative_groups;
   constexpr P3States S = p3_states();
@@ -315,66 +247,10 @@ __global__ void __launch_bounds__(kP3Threads) k_p3(const __grid_constant__ P3Arg
     if (job >= A.n) break;
     const int i = A.order[job];
     const int la = A.len[0][i], lb = A.len[1][i], lc = A.len[2][i];
-    const uint8_t *src[3] = {A.seq + A.off[0][i], A.seq + A.off[1][i], A.seq + A.off[2][i]};
     const int cap = (la + lb + lc + 3) & ~3;
     uint8_t *o = A.out + A.out_off[i];
-
-    if (A.mode == 1) {
-      // readjust_3d's early returns (sequence.ml:1118-1129); is_empty is
-      // sequence.ml:442-450
-      const int lm = A.len[3][i];
-      const uint8_t *m = A.seq + A.off[3][i];
-      int keep = 0;  // 1 m, 2 b, 3 a, 4 c
-      if (la == lb && lm == lc && la == lm) {
-        keep = 1;
-      } else {
-        bool e[3] = {true, true, true};
-        for (int q = 0; q < 3; ++q) {
-          const int l = q == 0 ? la : q == 1 ? lb : lc;
-          bool all = true;
-          for (int x = tid; x < l; x += kP3Threads) all &= src[q][x] == A.gap;
-          e[q] = __syncthreads_and(all);
-        }
-        keep = (e[0] && !e[1]) ? 2 : (e[1] && !e[0]) ? 3 : e[2] ? 4 : 0;
-      }
-      if (keep) {
-        const uint8_t *k = keep == 1 ? m : keep == 2 ? src[1] : keep == 3 ? src[0] : src[2];
-        const int lk = keep == 1 ? lm : keep == 2 ? lb : keep == 3 ? la : lc;
-        bool diff = lk != lm;
-        for (int x = tid; x < lk; x += kP3Threads) {
-          if (lead) o[4 * cap - lk + x] = k[x];
-          if (lk == lm) diff |= k[x] != m[x];
-        }
-        diff = __syncthreads_or(diff);
-        if (lead && tid == 0) {
-          A.cost[i] = 0;
-          A.out_len[2 * i] = 0;
-          A.out_len[2 * i + 1] = lk;
-          A.changed[i] = diff ? 1 : 0;
-        }
-        bar();
-        continue;
-      }
-    }
-
-    // the characters Powell's code aligns (copySequence, ukkCommon.c:84-105)
-    bool bad = false;
-    for (int q = 0; q < 3; ++q) {
-      const int l = q == 0 ? la : q == 1 ? lb : lc;
-      for (int x = 1 + tid; x < l; x += kP3Threads) {
-        const int c = p3_code(src[q][x]);
-        bad |= c == 0;
-        sqw[q][x] = (uint8_t)c;
-      }
-    }
-    if (__syncthreads_or(bad)) {
-      if (lead && tid == 0) {
-        A.cost[i] = -1;
-        A.out_len[2 * i] = -1;
-        A.out_len[2 * i + 1] = -1;
-        if (A.mode == 1) A.changed[i] = 0;
-        atomicOr(A.err, 1);
-      }
+    if (!p3_begin(A, i, lead, tid, kP3Threads,
+                  [&](int q, int x, int c) { sqw[q][x] = (uint8_t)c; })) {
       bar();
       continue;
     }
@@ -406,7 +282,7 @@ __global__ void __launch_bounds__(kP3Threads) k_p3(const __grid_constant__ P3Arg
               src[d - 1] = ok ? ring16 + rb[d - 1] + b16 : infc;
             }
             const int cmb = (i0 * 5 + (b ? __ffs(sq[1][b]) : 0)) * 5 + (c ? __ffs(sq[2][c]) : 0);
-            dir[drow + b] = p3_cell16<GO0, CL>(src, ring16 + ob + b16, gg, ctab[2 * cmb],
+            dir[drow + b] = p3_cell16<CL>(src, ring16 + ob + b16, gg, ctab[2 * cmb],
                                            ctab[2 * cmb + 1]);
           }
           continue;
@@ -522,7 +398,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     CK3(cudaMemcpyAsync(hl[q].data(), len[q], sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
   }
   CK3(cudaStreamSynchronize(st));
-  int64_t ring_max = 0, dir_max = 0;
+  int64_t ring_max = 0, dir_max = 0, lin_plane = 0, lin_dir = 0;
   int smax = 16;
   std::vector<int64_t> work(n);
   const int64_t step_max = 2LL * go + 2LL * ge + 2LL * mm;
@@ -538,7 +414,11 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     dir_max = std::max(dir_max, la * lb * lc);
     smax = std::max<int>(smax, (int)std::max(la, std::max(lb, lc)));
     work[i] = la * lb * lc;
+    const P3LinearPlan lp = p3_linear_plan(la, lb, lc);
+    lin_plane = std::max(lin_plane, lp.plane);
+    lin_dir = std::max(lin_dir, lp.dir);
   }
+  const int longest = smax;
   smax = (smax + 15) & ~15;
   std::vector<int32_t> order;
   longest_first(work, order);
@@ -548,18 +428,14 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   CK3(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   size_t fr = 0, tot = 0;
   CK3(cudaMemGetInfo(&fr, &tot));
-  const int64_t per_block = ring_max * 4 + dir_max * 8;
-  // the choice cubes dominate: one per resident block, sized for the
-  // largest triple; by default at most 60 % of the free memory, 120 GiB
+  // the choices dominate: one set per resident block, sized for the largest
+  // triple; by default at most 60 % of the free memory, 120 GiB
   int64_t budget = std::min<int64_t>((int64_t)(fr * 0.6), 120LL << 30);
   if (const char *e = getenv("POYD_P3_BUDGET_MB")) budget = std::max<int64_t>(1, atoll(e)) << 20;
-  int64_t blocks = std::min<int64_t>({(int64_t)n, 3LL * sms, std::max<int64_t>(1, budget / per_block)});
 
   Workspace *w = workspace(st);
-  int32_t *ring = (int32_t *)ws_buffer(w, WS_P3_RING, (size_t)(ring_max * 4 * blocks));
-  uint64_t *dirp = (uint64_t *)ws_buffer(w, WS_P3_DIR, (size_t)(dir_max * 8 * blocks));
   int32_t *meta = (int32_t *)ws_buffer(w, WS_P3_META, sizeof(int32_t) * ((size_t)n + 4));
-  if (!ring || !dirp || !meta) return fail(POYD_ENOMEM, "three-sequence workspace (%lld blocks)", (long long)blocks);
+  if (!meta) return fail(POYD_ENOMEM, "three-sequence workspace");
   order.push_back(0);  // counter
   order.push_back(0);  // err
   CK3(cudaMemcpyAsync(meta, order.data(), sizeof(int32_t) * ((size_t)n + 2), cudaMemcpyHostToDevice, st));
@@ -581,10 +457,6 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   A.order = meta;
   A.counter = meta + n;
   A.err = meta + n + 1;
-  A.ring = ring;
-  A.ring_stride = ring_max;
-  A.dir = dirp;
-  A.dir_stride = dir_max;
   A.mm = mm;
   A.go = go;
   A.ge = ge;
@@ -599,13 +471,60 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
               median3 ? median3[(st5[x] << 10) | (st5[y] << 5) | st5[z]] : (uint8_t)gap;
   }
   A.smax = smax;
-  const size_t smem = 3 * (size_t)smax + 125 * 8 * sizeof(unsigned);
+  // the launch's error bits; bit 2: an optimum reached the 16-bit clamp, the
+  // batch is redone in 32 bits
+  auto finish = [&](bool *redo) -> int {
+    int32_t herr = 0;
+    CK3(cudaGetLastError());
+    CK3(cudaMemcpyAsync(&herr, A.err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    CK3(cudaStreamSynchronize(st));
+    *redo = false;
+    if (herr & 1)
+      return fail(POYD_EINVAL, "an element holds none of A, C, G, T (powell_3D_align fails, "
+                               "ukkCommon.c:101): its triple has cost -1");
+    if (herr & 2) return fail(POYD_ERANGE, "three-sequence traceback left the cube");
+    if (!(herr & 4)) return POYD_OK;
+    *redo = true;
+    const int32_t zero2[2] = {0, 0};
+    CK3(cudaMemcpyAsync(A.counter, zero2, sizeof(zero2), cudaMemcpyHostToDevice, st));
+    return POYD_OK;
+  };
   // 16-bit halves while every addend of a half stays below 0x4000
-  // (openings, column costs); a triple whose optimum reaches the clamp
-  // sets err bit 4 and the batch is redone in 32 bits
+  // (openings, column costs)
   const char *pk = getenv("POYD_P3_PACKED");
   bool packed = !(pk && pk[0] == '0') && 48LL * go + 15 < 0x4000 &&
                 16LL * (2LL * mm + 3LL * ge) < 0x4000;
+  if (packed && go == 0) {
+    // Warps per triple: consecutive strips run kP3LinLag steps apart, so a
+    // triple feeds about (steps of a strip) / kP3LinLag warps.  A batch that
+    // fills the SMs takes at most 4 (more blocks per SM share the issue
+    // slots alike, and its shorter triples waste fewer warps); a small one
+    // takes what its longest triple can use.
+    int warps = 1;
+    const int most = (int64_t)n * 4 >= 8LL * sms ? 4 : 16;
+    while (2 * warps <= most && 2 * warps * kP3LinLag <= longest + 40) warps *= 2;
+    const int64_t per = lin_plane + lin_dir;
+    const int blocks = (int)std::min<int64_t>(
+        {(int64_t)n, (int64_t)p3_linear_blocks(warps, longest), std::max<int64_t>(1, budget / per)});
+    uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(lin_plane * blocks));
+    uint8_t *dirb = (uint8_t *)ws_buffer(w, WS_P3_DIR, (size_t)(lin_dir * blocks));
+    if (!plane || !dirb) return fail(POYD_ENOMEM, "three-sequence workspace (%d blocks)", blocks);
+    int rc = launch_p3_linear(A, warps, longest, blocks, plane, lin_plane, dirb, lin_dir, st);
+    if (rc) return rc;
+    bool redo = false;
+    rc = finish(&redo);
+    if (rc || !redo) return rc;
+    packed = false;
+  }
+  const int64_t per_block = ring_max * 4 + dir_max * 8;
+  int64_t blocks = std::min<int64_t>({(int64_t)n, 3LL * sms, std::max<int64_t>(1, budget / per_block)});
+  A.ring = (int32_t *)ws_buffer(w, WS_P3_RING, (size_t)(ring_max * 4 * blocks));
+  A.dir = (uint64_t *)ws_buffer(w, WS_P3_DIR, (size_t)(dir_max * 8 * blocks));
+  if (!A.ring || !A.dir)
+    return fail(POYD_ENOMEM, "three-sequence workspace (%lld blocks)", (long long)blocks);
+  A.ring_stride = ring_max;
+  A.dir_stride = dir_max;
+  const size_t smem = 3 * (size_t)smax + 125 * 8 * sizeof(unsigned);
   // small batches: a cluster of up to 8 blocks per triple, so that the
   // batch still covers the SMs (POYD_P3_CLUSTER=0: one block per triple)
   int csize = 1;
@@ -616,9 +535,8 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
       while (csize < 8 && 2 * csize <= want) csize *= 2;
   }
   for (;;) {
-    auto kern = packed ? (go == 0 ? k_p3<true, true, false> : k_p3<true, false, false>)
-                       : k_p3<false, false, false>;
-    auto kcl = go == 0 ? k_p3<true, true, true> : k_p3<true, false, true>;
+    auto kern = packed ? k_p3<true, false> : k_p3<false, false>;
+    auto kcl = k_p3<true, true>;
     bool launched = false;
     if (packed && csize > 1) {
       cudaLaunchConfig_t cfg = {};
@@ -651,18 +569,10 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
       ProfScope ps("p3", st);
       kern<<<(unsigned)blocks, kP3Threads, smem, st>>>(A);
     }
-    CK3(cudaGetLastError());
-    int32_t herr = 0;
-    CK3(cudaMemcpyAsync(&herr, A.err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    CK3(cudaStreamSynchronize(st));
-    if (herr & 1)
-      return fail(POYD_EINVAL, "an element holds none of A, C, G, T (powell_3D_align fails, "
-                               "ukkCommon.c:101): its triple has cost -1");
-    if (herr & 2) return fail(POYD_ERANGE, "three-sequence traceback left the cube");
-    if (!(herr & 4)) return POYD_OK;
-    packed = false;  // some optimum reached the 16-bit clamp
-    const int32_t zero2[2] = {0, 0};
-    CK3(cudaMemcpyAsync(A.counter, zero2, sizeof(zero2), cudaMemcpyHostToDevice, st));
+    bool redo = false;
+    const int rc = finish(&redo);
+    if (rc || !redo) return rc;
+    packed = false;
   }
 }
 
