@@ -7,33 +7,30 @@
 // of Ukkonen's algorithm over 16 column states, with check-pointing
 // (ukk.checkp.c).  Its cost is the optimum of a fixed cost model
 // (alignmentCost, ukkCommon.c:345-391), which does not depend on how the
-// optimum is searched.  Without gap openings (go = 0) the 16 states share
-// one optimum per cell and three_linear.cu takes the batch; with them, here,
-// each triple is one dynamic program over the
-// full (la x lb x lc) cube and the 16 states, swept by hyperplanes
-// h = i + j + k (a cell depends only on the three hyperplanes before it):
-//   * one block per triple (a cluster of 2-8 blocks for small batches),
-//     persistent over a largest-first queue; a warp takes a row (fixed i)
-//     of the hyperplane, a lane one cell of it;
-//   * a thread computes all 16 states of its cell: every state reads one
-//     neighbour cell (the one its column consumes from), so a cell loads 7
-//     neighbours of 16 values; values are stored x16 with a state number
-//     in the low 4 bits, so that one add-min per (previous, next) state
-//     pair keeps the least cost and, on ties, the lowest-numbered previous
-//     state; by default two states per 32-bit word (16-bit halves), the
-//     32-bit values as the fallback for large costs;
-//   * the last four hyperplanes' values in a ring in global memory
-//     ([h & 3][i][j][state]); the 16 choices of a cell (4 bits each) in
-//     one 64-bit word of a per-triple cube laid out [i][j + k][j] so that
-//     a hyperplane's cells of one i are contiguous;
-//   * then one thread walks the choices back and writes the three aligned
-//     rows and the column medians (Cost_matrix.Three_D.median) right-aligned
-//     into the triple's slot.
+// optimum is searched.  Each triple is one dynamic program over the full
+// (la x lb x lc) cube, one cell's states from its seven neighbours', by one of
+// three kernels:
+//   * three_linear.cu: no gap openings (go = 0, the linear model), 16-bit
+//     values, one optimum per cell;
+//   * three_open.cu: gap openings, 16-bit values;
+//   * k_p3 (here): 32-bit values, for batches whose costs may not fit 16 bits,
+//     swept by hyperplanes h = i + j + k (a cell depends only on the three
+//     hyperplanes before it): one block per triple, persistent over a
+//     largest-first queue; a warp takes a row (fixed i) of the hyperplane, a
+//     lane one cell of it.  Every state reads one neighbour cell (the one its
+//     column consumes from); values are stored x16 with a state number in the
+//     low 4 bits, so that one add-min per (previous, next) state pair keeps
+//     the least cost and, on ties, the lowest-numbered previous state.  The
+//     last four hyperplanes' values are a ring in global memory
+//     ([h & 3][i][j][state]); the 16 choices of a cell (4 bits each) one
+//     64-bit word of a per-triple cube laid out [i][j + k][j] so that a
+//     hyperplane's cells of one i are contiguous.
+// One warp then walks the choices back (three_kernels.cuh) and writes the
+// three aligned rows and the column medians (Cost_matrix.Three_D.median)
+// right-aligned into the triple's slot.
 // Among equally cheap alignments the walk keeps the lowest-numbered final
 // state and at every column the lowest-numbered previous state; Powell's
 // recursion may return another of the optimal alignments.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -118,189 +115,43 @@ __device__ __forceinline__ uint64_t p3_cell(int32_t *ring, int64_t pl, int nb, i
   return word;
 }
 
-// The same cell with two values per 32-bit word, for batches whose costs
-// stay small: x16 values in 16-bit halves of a uint16 ring, each value
-// carrying its own state number in the low 4 bits, so that a value loaded
-// as a previous state already holds its rank, and one __viaddmin_u16x2
-// tries two previous states.  Infinity is 0xC000; every value is clamped
-// to it and every addend stays below 0x4000, so no half wraps.  A value
-// that reaches the clamp is not exact; a triple whose optimum reaches it is
-// redone by the 32-bit cell (the cells of an optimal path never exceed the
-// optimum, so a smaller optimum is exact).  Neighbours outside the cube
-// are read from a constant infinite cell, so the 14 loads of a cell issue
-// before any of its arithmetic.
-constexpr unsigned kP3Inf2 = 0xC000C000u;
-__device__ __forceinline__ unsigned p3_min2(unsigned a, unsigned b) { return __vminu2(a, b); }
-template <bool CL>
-__device__ __forceinline__ uint64_t p3_cell16(const uint16_t *const *src, uint16_t *dst,
-                                              const unsigned *gg, const uint4 ca,
-                                              const uint4 cb) {
-  constexpr P3States S = p3_states();
-  uint4 u[7][2];
-#pragma unroll
-  for (int d = 0; d < 7; ++d) {
-    const uint4 *p = reinterpret_cast<const uint4 *>(src[d]);
-    // a cluster's blocks write each other's neighbours: read them from L2
-    u[d][0] = CL ? __ldcg(p) : p[0];
-    u[d][1] = CL ? __ldcg(p + 1) : p[1];
-  }
-  unsigned best[kP3States];
-#pragma unroll
-  for (int t = 0; t < kP3States; ++t) best[t] = kP3Inf2;
-#pragma unroll
-  for (int d = 1; d < 8; ++d) {
-    const unsigned w[8] = {u[d - 1][0].x, u[d - 1][0].y, u[d - 1][0].z, u[d - 1][0].w,
-                           u[d - 1][1].x, u[d - 1][1].y, u[d - 1][1].z, u[d - 1][1].w};
-#pragma unroll
-    for (int t = 0; t < kP3States; ++t) {
-      if (S.adv[t] != d) continue;
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        best[t] = __viaddmin_u16x2(w[q], gg[4 * S.ngo[2 * q][t] + S.ngo[2 * q + 1][t]], best[t]);
-    }
-  }
-  const unsigned col2[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-  uint64_t word = 0;
-  unsigned v[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {  // states 2k (low half) and 2k + 1 (high half)
-    const unsigned lo = __byte_perm(best[2 * k], best[2 * k + 1], 0x5410);
-    const unsigned hi = __byte_perm(best[2 * k], best[2 * k + 1], 0x7632);
-    const unsigned m = p3_min2(lo, hi);
-    const unsigned own = (unsigned)(2 * k) | (unsigned)(2 * k + 1) << 16;
-    v[k] = p3_min2((m & 0xFFF0FFF0u) + col2[k], kP3Inf2 + own);
-    word |= (uint64_t)(m & 15u) << (8 * k) | (uint64_t)(m >> 16 & 15u) << (8 * k + 4);
-  }
-  uint4 *o = reinterpret_cast<uint4 *>(dst);
-  o[0] = make_uint4(v[0], v[1], v[2], v[3]);
-  o[1] = make_uint4(v[4], v[5], v[6], v[7]);
-  return word;
-}
-
-// Column costs of the packed cell (x16, each state's own number added):
-// state pairs (2k, 2k + 1) for the characters x0, x1, x2 (0: none) of a
-// cell; an entry whose state needs a missing character is never used.
-__device__ __forceinline__ unsigned p3_col2(int k, int x0, int x1, int x2, int mm16, int ge16) {
-  const P3States &S = c_p3;
-  unsigned r = 0;
-  for (int h = 0; h < 2; ++h) {
-    const int t = 2 * k + h, d = S.adv[t];
-    const int ch = ((d & 1) ? x0 : 0) | ((d & 2) ? x1 : 0) | ((d & 4) ? x2 : 0);
-    const int col = S.ins[t] ? ge16 : mm16 * max(__popc(ch) - 1, 0) + S.ndel[t] * ge16;
-    r |= (unsigned)(col + t) << (16 * h);
-  }
-  return r;
-}
-
-// CL: a thread-block cluster per triple (small batches): the rows of a
-// hyperplane are spread over the cluster's blocks and a cluster barrier
-// ends each hyperplane; block 0 of the cluster takes the jobs, writes the
-// early-return outputs and walks the choices back.  Every branch depends
-// only on data all blocks read alike, so all blocks reach every barrier.
-template <bool PACKED, bool CL>
 __global__ void __launch_bounds__(kP3Threads) k_p3(const __grid_constant__ P3Args A) {
-  namespace cg = cooperative_groups;
-  constexpr P3States S = p3_states();
   extern __shared__ uint8_t p3_sm[];
   __shared__ int s_job;
-  const int rank = CL ? (int)cg::this_cluster().block_rank() : 0;
-  const int csz = CL ? (int)cg::this_cluster().num_blocks() : 1;
-  const bool lead = rank == 0;
-  auto bar = [&]() {
-    if (CL) cg::this_cluster().sync();
-    else __syncthreads();
-  };
-  const uint8_t *sq[3] = {p3_sm, p3_sm + A.smax, p3_sm + 2 * A.smax};
-  uint8_t *sqw[3] = {p3_sm, p3_sm + A.smax, p3_sm + 2 * A.smax};
+  uint8_t *sq[3] = {p3_sm, p3_sm + A.smax, p3_sm + 2 * A.smax};
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kWarps = kP3Threads / 32;
   // x16 costs: g16[k] = k gap openings, g16[4] = one extension
   const int g16[5] = {0, 16 * A.go, 32 * A.go, 48 * A.go, 16 * A.ge};
-  const int64_t slot = CL ? blockIdx.x / csz : blockIdx.x;  // the block's (cluster's) scratch
-  int32_t *ring = A.ring + slot * A.ring_stride;
-  // packed: [infinite cell | ring]; the column-cost table after the
-  // sequences in shared memory, 8 words per (x0, x1, x2), each 0..4
-  uint16_t *const infc = reinterpret_cast<uint16_t *>(ring);
-  uint16_t *const ring16 = infc + kP3States;
-  uint4 *const ctab = reinterpret_cast<uint4 *>(p3_sm + 3 * A.smax);
-  unsigned gg[16];  // packed opening costs of two previous states
-#pragma unroll
-  for (int k = 0; k < 16; ++k) gg[k] = (unsigned)g16[k >> 2] | (unsigned)g16[k & 3] << 16;
-  if (PACKED) {
-    if (lead && tid < 2)
-      reinterpret_cast<uint4 *>(infc)[tid] = make_uint4(kP3Inf2, kP3Inf2, kP3Inf2, kP3Inf2);
-    for (int e = tid; e < 125 * 8; e += kP3Threads) {
-      const int cmb = e >> 3, k = e & 7;
-      const int i0 = cmb / 25, i1 = cmb / 5 % 5, i2 = cmb % 5;
-      reinterpret_cast<unsigned *>(ctab)[e] =
-          p3_col2(k, i0 ? 1 << (i0 - 1) : 0, i1 ? 1 << (i1 - 1) : 0, i2 ? 1 << (i2 - 1) : 0,
-                  16 * A.mm, g16[4]);
-    }
-  }
-  uint64_t *dir = A.dir + slot * A.dir_stride;
+  int32_t *ring = A.ring + blockIdx.x * A.ring_stride;
+  uint64_t *dir = A.dir + blockIdx.x * A.dir_stride;
 
   for (;;) {
-    if (lead && tid == 0) s_job = atomicAdd(A.counter, 1);
-    bar();
-    const int job = CL ? *cg::this_cluster().map_shared_rank(&s_job, 0) : s_job;
-    if (CL) cg::this_cluster().sync();  // every block has read block 0's s_job
-    if (job >= A.n) break;
-    const int i = A.order[job];
+    __syncthreads();
+    if (tid == 0) s_job = atomicAdd(A.counter, 1);
+    __syncthreads();
+    if (s_job >= A.n) break;
+    const int i = A.order[s_job];
     const int la = A.len[0][i], lb = A.len[1][i], lc = A.len[2][i];
-    const int cap = (la + lb + lc + 3) & ~3;
-    uint8_t *o = A.out + A.out_off[i];
-    if (!p3_begin(A, i, lead, tid, kP3Threads,
-                  [&](int q, int x, int c) { sqw[q][x] = (uint8_t)c; })) {
-      bar();
+    if (!p3_begin(A, i, true, tid, kP3Threads,
+                  [&](int q, int x, int c) { sq[q][x] = (uint8_t)c; }))
       continue;
-    }
 
     const int na = la - 1, nb = lb - 1, nc = lc - 1, H = na + nb + nc;
     const int64_t pl = (int64_t)(na + 1) * (nb + 1);  // ring plane (cells)
     const int64_t bcs = (int64_t)(nb + 1) * (nc + 1); // choice-cube i-slice
     for (int h = 0; h <= H; ++h) {
       const int a_lo = max(0, h - nb - nc), a_hi = min(na, h);
-      for (int a = a_lo + rank * kWarps + warp; a <= a_hi; a += kWarps * csz) {  // a warp per row
+      for (int a = a_lo + warp; a <= a_hi; a += kWarps) {  // a warp per row
         const int s = h - a, blo = max(0, s - nc), bhi = min(nb, s);
         const int64_t drow = (int64_t)a * bcs + p3_soff(s, nb, nc) - blo;
-        if (PACKED && h > 0) {
-          // row bases (uint16 units) of the 7 neighbours and of the cell
-          int rb[7];
-#pragma unroll
-          for (int d = 1; d < 8; ++d) {
-            const int da = d & 1, db = d >> 1 & 1, dc = d >> 2 & 1;
-            rb[d - 1] = (((h - da - db - dc) & 3) * (int)pl + (a - da) * (nb + 1) - db) * kP3States;
-          }
-          const int ob = ((h & 3) * (int)pl + a * (nb + 1)) * kP3States;
-          const int i0 = a ? __ffs(sq[0][a]) : 0;
-          for (int b = blo + lane; b <= bhi; b += 32) {
-            const int c = s - b, b16 = b * kP3States;
-            const uint16_t *src[7];
-#pragma unroll
-            for (int d = 1; d < 8; ++d) {
-              const bool ok = (a >= (d & 1)) && (b >= (d >> 1 & 1)) && (c >= (d >> 2 & 1));
-              src[d - 1] = ok ? ring16 + rb[d - 1] + b16 : infc;
-            }
-            const int cmb = (i0 * 5 + (b ? __ffs(sq[1][b]) : 0)) * 5 + (c ? __ffs(sq[2][c]) : 0);
-            dir[drow + b] = p3_cell16<CL>(src, ring16 + ob + b16, gg, ctab[2 * cmb],
-                                           ctab[2 * cmb + 1]);
-          }
-          continue;
-        }
         for (int b = blo + lane; b <= bhi; b += 32) {
           const int c = s - b;
           uint64_t word = 0;
           if (h == 0) {  // the start: MMM at cost 0
-            if (PACKED) {
-              uint4 *r = reinterpret_cast<uint4 *>(ring16);
-              // every value carries its own state number
-              r[0] = make_uint4(0xC0010000u, 0xC003C002u, 0xC005C004u, 0xC007C006u);
-              r[1] = make_uint4(0xC009C008u, 0xC00BC00Au, 0xC00DC00Cu, 0xC00FC00Eu);
-            } else {
-              int4 *r = reinterpret_cast<int4 *>(ring);
-              r[0] = make_int4(0, kP3Inf, kP3Inf, kP3Inf);
-              for (int q = 1; q < 4; ++q) r[q] = make_int4(kP3Inf, kP3Inf, kP3Inf, kP3Inf);
-            }
+            int4 *r = reinterpret_cast<int4 *>(ring);
+            r[0] = make_int4(0, kP3Inf, kP3Inf, kP3Inf);
+            for (int q = 1; q < 4; ++q) r[q] = make_int4(kP3Inf, kP3Inf, kP3Inf, kP3Inf);
           } else {
             // alignmentCost's mismatches (ukkCommon.c:381-389), x16, by the
             // sequences a column consumes: mm per extra distinct character
@@ -317,64 +168,25 @@ __global__ void __launch_bounds__(kP3Threads) k_p3(const __grid_constant__ P3Arg
           dir[drow + b] = word;
         }
       }
-      bar();
+      __syncthreads();
     }
-
-    if (lead && tid == 0) {
-      const int64_t fo = ((int64_t)(H & 3) * pl + (int64_t)na * (nb + 1) + nb) * kP3States;
-      const int inf = PACKED ? 0xC000 : kP3Inf;
-      int best = inf, st = 0;
-      for (int s = 0; s < kP3States; ++s) {
-        const int f = PACKED ? (int)(__ldcg(ring16 + fo + s) & 0xFFF0u) : __ldcg(ring + fo + s);
-        if (f < best) best = f, st = s;
-      }
-      if (PACKED && best >= inf) {  // the optimum reached the clamp: redo in 32 bits
-        if (tid == 0) atomicOr(A.err, 4);
-      }
-      int a = na, b = nb, c = nc, n = 0, nm = 0;
-      bool okw = best < inf;
-      while (okw && (a | b | c)) {
-        const int s = b + c;
-        const uint64_t wd =
-            __ldcg(dir + (int64_t)a * bcs + p3_soff(s, nb, nc) + (b - max(0, s - nc)));
-        const int prev = (int)(wd >> (4 * st) & 15);
-        const int ad = c_p3.adv[st];
-        if ((ad & 1) > a || (ad >> 1 & 1) > b || (ad >> 2 & 1) > c) {
-          okw = false;  // cannot happen for a finite optimum; kept as a guard
-          break;
+    if (warp == 0) {
+      const int32_t *f = ring + ((int64_t)(H & 3) * pl + (int64_t)na * (nb + 1) + nb) * kP3States;
+      int best = kP3Inf, st = 0;
+      for (int s = 0; s < kP3States; ++s)
+        if (f[s] < best) best = f[s], st = s;
+      auto nib = [&](int x, int y, int z, int t) -> int {
+        const int s = y + z;
+        return (int)(dir[(int64_t)x * bcs + p3_soff(s, nb, nc) + (y - max(0, s - nc))] >> (4 * t)) & 15;
+      };
+      if (best >= kP3Inf || !p3_walk_choices(A, c_p3, i, lane, best >> 4, st, nib)) {
+        if (lane == 0) {  // cannot happen for a finite optimum; kept as a guard
+          atomicOr(A.err, 2);
+          A.cost[i] = A.out_len[2 * i] = A.out_len[2 * i + 1] = -1;
+          if (A.mode == 1) A.changed[i] = 1;
         }
-        const int ca = (ad & 1) ? sq[0][a] : 16, cb = (ad & 2) ? sq[1][b] : 16,
-                  cc = (ad & 4) ? sq[2][c] : 16;
-        ++n;
-        o[cap - n] = (uint8_t)ca;
-        o[2 * cap - n] = (uint8_t)cb;
-        o[3 * cap - n] = (uint8_t)cc;
-        const int md = A.med[25 * p3_ix(ca) + 5 * p3_ix(cb) + p3_ix(cc)];
-        if (A.has_med && md != A.gap) o[4 * cap - ++nm] = (uint8_t)md;
-        a -= ad & 1;
-        b -= ad >> 1 & 1;
-        c -= ad >> 2 & 1;
-        st = prev;
-      }
-      ++n;  // the leading gap column (printTraceBack, ukk.checkp.c)
-      o[cap - n] = o[2 * cap - n] = o[3 * cap - n] = 16;
-      if (A.has_med) o[4 * cap - ++nm] = (uint8_t)A.gap;
-      if (!okw) {
-        if (!PACKED) atomicOr(A.err, 2);
-        n = nm = -1;
-      }
-      A.cost[i] = okw ? best >> 4 : -1;
-      A.out_len[2 * i] = n;
-      A.out_len[2 * i + 1] = A.has_med ? nm : 0;
-      if (A.mode == 1) {
-        const int lm = A.len[3][i];
-        const uint8_t *m = A.seq + A.off[3][i];
-        bool diff = nm != lm;
-        for (int x = 0; !diff && x < lm; ++x) diff = o[4 * cap - nm + x] != m[x];
-        A.changed[i] = diff ? 1 : 0;
       }
     }
-    bar();
   }
 }
 
@@ -399,7 +211,8 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   }
   CK3(cudaStreamSynchronize(st));
   int64_t ring_max = 0, dir_max = 0, lin_plane = 0, lin_dir = 0;
-  int smax = 16;
+  int64_t open_plane = 0, open_dir = 0;
+  int smax = 16, max_b = 1;
   std::vector<int64_t> work(n);
   const int64_t step_max = 2LL * go + 2LL * ge + 2LL * mm;
   for (int32_t i = 0; i < n; ++i) {
@@ -417,6 +230,10 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     const P3LinearPlan lp = p3_linear_plan(la, lb, lc);
     lin_plane = std::max(lin_plane, lp.plane);
     lin_dir = std::max(lin_dir, lp.dir);
+    const P3OpenPlan op = p3_open_plan(la, lb, lc);
+    open_plane = std::max(open_plane, op.plane);
+    open_dir = std::max(open_dir, op.dir);
+    max_b = std::max(max_b, (int)lb);
   }
   const int longest = smax;
   smax = (smax + 15) & ~15;
@@ -492,7 +309,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   // 16-bit halves while every addend of a half stays below 0x4000
   // (openings, column costs)
   const char *pk = getenv("POYD_P3_PACKED");
-  bool packed = !(pk && pk[0] == '0') && 48LL * go + 15 < 0x4000 &&
+  const bool packed = !(pk && pk[0] == '0') && 48LL * go + 15 < 0x4000 &&
                 16LL * (2LL * mm + 3LL * ge) < 0x4000;
   if (packed && go == 0) {
     // Warps per triple: consecutive strips run kP3LinLag steps apart, so a
@@ -514,66 +331,43 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     bool redo = false;
     rc = finish(&redo);
     if (rc || !redo) return rc;
-    packed = false;
+  } else if (packed) {
+    // Small batches take a cluster of blocks per triple: a triple feeds
+    // (strips of b) x (steps of a task / the rows' lag) warps.  Two blocks an
+    // SM at most (POYD_P3_CLUSTER=0: one block per triple).
+    const int64_t useful = (int64_t)((max_b + 31) / 32) * ((longest + 40) / 24 + 1);
+    int csize = 1;
+    const char *ce = getenv("POYD_P3_CLUSTER");
+    if (!(ce && ce[0] == '0'))
+      while (csize < 8 && (int64_t)csize * p3_open_warps() < useful && (int64_t)n * csize <= sms) csize *= 2;
+    const int64_t per = open_plane + open_dir;
+    int blocks = (int)std::min<int64_t>({(int64_t)n, 2LL * sms, std::max<int64_t>(1, budget / per)});
+    uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(open_plane * blocks));
+    uint8_t *dirb = (uint8_t *)ws_buffer(w, WS_P3_DIR, (size_t)(open_dir * blocks));
+    if (!plane || !dirb) return fail(POYD_ENOMEM, "three-sequence workspace (%d blocks)", blocks);
+    // a sum of an opened value and a column cost may pass 16 bits: cut it off
+    const bool clamp = 48LL * go + 16LL * (2LL * mm + 3LL * ge) + 31 >= 0x4000;
+    int rc = launch_p3_open(A, clamp, longest, blocks, csize, plane, open_plane, dirb, open_dir, st);
+    if (rc) return rc;
+    bool redo = false;
+    rc = finish(&redo);
+    if (rc || !redo) return rc;
   }
   const int64_t per_block = ring_max * 4 + dir_max * 8;
-  int64_t blocks = std::min<int64_t>({(int64_t)n, 3LL * sms, std::max<int64_t>(1, budget / per_block)});
+  const int64_t blocks = std::min<int64_t>({(int64_t)n, 3LL * sms, std::max<int64_t>(1, budget / per_block)});
   A.ring = (int32_t *)ws_buffer(w, WS_P3_RING, (size_t)(ring_max * 4 * blocks));
   A.dir = (uint64_t *)ws_buffer(w, WS_P3_DIR, (size_t)(dir_max * 8 * blocks));
   if (!A.ring || !A.dir)
     return fail(POYD_ENOMEM, "three-sequence workspace (%lld blocks)", (long long)blocks);
   A.ring_stride = ring_max;
   A.dir_stride = dir_max;
-  const size_t smem = 3 * (size_t)smax + 125 * 8 * sizeof(unsigned);
-  // small batches: a cluster of up to 8 blocks per triple, so that the
-  // batch still covers the SMs (POYD_P3_CLUSTER=0: one block per triple)
-  int csize = 1;
+  const size_t smem = 3 * (size_t)smax;
   {
-    const char *ce = getenv("POYD_P3_CLUSTER");
-    const int64_t want = 3LL * sms / std::max<int64_t>(blocks, 1);
-    if (!(ce && ce[0] == '0'))
-      while (csize < 8 && 2 * csize <= want) csize *= 2;
+    ProfScope ps("p3", st);
+    k_p3<<<(unsigned)blocks, kP3Threads, smem, st>>>(A);
   }
-  for (;;) {
-    auto kern = packed ? k_p3<true, false> : k_p3<false, false>;
-    auto kcl = k_p3<true, true>;
-    bool launched = false;
-    if (packed && csize > 1) {
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = (unsigned)csize;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3((unsigned)(blocks * csize));
-      cfg.blockDim = dim3(kP3Threads);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = st;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      if (smem > 48 * 1024)
-        CK3(cudaFuncSetAttribute(kcl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      int ncl = 0;
-      if (cudaOccupancyMaxActiveClusters(&ncl, kcl, &cfg) == cudaSuccess && ncl > 0) {
-        ProfScope ps("p3", st);
-        CK3(cudaLaunchKernelEx(&cfg, kcl, A));
-        launched = true;
-      } else {
-        cudaGetLastError();
-        csize = 1;
-      }
-    }
-    if (!launched) {
-      if (smem > 48 * 1024)
-        CK3(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      ProfScope ps("p3", st);
-      kern<<<(unsigned)blocks, kP3Threads, smem, st>>>(A);
-    }
-    bool redo = false;
-    const int rc = finish(&redo);
-    if (rc || !redo) return rc;
-    packed = false;
-  }
+  bool redo = false;
+  return finish(&redo);
 }
 
 // Cost_matrix.Three_D.of_two_dim_comb (cost_matrix.ml:803-851): the median

@@ -148,38 +148,30 @@ __device__ __forceinline__ int p3_col(const P3States &S, const P3Args &A, int t,
   return A.mm * (__popc(ch) - 1) + S.ndel[t] * A.ge;
 }
 
-// The alignment of triple i walked back by one warp.  nib(a, b, c, st) is the
-// choice stored for a cell: for the zero-opening kernel the cell's own best
-// state.  Most columns are MMM, so lane k reads the cell k columns up the
-// diagonal; the run up to the first other state and that state's column are
-// taken at once.  Writes the slot, lengths, cost and changed flag; returns
-// false when the path left the cube or its cost is not exact (>= most).
-template <class Nib>
-__device__ __forceinline__ bool p3_walk_states(const P3Args &A, const P3States &S, int i, int lane,
-                                               int most, Nib nib) {
-  const int la = A.len[0][i], lb = A.len[1][i], lc = A.len[2][i];
-  const uint8_t *s0 = A.seq + A.off[0][i], *s1 = A.seq + A.off[1][i], *s2 = A.seq + A.off[2][i];
-  const int cap = (la + lb + lc + 3) & ~3;
-  uint8_t *o = A.out + A.out_off[i];
-  int a = la - 1, b = lb - 1, c = lc - 1, n = 0, nm = 0, cost = 0;
-  while (a | b | c) {
-    const int x = a - lane, y = b - lane, z = c - lane;
-    const bool in = x >= 0 && y >= 0 && z >= 0 && (x | y | z);
-    const int st = in ? nib(x, y, z) : 0;
-    // a state this cell cannot be in ends the walk (the path is not exact)
-    const int ad = S.adv[st];
-    const bool ok = in && !((ad & 1) > x || (ad >> 1 & 1) > y || (ad >> 2 & 1) > z);
-    const unsigned stop = __ballot_sync(0xffffffffu, !in || !ok || st != 0);
-    const int f = stop ? __ffs(stop) - 1 : 32;  // lanes below f: MMM columns
-    const unsigned good = __ballot_sync(0xffffffffu, ok);
-    const bool step_f = f < 32 && (good >> (f & 31) & 1);
-    const int in_f = __shfl_sync(0xffffffffu, (int)in, f & 31);
-    if (f < 32 && !step_f && (f == 0 || in_f)) return false;
-    const bool writes = lane < f || (lane == f && step_f);
+// The outputs of one triple written from the end by one warp, 32 columns at a
+// time: the walk tells which columns, this writes them.
+struct P3Writer {
+  const P3Args &A;
+  const P3States &S;
+  int i, lane, cap;
+  const uint8_t *sq[3];
+  uint8_t *o;
+  int n, nm, cost;
+
+  __device__ __forceinline__ P3Writer(const P3Args &A_, const P3States &S_, int i_, int lane_)
+      : A(A_), S(S_), i(i_), lane(lane_), n(0), nm(0), cost(0) {
+    for (int q = 0; q < 3; ++q) sq[q] = A.seq + A.off[q][i];
+    cap = (A.len[0][i] + A.len[1][i] + A.len[2][i] + 3) & ~3;
+    o = A.out + A.out_off[i];
+  }
+  // column n + lane of cell (x, y, z) in state st on the lanes with `writes`
+  // (lanes 0 .. count - 1)
+  __device__ __forceinline__ void put(bool writes, int count, int st, int x, int y, int z) {
     int md = A.gap, col = 0;
     if (writes) {
-      const int ca = (ad & 1) ? p3_code(s0[x]) : 16, cb = (ad & 2) ? p3_code(s1[y]) : 16,
-                cc = (ad & 4) ? p3_code(s2[z]) : 16;
+      const int ad = S.adv[st];
+      const int ca = (ad & 1) ? p3_code(sq[0][x]) : 16, cb = (ad & 2) ? p3_code(sq[1][y]) : 16,
+                cc = (ad & 4) ? p3_code(sq[2][z]) : 16;
       col = p3_col(S, A, st, ca, cb, cc);
       md = A.med[25 * p3_ix(ca) + 5 * p3_ix(cb) + p3_ix(cc)];
       const int p = cap - 1 - (n + lane);
@@ -191,37 +183,104 @@ __device__ __forceinline__ bool p3_walk_states(const P3Args &A, const P3States &
     const unsigned kb = __ballot_sync(0xffffffffu, keep);
     if (keep) o[4 * cap - 1 - (nm + __popc(kb & ((1u << lane) - 1u)))] = (uint8_t)md;
     cost += __reduce_add_sync(0xffffffffu, col);
-    const int ad_f = __shfl_sync(0xffffffffu, ad, f & 31);
-    n += f + step_f;
+    n += count;
     nm += __popc(kb);
-    a -= f + (step_f ? ad_f & 1 : 0);
-    b -= f + (step_f ? ad_f >> 1 & 1 : 0);
-    c -= f + (step_f ? ad_f >> 2 & 1 : 0);
   }
-  if (cost >= most) return false;
-  __syncwarp();
-  ++n;  // the leading gap column (printTraceBack, ukk.checkp.c)
-  if (lane == 0) {
-    o[cap - n] = o[2 * cap - n] = o[3 * cap - n] = 16;
-    if (A.has_med) o[4 * cap - 1 - nm] = (uint8_t)A.gap;
+  // the leading gap column (printTraceBack, ukk.checkp.c), lengths, cost and
+  // changed flag
+  __device__ __forceinline__ void finish(int total) {
+    ++n;
+    if (lane == 0) {
+      o[cap - n] = o[2 * cap - n] = o[3 * cap - n] = 16;
+      if (A.has_med) o[4 * cap - 1 - nm] = (uint8_t)A.gap;
+    }
+    if (A.has_med) ++nm;
+    __syncwarp();
+    bool diff = false;
+    if (A.mode == 1) {
+      const int lm = A.len[3][i];
+      const uint8_t *m = A.seq + A.off[3][i];
+      diff = nm != lm;
+      if (!diff)
+        for (int x = lane; x < lm; x += 32) diff |= o[4 * cap - nm + x] != m[x];
+      diff = __any_sync(0xffffffffu, diff);
+    }
+    if (lane == 0) {
+      A.cost[i] = total;
+      A.out_len[2 * i] = n;
+      A.out_len[2 * i + 1] = A.has_med ? nm : 0;
+      if (A.mode == 1) A.changed[i] = diff ? 1 : 0;
+    }
   }
-  if (A.has_med) ++nm;
-  __syncwarp();
-  bool diff = false;
-  if (A.mode == 1) {
-    const int lm = A.len[3][i];
-    const uint8_t *m = A.seq + A.off[3][i];
-    diff = nm != lm;
-    if (!diff)
-      for (int x = lane; x < lm; x += 32) diff |= o[4 * cap - nm + x] != m[x];
-    diff = __any_sync(0xffffffffu, diff);
+};
+
+// The walk of the zero-opening kernel, by one warp: nib(a, b, c) is a cell's
+// own best state.  Most columns are MMM, so lane k reads the cell k columns up
+// the diagonal; the run up to the first other state and that state's column
+// are taken at once.  Returns false when the path left the cube or its cost
+// is not exact (>= most).
+template <class Nib>
+__device__ __forceinline__ bool p3_walk_states(const P3Args &A, const P3States &S, int i, int lane,
+                                               int most, Nib nib) {
+  P3Writer w(A, S, i, lane);
+  int a = A.len[0][i] - 1, b = A.len[1][i] - 1, c = A.len[2][i] - 1;
+  while (a | b | c) {
+    const int x = a - lane, y = b - lane, z = c - lane;
+    const bool in = x >= 0 && y >= 0 && z >= 0 && (x | y | z);
+    const int st = in ? nib(x, y, z) : 0;
+    // a state this cell cannot be in ends the walk (the path is not exact)
+    const int ad = S.adv[st];
+    const bool ok = in && !((ad & 1) > x || (ad >> 1 & 1) > y || (ad >> 2 & 1) > z);
+    const unsigned stop = __ballot_sync(0xffffffffu, !ok || st != 0);
+    const int f = stop ? __ffs(stop) - 1 : 32;  // lanes below f: MMM columns
+    const bool step_f = f < 32 && (__ballot_sync(0xffffffffu, ok) >> (f & 31) & 1);
+    const int in_f = __shfl_sync(0xffffffffu, (int)in, f & 31);
+    if (f < 32 && !step_f && (f == 0 || in_f)) return false;
+    const int ad_f = step_f ? __shfl_sync(0xffffffffu, ad, f & 31) : 0;
+    w.put(lane < f + step_f, f + step_f, st, x, y, z);
+    a -= f + (ad_f & 1);
+    b -= f + (ad_f >> 1 & 1);
+    c -= f + (ad_f >> 2 & 1);
   }
-  if (lane == 0) {
-    A.cost[i] = cost;
-    A.out_len[2 * i] = n;
-    A.out_len[2 * i + 1] = A.has_med ? nm : 0;
-    if (A.mode == 1) A.changed[i] = diff ? 1 : 0;
+  if (w.cost >= most) return false;
+  w.finish(w.cost);
+  return true;
+}
+
+// The walk of the kernels with openings: nib(a, b, c, st) is the state before
+// a column in state st at the cell; the walk starts in state st with the
+// optimum `total`.  A run of MMM columns ends after the one whose previous
+// state is another.
+template <class Nib>
+__device__ __forceinline__ bool p3_walk_choices(const P3Args &A, const P3States &S, int i, int lane,
+                                                int total, int st, Nib nib) {
+  P3Writer w(A, S, i, lane);
+  int a = A.len[0][i] - 1, b = A.len[1][i] - 1, c = A.len[2][i] - 1;
+  while (a | b | c) {
+    const int ad = S.adv[st];
+    if ((ad & 1) > a || (ad >> 1 & 1) > b || (ad >> 2 & 1) > c) return false;
+    if (st != 0) {
+      const int prev = nib(a, b, c, st);
+      w.put(lane == 0, 1, st, a, b, c);
+      a -= ad & 1;
+      b -= ad >> 1 & 1;
+      c -= ad >> 2 & 1;
+      st = prev;
+      continue;
+    }
+    const int x = a - lane, y = b - lane, z = c - lane;
+    const bool in = x > 0 && y > 0 && z > 0;
+    const int prev = in ? nib(x, y, z, 0) : 0;
+    const unsigned stop = __ballot_sync(0xffffffffu, !in || prev != 0);
+    const int f = stop ? __ffs(stop) - 1 : 32;
+    const bool step_f = f < 32 && (__ballot_sync(0xffffffffu, in) >> (f & 31) & 1);
+    st = step_f ? __shfl_sync(0xffffffffu, prev, f & 31) : 0;
+    w.put(lane < f + step_f, f + step_f, 0, x, y, z);
+    a -= f + step_f;
+    b -= f + step_f;
+    c -= f + step_f;
   }
+  w.finish(total);
   return true;
 }
 
@@ -236,5 +295,15 @@ int p3_linear_blocks(int warps, int longest);  // resident blocks of the device
 int launch_p3_linear(const P3Args &A, int warps, int longest, int blocks, uint8_t *plane,
                      int64_t plane_stride, uint8_t *dir, int64_t dir_stride, cudaStream_t st);
 constexpr int kP3LinLag = 48;  // steps between consecutive strips
+
+// The 16-bit kernel with openings (three_open.cu): scratch bytes per triple in
+// flight, warps of a block, and the launch of `blocks` clusters of csize.
+struct P3OpenPlan {
+  int64_t plane, dir;
+};
+P3OpenPlan p3_open_plan(int64_t la, int64_t lb, int64_t lc);
+int p3_open_warps();
+int launch_p3_open(const P3Args &A, bool clamp, int longest, int blocks, int csize, uint8_t *plane,
+                   int64_t plane_stride, uint8_t *dir, int64_t dir_stride, cudaStream_t st);
 
 }  // namespace poyd
