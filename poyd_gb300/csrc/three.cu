@@ -332,14 +332,17 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     rc = finish(&redo);
     if (rc || !redo) return rc;
   } else if (packed) {
-    // Small batches take a cluster of blocks per triple: a triple feeds
-    // (strips of b) x (steps of a task / the rows' lag) warps.  Two blocks an
-    // SM at most (POYD_P3_CLUSTER=0: one block per triple).
-    const int64_t useful = (int64_t)((max_b + 31) / 32) * ((longest + 40) / 24 + 1);
-    int csize = 1;
+    // Small batches take a cluster of blocks per triple, an SM each: a triple
+    // feeds (strips of b) x (steps of a task / the rows' lag) warps.  The
+    // largest size of which the whole batch is resident at once (a cluster
+    // sits in one GPC, whose SMs a size may not divide: 20 clusters of 6 ran
+    // in two waves, 2.5 ms against 1.6 for one wave).
+    // POYD_P3_CLUSTER=0: one block per triple.
+    const int64_t useful = (int64_t)((max_b + 31) / 32) * ((longest + 40) / 32 + 1);
     const char *ce = getenv("POYD_P3_CLUSTER");
-    if (!(ce && ce[0] == '0'))
-      while (csize < 8 && (int64_t)csize * p3_open_warps() < useful && (int64_t)n * csize <= sms) csize *= 2;
+    int csize = ce && ce[0] == '0' ? 1 : (int)std::min<int64_t>(
+        {8, (useful + p3_open_warps() - 1) / p3_open_warps(), std::max<int64_t>(1, sms / n)});
+    while (csize > 1 && p3_open_clusters(csize) < n) --csize;
     const int64_t per = open_plane + open_dir;
     int blocks = (int)std::min<int64_t>({(int64_t)n, 2LL * sms, std::max<int64_t>(1, budget / per)});
     uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(open_plane * blocks));

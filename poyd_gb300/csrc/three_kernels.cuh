@@ -303,6 +303,7 @@ struct P3OpenPlan {
 };
 P3OpenPlan p3_open_plan(int64_t la, int64_t lb, int64_t lc);
 int p3_open_warps();
+int p3_open_clusters(int csize);  // clusters of csize blocks the device holds at once
 int launch_p3_open(const P3Args &A, bool clamp, int longest, int blocks, int csize, uint8_t *plane,
                    int64_t plane_stride, uint8_t *dir, int64_t dir_stride, cudaStream_t st);
 

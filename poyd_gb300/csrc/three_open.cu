@@ -15,9 +15,11 @@
 // Costs, choices and ties are those of the 32-bit kernel (k_p3), which takes
 // batches whose values may not fit.
 //
-// Bound: integer issue, ~100 instructions a cell.  Measured (20 triples of
-// 150-200 bp): 15.1 ms with 16 x 16 state pairs and a cluster barrier per
-// hyperplane; see the launch for the figures here.
+// Bound: integer issue (~130 instructions a cell, most on the half-rate ALU
+// pipe), and for small batches the barriers.  Measured (20 triples of 150-200
+// bp): 15 ms with 16 x 16 state pairs and a cluster barrier per hyperplane,
+// 1.8 ms here with clusters of 6 blocks (8.9 ms with one block a triple, 2.3
+// with clusters of 8, which do not all fit at once).
 //
 // Layout.  A warp takes two rows of sequence a by 32 of b (a task) and
 // marches along c, lane k one column behind lane k - 1; a thread's registers
@@ -26,15 +28,16 @@
 // seven shuffles; a-neighbours from the task two rows up, through a ring in
 // global memory (16 bytes per lane and step); the b-neighbour of lane 0 from
 // the task to its left, through a 32-byte record per step.  Both are brought
-// into shared memory 8 steps ahead with cp.async.  Tasks start kOpenLagA = 24
-// steps after the one above (8 of prefetch, 8 between barriers, one for the
-// second row, rounded up to 8) and kOpenLagB = 48 after the one to the left
-// (31 lanes more); a barrier every 8 steps orders them.  The warps of a block,
-// or of a cluster of blocks when the batch is small, take the tasks round
-// robin; a b longer than the warps' strips runs in panels.
+// into shared memory 8 steps ahead with cp.async.  Tasks start kOpenLagA = 32
+// steps after the one above (8 of prefetch, 16 until a chunk's stores are
+// visible, one for the second row, rounded up to 8) and kOpenLagB = 56 after
+// the one to the left (31 lanes more); a barrier every 8 steps orders them.
+// The warps of a block, or of a cluster of blocks when the batch is small,
+// take the tasks round robin; a b longer than the warps' strips runs in panels.
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include "three_kernels.cuh"
 
 namespace poyd {
@@ -45,7 +48,7 @@ __constant__ P3States c_p3o = p3_states();
 constexpr unsigned kOInf2 = 0xC000C000u;
 constexpr unsigned kOClear = 0xFFF0FFF0u;
 constexpr int kOpenWarps = 8;
-constexpr int kOpenLagA = 24, kOpenLagB = 48, kOpenRing = 3;
+constexpr int kOpenLagA = 32, kOpenLagB = 56, kOpenRing = 3;
 
 struct OpenArgs {
   P3Args A;
@@ -53,6 +56,7 @@ struct OpenArgs {
   int64_t plane_stride;
   uint8_t *dir;
   int64_t dir_stride;
+  unsigned one, sixteen, m1;  // multipliers the compiler does not know: 1, 16, -1
 };
 
 // The states of one advance d (bits: the sequences), in increasing order.
@@ -71,6 +75,12 @@ __device__ __forceinline__ unsigned o_prmt(unsigned a, unsigned b, unsigned s) {
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
   return d;
 }
+// An add kept on the multiply-add pipe: the ALU pipe is the busier one.
+__device__ __forceinline__ unsigned o_mad(unsigned a, unsigned b, unsigned c) {
+  unsigned d;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
 __device__ __forceinline__ void o_cp16(uint32_t dst, const void *src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
                : "memory");
@@ -79,7 +89,7 @@ __device__ __forceinline__ void o_cp16(uint32_t dst, const void *src, bool ok) {
 // One sequence's pass of T (stride 1, 3 or 9 in the 27 combinations of M, D,
 // I); h: which combinations hold a value.
 template <int ST>
-__device__ __forceinline__ void o_pass(unsigned (&x)[27], bool (&h)[27], unsigned go2) {
+__device__ __forceinline__ void o_pass(unsigned (&x)[27], bool (&h)[27], unsigned go2, unsigned one) {
 #pragma unroll
   for (int e = 0; e < 27; ++e) {
     if (e / ST % 3 != 0) continue;
@@ -88,8 +98,8 @@ __device__ __forceinline__ void o_pass(unsigned (&x)[27], bool (&h)[27], unsigne
     unsigned m = h[M] ? x[M] : h[D] ? x[D] : x[I];
     if (h[M] && h[D]) m = __vminu2(m, x[D]);
     if ((h[M] || h[D]) && h[I]) m = __vminu2(m, x[I]);
-    x[D] = h[D] ? __viaddmin_u16x2(m, go2, x[D]) : m + go2;
-    x[I] = h[I] ? __viaddmin_u16x2(m, go2, x[I]) : m + go2;
+    x[D] = h[D] ? __viaddmin_u16x2(m, go2, x[D]) : o_mad(m, one, go2);
+    x[I] = h[I] ? __viaddmin_u16x2(m, go2, x[I]) : o_mad(m, one, go2);
     x[M] = m;
     h[M] = h[D] = h[I] = true;
   }
@@ -186,8 +196,11 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
               plane + ((int64_t)((ra + kOpenRing - 1) % kOpenRing) * NP + vin) * row_bytes + lane * 16;
 #pragma unroll
           for (int u = 0; u < 8; ++u) {  // the row above at this lane's column: one step later there
-            const bool ok = ra > 0 && s + u + 1 < NS;
-            o_cp16(st_row_a + ((par * 8 + u) * 32 + lane) * 16, p + (ok ? (int64_t)(s + u + 1) * 512 : 0), ok);
+            const bool ok = s + u + 1 < NS;  // else past its last column
+            if (ra > 0)
+              o_cp16(st_row_a + ((par * 8 + u) * 32 + lane) * 16, p + (ok ? (int64_t)(s + u + 1) * 512 : 0), ok);
+            else
+              st_row[(par * 8 + u) * 32 + lane] = make_uint4(kOInf2, kOInf2, kOInf2, kOInf2);
           }
           if (v > 0 && lane < 16) {
             const int sp = s + (lane >> 1) + 31;
@@ -211,7 +224,16 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
       }
       for (int T = 0; T < dur; T += 8, par ^= 1) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        bar();
+        // a cluster's barrier is in two halves, a chunk apart: what chunk
+        // q - 2 wrote is visible in chunk q, and nobody waits for the stores
+        // of the chunk just done
+        if (CL) {
+          __syncwarp();
+          if (T) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+          asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        } else {
+          __syncthreads();
+        }
         {
           int s = 0;
           const int ra = task_at(T + 8, s);
@@ -244,11 +266,9 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
         const int cap = ra == e_ra && v == e_v && lane == (nb & 31) ? e_s - s : -1;
 #pragma unroll 4
         for (int u = 0; u < 8; ++u) {
-          // boundary words are stored xor infinity: zero-filled is infinite
-          uint4 rw = in_row[u * 32];
+          const uint4 rw = in_row[u * 32];
           const uint4 c0 = in_cor[2 * u], c1 = in_cor[2 * u + 1];
           const unsigned sl = selp[u];
-          rw.x ^= kOInf2, rw.y ^= kOInf2, rw.z ^= kOInf2, rw.w ^= kOInf2;
           unsigned X[kP3States];  // T of the cell each state comes from
           // c alone: this cell one column back
 #pragma unroll
@@ -280,16 +300,21 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
           X[R.t[5][0]] = U5;
           U5 = o_prmt(rw.z, Tp[R.t[5][0]], 0x5410);
           U3 = o_prmt(rw.z, Tp[R.t[3][0]], 0x5432);
-          U7 = o_prmt(rw.w, Tp[R.t[7][0]], 0x5410);
+          U7 = o_prmt(rw.w, Tp[R.t[7][0]], 0x5432);
           // the choices, four states a word (a nibble per half and state)
           uint4 w;
           unsigned *wp = &w.x;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            unsigned z = X[4 * k + 3] & ~kOClear;
+            // sum of 16^q (X - X cleared), all multiply-adds (the ALU pipe is
+            // the busier one); the true sum fits, whatever wraps on the way
+            unsigned z = X[4 * k + 3], c = X[4 * k + 3] & kOClear;
 #pragma unroll
-            for (int q = 2; q >= 0; --q) z = z * 16 + (X[4 * k + q] & ~kOClear);
-            wp[k] = z;
+            for (int q = 2; q >= 0; --q) {
+              z = o_mad(z, B.sixteen, X[4 * k + q]);
+              c = o_mad(c, B.sixteen, X[4 * k + q] & kOClear);
+            }
+            wp[k] = o_mad(c, B.m1, z);
           }
           dw[u * 32] = w;
           // column costs: one extension per D, one for an I; mismatches of the
@@ -303,28 +328,27 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
           for (int t = 0; t < kP3States; ++t) {
             const unsigned own = (unsigned)t * 0x10001u;
             unsigned col = S.ins[t] ? ge2 : S.ndel[t] == 2 ? 2 * ge2 : S.ndel[t] == 1 ? ge2 : 0u;
-            if (S.adv[t] == 3) col += n01;
-            if (S.adv[t] == 5) col += n5 & mm2;
-            if (S.adv[t] == 6) col += n6 & mm2;
-            if (S.adv[t] == 7) col += n01 + (n5 & n6 & mm2);
+            if (S.adv[t] == 3) col = o_mad(n01, B.one, col);
+            if (S.adv[t] == 5) col = o_mad(n5 & mm2, B.one, col);
+            if (S.adv[t] == 6) col = o_mad(n6 & mm2, B.one, col);
+            if (S.adv[t] == 7) col = o_mad(n01, B.one, n5 & n6 & mm2);
             unsigned c = X[t] & kOClear;
             if (CLAMP) c = __vminu2(c, kOInf2);
-            unsigned val = __viaddmin_u16x2(c, col + own, kOInf2 + own);
+            unsigned val = __viaddmin_u16x2(c, o_mad(col, B.one, own), kOInf2 + own);
             if (t == 0 && start && u == 0) val &= 0xFFFF0000u;  // MMM at cost 0
             x[S.code[t]] = val;
             h[S.code[t]] = true;
           }
-          o_pass<1>(x, h, go2);
-          o_pass<3>(x, h, go2);
-          o_pass<9>(x, h, go2);
+          o_pass<1>(x, h, go2, B.one);
+          o_pass<3>(x, h, go2, B.one);
+          o_pass<9>(x, h, go2, B.one);
 #pragma unroll
           for (int t = 0; t < kP3States; ++t) Tp[t] = x[S.code[t]];
           if (u == cap) endv = Tp[0];  // MMM opens nothing: the cell's least state
           row_out[(s + u) * 32] =
-              make_uint4(o_prmt(Tp[R.t[1][0]], Tp[R.t[1][1]], 0x7632) ^ kOInf2,
-                         o_prmt(Tp[R.t[1][2]], Tp[R.t[1][3]], 0x7632) ^ kOInf2,
-                         o_prmt(Tp[R.t[5][0]], Tp[R.t[3][0]], 0x7632) ^ kOInf2,
-                         (Tp[R.t[7][0]] >> 16) ^ kOInf2);
+              make_uint4(o_prmt(Tp[R.t[1][0]], Tp[R.t[1][1]], 0x7632),
+                         o_prmt(Tp[R.t[1][2]], Tp[R.t[1][3]], 0x7632),
+                         o_prmt(Tp[R.t[5][0]], Tp[R.t[3][0]], 0x7632), Tp[R.t[7][0]]);
           if (lane == 31) {
             left_out[2 * (s + u)] = make_uint4(Tp[R.t[2][0]], Tp[R.t[2][1]], Tp[R.t[2][2]], Tp[R.t[2][3]]);
             left_out[2 * (s + u) + 1] = make_uint4(Tp[R.t[6][0]], U3, U7, 0);
@@ -336,6 +360,7 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
         }
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (CL) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     bar();
     if (rank == 0 && warp == 0) {
@@ -368,26 +393,60 @@ P3OpenPlan p3_open_plan(int64_t la, int64_t lb, int64_t lc) {
 
 int p3_open_warps() { return kOpenWarps; }
 
-int launch_p3_open(const P3Args &A, bool clamp, int longest, int blocks, int csize, uint8_t *plane,
-                   int64_t plane_stride, uint8_t *dir, int64_t dir_stride, cudaStream_t st) {
-  const OpenArgs B = {A, plane, plane_stride, dir, dir_stride};
-  const size_t sm = open_smem(longest);
+namespace {
+
+// A cluster's blocks get an SM each: two on one would halve its issue rate.
+// (The request is the same for every length the entry points take.)
+constexpr size_t kOpenClusterSmem = 116 * 1024;
+
+cudaLaunchConfig_t open_config(int blocks, int csize, int longest, cudaLaunchAttribute *at,
+                               cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)csize;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)csize;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
   cfg.gridDim = dim3((unsigned)(blocks * csize));
   cfg.blockDim = dim3(32 * kOpenWarps);
-  cfg.dynamicSmemBytes = sm;
+  cfg.dynamicSmemBytes = csize > 1 ? kOpenClusterSmem : open_smem(longest);
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = csize > 1 ? 1 : 0;
+  return cfg;
+}
+
+}  // namespace
+
+int p3_open_clusters(int csize) {
+  static std::atomic<int> cache[64][9];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<int> &c = cache[dev & 63][csize];
+  if (c.load() == 0) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = open_config(1, csize, 1, &at, nullptr);
+    int n = 0;
+    if (cudaFuncSetAttribute(k_p3_open<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, k_p3_open<true, false>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    c.store(n > 0 ? n : -1);
+  }
+  return std::max(c.load(), 0);
+}
+
+int launch_p3_open(const P3Args &A, bool clamp, int longest, int blocks, int csize, uint8_t *plane,
+                   int64_t plane_stride, uint8_t *dir, int64_t dir_stride, cudaStream_t st) {
+  const OpenArgs B = {A, plane, plane_stride, dir, dir_stride, 1u, 16u, ~0u};
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = open_config(blocks, csize, longest, &at, st);
   auto kern = csize > 1 ? (clamp ? k_p3_open<true, true> : k_p3_open<true, false>)
                         : (clamp ? k_p3_open<false, true> : k_p3_open<false, false>);
   cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)cfg.dynamicSmemBytes);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_p3_open)");
   ProfScope ps("p3", st);
   e = cudaLaunchKernelEx(&cfg, kern, B);
