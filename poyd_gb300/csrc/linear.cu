@@ -807,35 +807,37 @@ __global__ void __launch_bounds__(1024) k_order_small(int n, const LinPlan *plan
                                                       LinOrderScratch *os, int *counter,
                                                       int *batch_done, int nbatch) {
   __shared__ unsigned long long part[32];
-  __shared__ int wmax[32];
+  __shared__ int wmax[32], smax[32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const unsigned long long w = t < n ? (unsigned long long)dm_words[t] : 0ull;
-  int wd = t < n ? plans[t].wd : 0;
+  int wd = t < n ? plans[t].wd : 0, sum = t < n ? plans[t].l1 + plans[t].l2 : 0;
   unsigned long long incl = w;
   for (int d = 1; d < 32; d <<= 1) {
     const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, d);
     if (lane >= d) incl += x;
   }
-  for (int d = 16; d > 0; d >>= 1) wd = max(wd, __shfl_xor_sync(0xffffffffu, wd, d));
+  wd = __reduce_max_sync(0xffffffffu, wd);
+  sum = __reduce_max_sync(0xffffffffu, sum);
   if (lane == 31) part[warp] = incl;
-  if (lane == 0) wmax[warp] = wd;
+  if (lane == 0) wmax[warp] = wd, smax[warp] = sum;
   __syncthreads();
   if (warp == 0) {
     unsigned long long p = part[lane];
-    int m = wmax[lane];
+    const int m = __reduce_max_sync(0xffffffffu, wmax[lane]);
+    const int ms = __reduce_max_sync(0xffffffffu, smax[lane]);
     for (int d = 1; d < 32; d <<= 1) {
       const unsigned long long x = __shfl_up_sync(0xffffffffu, p, d);
       if (lane >= d) p += x;
     }
-    for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
     part[lane] = p;  // inclusive over warps
-    if (lane == 0) wmax[0] = m;
+    if (lane == 0) wmax[0] = m, smax[0] = ms;
   }
   __syncthreads();
   if (t < n) dm_off[t] = (int64_t)((warp ? part[warp - 1] : 0ull) + incl - w);
   if (t == 0) {
     os->total = part[31];
     os->maxwd = wmax[0];
+    os->maxsum = smax[0];
     *counter = 0;
   }
   if (batch_done)

@@ -86,7 +86,9 @@ struct LinOrderScratch {
   int base[1024];           // first order position of each bucket
   unsigned long long total; // direction-matrix words of the batch
   int maxwd;                // widest band
-  int pad;
+  int pad;                  // the plan's error bits
+  int maxsum;               // largest l1 + l2 (k_order_small)
+  int pad2;
 };
 void launch_lin_order(int n, const LinPlan *plans, const int64_t *dm_words, int64_t *dm_off,
                       LinOrderScratch *os, int32_t *order, cudaStream_t st);
@@ -103,6 +105,15 @@ void launch_lin_dp(const LinDpArgs &A, int mode, int blocks, cudaStream_t st);
 int lin_dp4_blocks(int mode);
 int lin_dp4_warps();
 void launch_lin_dp4(const LinDpArgs &A, int mode, int blocks, cudaStream_t st);
+// Low-latency DP (linear_team.cu): a block per pair, for small batches that
+// k_lin_dp4 could run.  lin_team_width: diagonals per lane for the batch's
+// widest band and longest pair (0: does not fit); lin_team_words: direction
+// matrix words per pair.
+constexpr uint32_t kTeamSmemMax = 200 * 1024;
+int lin_team_width(int maxwd, int maxsum);
+int64_t lin_team_words(int width, int maxsum);
+int launch_lin_team(const LinDpArgs &D, int mode, int width, int64_t dm_stride, int maxsum,
+                    cudaStream_t st);
 void launch_lin_traceback(const LinTbArgs &A, cudaStream_t st);
 void launch_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
                             const int32_t *a_len, const int32_t *b_len,

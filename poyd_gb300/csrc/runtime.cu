@@ -3,6 +3,7 @@
 // affine DO path.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -207,6 +208,20 @@ static thread_local const LinVariant *g_force = nullptr;  // set while tuning
 static thread_local TuneKey g_last_key{-1, -1, -1, -1};  // class of the last batch
 static thread_local bool g_last_eligible = false;         // ... packed-eligible
 
+static int sm_count() {
+  static std::atomic<int> cache[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int c = cache[dev & 63].load();
+  if (!c) {
+    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+    cache[dev & 63].store(c = std::max(c, 1));
+  }
+  return c;
+}
+
+constexpr int kTeamPairsPerSm = 3;
+
 static int ilog2_64(int64_t x) {
   int r = 0;
   while (x > 1) {
@@ -271,9 +286,9 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   CK(cudaGetLastError());
   struct {
     unsigned long long total;
-    int maxwd, err;
+    int maxwd, err, maxsum, pad;
   } tl;
-  static_assert(sizeof(tl) == 16, "order read-back");
+  static_assert(sizeof(tl) == 24, "order read-back");
   CK(cudaMemcpyAsync(&tl, &os->total, sizeof tl, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (tl.err & 1) return fail(POYD_EINVAL, "sequences must have length >= 1 (the leading gap)");
@@ -366,6 +381,38 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     }
   }
   if (var.packed == 0) packed = false;
+  // A small batch takes a block per pair (k_lin_team) unless a tuned variant
+  // says otherwise: up to three pairs an SM, beyond which a warp per pair
+  // keeps the SMs busier.
+  const int team = packed && small && !host_waves && var.packed < 0 && var.blocks_per_sm == 0 &&
+                           var.solo < 0 && n <= kTeamPairsPerSm * sm_count()
+                       ? lin_team_width(maxwd, tl.maxsum) : 0;
+  if (team) {
+    const int64_t words = want_align ? lin_team_words(team, tl.maxsum) : 0;
+    uint32_t *tdm = dm;
+    if (want_align && words * n > max_words)
+      tdm = words * n <= budget ? (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)(words * n))
+                                : nullptr;
+    if (tdm || !want_align) {
+      LinDpArgs DA = {};
+      DA.n = n; DA.seq = seq; DA.plans = plans; DA.tables = tabs; DA.gap = cm->gap;
+      DA.dm = tdm; DA.cost = cost; DA.k = dp_constants();
+      DA.tb.n = n; DA.tb.seq = seq; DA.tb.plans = plans; DA.tb.tables = tabs; DA.tb.gap = cm->gap;
+      DA.tb.out = out; DA.tb.out_off = out_off; DA.tb.out_len = out_len;
+      DA.tb.swaped = -1; DA.tb.mode = mode;
+      {
+        ProfScope ps(want_align ? "lin_dp_dm" : "lin_dp_cost", st);
+        rc = launch_lin_team(DA, mode, team, words, tl.maxsum, st);
+      }
+      if (rc) return rc;
+      CK(cudaGetLastError());
+      return POYD_OK;
+    }
+    // the larger matrix could not be had: the buffer of the other kernel again
+    dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)max_words);
+    if (!dm) return fail(POYD_ENOMEM, "direction matrix allocation (%lld bytes) failed",
+                         (long long)(max_words * 4));
+  }
   int blocks = packed ? lin_dp4_blocks(mode) : lin_dp_blocks(mode);
   if (var.blocks_per_sm > 0) {
     int dev = 0, sms = 1;
