@@ -6,7 +6,7 @@
 // the next lane's by 7 steps, strips of 128 rows follow one another at least
 // 288 steps apart and the warp stages its own columns, about 95 cycles a
 // step.  Here one warp sweeps the band by antidiagonals t = r + j and the
-// other eight warps of the block prepare its costs:
+// eight other warps of the block prepare its costs:
 //   * lane k owns the D diagonals i = D k .. D k + D - 1 of the band (i = j - r
 //     - dlo), two cells to a register (16-bit halves, the values of
 //     k_lin_dp4): E[q] holds i = 2q and 2q + D/2, O[q] the odd ones above
@@ -39,8 +39,10 @@ namespace {
 
 constexpr unsigned kTFull = 0xffffffffu;
 constexpr uint32_t kTInf2 = 0xC000C000u;
-constexpr int kTHelpers = 8;                    // helper warps
-constexpr int kTThreads = 32 * (1 + kTHelpers);
+// Warp 0 sweeps; the warps w with w % 4 != 0 below 11 are its eight helpers: a
+// scheduler of their own each, so that warp 0 issues alone (warps 4 and 8
+// only write results).
+constexpr int kTThreads = 32 * 11;
 constexpr int kTChunk = 8;                      // double steps per chunk
 constexpr int kTStride = 36;                    // bytes per row of the cost table
 constexpr int kTPadChar = 32;
@@ -59,7 +61,11 @@ struct TeamDim {
   static constexpr uint32_t kMed = kG + 2 * 36 * 2;
   static constexpr uint32_t kEnd = kMed + 1024;                  // final registers [NQ][32]
   static constexpr uint32_t kSeq = kEnd + NQ * 128;              // the two sequences, padded
-  static constexpr uint32_t bytes(int sum) { return kSeq + (uint32_t)sum + 4 * kPad + 16; }
+  // then the path, a byte per column (at most the slot's capacity)
+  __host__ __device__ static constexpr uint32_t path(int sum) { return kSeq + (uint32_t)sum + 4 * kPad; }
+  static constexpr uint32_t bytes(int mode, int sum) {
+    return path(sum) + (mode == kDpChoice ? (uint32_t)sum + 16 : 16);
+  }
   static_assert(kTWalk * 3 * (D / 2) * 4 <= (int)kRing, "the walk's window fits the ring");
 };
 
@@ -87,8 +93,10 @@ __device__ __forceinline__ uint32_t t_mad(uint32_t a, uint32_t b, uint32_t c) {
   return d;
 }
 
-// Where a pair's cells are: dlo rounded down to even (the diagonal below the
-// band, if any, is masked), the band's indices [lo, hi).
+// Where a pair's cells are: dlo lowered to an even diagonal below the band, the
+// band's indices [lo, hi), lo 1 or 2.  Index 0 and the last (hi <= 32 D - 1) are
+// masked, so that the lanes' ring shuffles bring the first and the last lane
+// an infinite neighbour.
 struct TeamGeo {
   int L1, L2, dlo, lo, hi;
   int r0, j0;  // row and column of lane 0's first cell at double step 0
@@ -97,7 +105,7 @@ struct TeamGeo {
 __device__ __forceinline__ TeamGeo team_geo(const LinPlan &P) {
   TeamGeo g;
   g.L1 = P.l1, g.L2 = P.l2;
-  g.lo = P.dlo & 1;
+  g.lo = 2 - (P.dlo & 1);
   g.dlo = P.dlo - g.lo;
   g.hi = P.wd + g.lo;
   g.r0 = -(g.dlo >> 1);
@@ -113,6 +121,16 @@ struct TeamState {
   uint32_t kE[NQ], iE[NQ], kO[NQ], iO[NQ];  // masks: bits kept, infinity forced
   uint32_t aE[NQ], aO[NQ];                  // the moves of 8 steps
 };
+
+// Appends a register's moves (the two low bits of x's halves; y is x with them
+// cleared and the cells outside the band forced) to acc: as x - y, on the
+// multiply-add pipe, where a forced low half never shares the register with a
+// cell of the band (its borrow would reach the high half), i.e. but for q = 0.
+__device__ __forceinline__ uint32_t team_move(uint32_t acc, uint32_t x, uint32_t y, int q,
+                                              const DpK &K) {
+  if (q == 0) return t_mad(acc, (uint32_t)K.four, x & 0x00030003u);
+  return t_mad(y, (uint32_t)K.m1, t_mad(acc, (uint32_t)K.four, x));
+}
 
 // One double step.  cap: the final cell is in this one (0 even, 1 odd step):
 // its registers go to `end`.
@@ -131,15 +149,14 @@ __device__ __forceinline__ void team_step(TeamState<MODE, D> &S, const uint4 *cv
   for (int q = NQ - 1; q > 0; --q) S.gd[q] = S.gd[q - 1];
   S.gd[0] = g.y;
   {
-    uint32_t recv = __shfl_up_sync(kTFull, S.O[NQ - 1], 1);
-    if (lane == 0) recv = kTInf2;
+    const uint32_t recv = __shfl_sync(kTFull, S.O[NQ - 1], lane + 31);  // lane - 1, in a ring
     const uint32_t lw = t_prmt(recv, S.O[NQ - 1], 0x5432);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       uint32_t x = __viaddmin_u16x2(S.E[q], W[q], t_mad(S.O[q], one, S.gd[q]));
       x = __viaddmin_u16x2(q ? S.O[q - 1] : lw, S.gi[q], x);
-      if (MODE == kDpChoice) S.aE[q] = t_mad(S.aE[q], (uint32_t)K.four, x & 0x00030003u);
       S.E[q] = (x & S.kE[q]) | S.iE[q];
+      if (MODE == kDpChoice) S.aE[q] = team_move(S.aE[q], x, S.E[q], q, K);
     }
   }
   if (cap == 0) {
@@ -150,15 +167,14 @@ __device__ __forceinline__ void team_step(TeamState<MODE, D> &S, const uint4 *cv
   for (int q = 0; q + 1 < NQ; ++q) S.gi[q] = S.gi[q + 1];
   S.gi[NQ - 1] = g.x;
   {
-    uint32_t recv = __shfl_down_sync(kTFull, S.E[0], 1);
-    if (lane == 31) recv = kTInf2;
+    const uint32_t recv = __shfl_sync(kTFull, S.E[0], lane + 1);
     const uint32_t rw = t_prmt(S.E[0], recv, 0x5432);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       uint32_t x = __viaddmin_u16x2(S.O[q], W[NQ + q], t_mad(S.E[q], one, S.gi[q]));
       x = __viaddmin_u16x2(q + 1 < NQ ? S.E[q + 1] : rw, S.gd[q], x);
-      if (MODE == kDpChoice) S.aO[q] = t_mad(S.aO[q], (uint32_t)K.four, x & 0x00030003u);
       S.O[q] = (x & S.kO[q]) | S.iO[q];
+      if (MODE == kDpChoice) S.aO[q] = team_move(S.aO[q], x, S.O[q], q, K);
     }
   }
   if (cap == 1) {
@@ -167,37 +183,28 @@ __device__ __forceinline__ void team_step(TeamState<MODE, D> &S, const uint4 *cv
   }
 }
 
-// The traceback of one pair by one warp: tb_pair4_solo's walk (linear4.cu)
-// over this layout's moves.  A diagonal run stays on one lane's words, so the
-// window holds kTWalk chunks of that lane and its two neighbours.
+// The path of one pair by one warp: tb_pair4_solo's walk (linear4.cu) over this
+// layout's moves, one byte per column (0 both characters, 1 the column's only,
+// 2 the row's only) into `path`, last column first.  A diagonal run stays on
+// one lane's words, so the window holds kTWalk chunks of that lane and its two
+// neighbours.  Returns the number of columns, -1 when the path left the band.
 template <int D>
-__device__ __forceinline__ void team_walk(const LinTbArgs &A, const uint8_t *med, int id,
-                                          const LinPlan &P, const uint32_t *dm, uint4 *win,
-                                          const uint8_t *s1, const uint8_t *s2, int lane) {
+__device__ __forceinline__ int team_walk(const LinPlan &P, bool swaped, int64_t cap,
+                                         const uint32_t *dm, uint4 *win, uint8_t *path, int lane) {
   constexpr int NQ = D / 4, NV = D / 8;
   const TeamGeo g = team_geo(P);
-  const int gap = A.gap;
-  const int la = P.swap ? P.l2 : P.l1, lb = P.swap ? P.l1 : P.l2;
-  const int64_t cap = slot_cap(la, lb);
-  uint8_t *oa = A.out + A.out_off[id];
-  uint8_t *ob = oa + cap, *ow = ob + cap, *om = ow + cap;
   const uint4 *dm4 = reinterpret_cast<const uint4 *>(dm);
   const uint32_t *win4 = reinterpret_cast<const uint32_t *>(win);
   const int nch = g.me / kTChunk + 1;
-  const bool swaped = A.swaped < 0 ? !P.swap : (A.swaped != 0);
   int r = P.l1 - 1, j = P.l2 - 1;
-  int n = 0, nm = 0, wlo = nch, wk = 0;  // window: chunks [wlo, wlo + kTWalk), lanes [wk, wk + 3)
-  bool bad = false;
+  int n = 0, wlo = nch, wk = 0;  // window: chunks [wlo, wlo + kTWalk), lanes [wk, wk + 3)
   while (r > 0 || (r == 0 && j >= 0)) {
     const int i = j - r - g.dlo;
-    if (j < 0 || i < g.lo || i >= g.hi || n + 2 >= cap) {  // left the band: a bug
-      bad = true;
-      break;
-    }
+    if (j < 0 || i < g.lo || i >= g.hi || n + 2 >= cap) return -1;  // left the band: a bug
     const int k = i / D, c = (i % D) >> 1, par = i & 1;
     const int w = par * NQ + c % NQ, sh0 = 16 * (c / NQ);
     const int m0 = (r + j) >> 1;
-    if (m0 / kTChunk < wlo || m0 / kTChunk >= wlo + kTWalk || k < wk || k >= wk + 3) {
+    if (m0 / kTChunk < wlo || k < wk || k >= wk + 3) {
       wlo = max(m0 / kTChunk - kTWalk + 1, 0);
       wk = max(k - 1, 0);
       __syncwarp();
@@ -208,41 +215,89 @@ __device__ __forceinline__ void team_walk(const LinTbArgs &A, const uint8_t *med
       __syncwarp();
     }
     // lane l: the move of cell (r - l, j - l); 4 = not read
-    const int ri = r - lane, ji = j - lane, m = m0 - lane;
+    const int m = m0 - lane;
     uint32_t code = 4;
-    if (ri >= 0 && ji >= 0 && n + lane + 2 < cap && m / kTChunk >= wlo) {
+    if (r >= lane && j >= lane && n + lane + 2 < cap && m / kTChunk >= wlo) {
       const uint32_t x = win4[(((m / kTChunk - wlo) * NV + (w >> 2)) * 3 + (k - wk)) * 4 + (w & 3)];
       code = (x >> (2 * (7 - m % kTChunk) + sh0)) & 3u;
     }
     const uint32_t stop = __ballot_sync(kTFull, code != 0);
     const int f = stop ? __ffs(stop) - 1 : 32;  // lanes below f move diagonally
     const uint32_t cf = __shfl_sync(kTFull, code, f & 31);
-    const bool step_f = f < 32 && cf != 4;
-    const int move_f = step_f ? (((cf == 1u) == swaped) ? 1 : 2) : 0;
-    const bool writes = lane < f || (lane == f && step_f);
-    int md = gap;
-    if (writes) {
-      const bool dr = lane < f || move_f != 1, dj = lane < f || move_f != 2;
-      const int cr = dr ? (int)s1[ri] : gap, cc = dj ? (int)s2[ji] : gap;
-      const int ca = P.swap ? cc : cr, cb = P.swap ? cr : cc;
-      md = med[(ca << 5) | cb];
-      const int64_t pos = cap - 1 - (n + lane);
-      oa[pos] = (uint8_t)ca;
-      ob[pos] = (uint8_t)cb;
-      ow[pos] = (uint8_t)md;
-    }
-    const bool keep = writes && md != gap;
-    const uint32_t kb = __ballot_sync(kTFull, keep);
-    if (keep) om[cap - 1 - (nm + __popc(kb & ((1u << lane) - 1u)))] = (uint8_t)md;
-    n += f + (step_f ? 1 : 0);
-    nm += __popc(kb);
-    r -= f + ((step_f && move_f != 1) ? 1 : 0);
-    j -= f + ((step_f && move_f != 2) ? 1 : 0);
+    const int step = f < 32 && cf != 4;         // lane f's cell was read: its move too
+    const int move_f = step ? (((cf == 1u) == swaped) ? 1 : 2) : 0;
+    if (lane < f + step) path[n + lane] = (uint8_t)(lane == f ? move_f : 0);
+    n += f + step;
+    r -= f + (step && move_f != 1);
+    j -= f + (step && move_f != 2);
   }
-  if (lane == 0) {
-    if (!bad) om[cap - 1 - nm] = (uint8_t)gap;  // ancestor_2 ends with the leading gap (algn.c:4140-4141)
-    A.out_len[2 * id] = bad ? -1 : (int32_t)n;
-    A.out_len[2 * id + 1] = bad ? -1 : (int32_t)(nm + 1);
+  return n;
+}
+
+// The outputs of the path by the whole block (ancestor_2, median_2_with_gaps):
+// a thread takes consecutive columns; two block scans place its rows and
+// columns of the sequences and its part of the gap-free median.
+__device__ __forceinline__ void team_write(const LinTbArgs &A, const uint8_t *med, int id,
+                                           const LinPlan &P, const uint8_t *s1, const uint8_t *s2,
+                                           const uint8_t *path, int n, int64_t *scan) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int la = P.swap ? P.l2 : P.l1, lb = P.swap ? P.l1 : P.l2;
+  const int64_t cap = slot_cap(la, lb);
+  uint8_t *oa = A.out + A.out_off[id];
+  uint8_t *ob = oa + cap, *ow = ob + cap, *om = ow + cap;
+  if (n < 0) {
+    if (tid == 0) A.out_len[2 * id] = A.out_len[2 * id + 1] = -1;
+    return;
+  }
+  // inclusive sum over the block's threads
+  auto block_scan = [&](int64_t v, int64_t *total) {
+    int64_t x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(kTFull, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) scan[warp] = x;
+    __syncthreads();
+    int64_t before = 0, all = 0;
+    for (int w = 0; w < kTThreads / 32; ++w) {
+      before += w < warp ? scan[w] : 0;
+      all += scan[w];
+    }
+    *total = all;
+    return before + x;
+  };
+  const int per = (n + kTThreads - 1) / kTThreads, c0 = min(n, tid * per), c1 = min(n, c0 + per);
+  int64_t both = 0, total;
+  for (int c = c0; c < c1; ++c) both += (int64_t)(path[c] != 1) << 32 | (path[c] != 2);
+  const int64_t before = block_scan(both, &total) - both;
+  const int r0 = P.l1 - 1 - (int)(before >> 32), j0 = P.l2 - 1 - (int)(before & 0xffffffff);
+  int kept = 0;
+  for (int c = c0, r = r0, j = j0; c < c1; ++c) {
+    const int mv = path[c];
+    const int cr = mv != 1 ? (int)s1[r] : A.gap, cc = mv != 2 ? (int)s2[j] : A.gap;
+    r -= mv != 1;
+    j -= mv != 2;
+    const int ca = P.swap ? cc : cr, cb = P.swap ? cr : cc, md = med[(ca << 5) | cb];
+    oa[cap - 1 - c] = (uint8_t)ca;
+    ob[cap - 1 - c] = (uint8_t)cb;
+    ow[cap - 1 - c] = (uint8_t)md;
+    kept += md != A.gap;
+  }
+  int64_t nm;
+  int at = (int)(block_scan(kept, &nm) - kept);
+  for (int c = c0, r = r0, j = j0; c < c1; ++c) {
+    const int mv = path[c];
+    const int cr = mv != 1 ? (int)s1[r] : A.gap, cc = mv != 2 ? (int)s2[j] : A.gap;
+    r -= mv != 1;
+    j -= mv != 2;
+    const int md = med[P.swap ? (cc << 5) | cr : (cr << 5) | cc];
+    if (md != A.gap) om[cap - 1 - at++] = (uint8_t)md;
+  }
+  if (tid == 0) {
+    om[cap - 1 - nm] = (uint8_t)A.gap;  // ancestor_2 ends with the leading gap (algn.c:4140-4141)
+    A.out_len[2 * id] = n;
+    A.out_len[2 * id + 1] = (int32_t)nm + 1;
   }
 }
 
@@ -278,7 +333,10 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
   const bool swaped = !P.swap;  // backtrack priority (algn.c:3605-3666)
   const int rank_i = MODE == kDpChoice ? (swaped ? 1 : 2) : 0;
   const int rank_d = MODE == kDpChoice ? 3 - rank_i : 0;
-  for (int e = tid; e < 33 * 33; e += kTThreads) {
+#pragma unroll
+  for (int e0 = 0; e0 < 33 * 33; e0 += kTThreads) {
+    const int e = e0 + tid;
+    if (e >= 33 * 33) break;
     const int a = e / 33, b = e - 33 * a;
     tab[a * kTStride + b] =
         a < 32 && b < 32 ? (uint8_t)(sc * (A.tables->packed[(a << 5) | b] & 0xffffu)) : 0;
@@ -288,12 +346,15 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
     gd_t[tid] = (uint16_t)((tid < 32 ? sc * (A.tables->packed[(tid << 5) | A.gap] & 0xffffu) : 0) + rank_d);
   }
   if (MODE == kDpChoice)
-    for (int i = tid; i < 1024; i += kTThreads) med[i] = A.tables->median[i];
+    for (int i = tid; i < 256; i += kTThreads)
+      reinterpret_cast<uint32_t *>(med)[i] = reinterpret_cast<const uint32_t *>(A.tables->median)[i];
   uint8_t *s1 = team_sm + Dm::kSeq + Dm::kPad, *s2 = s1 + g.L1 + 2 * Dm::kPad;
+#pragma unroll 4
   for (int x = tid; x < g.L1 + 2 * Dm::kPad; x += kTThreads) {
     const int r = x - Dm::kPad;
     s1[r] = r >= 0 && r < g.L1 ? A.seq[P.s1_off + r] : (uint8_t)kTPadChar;
   }
+#pragma unroll 4
   for (int x = tid; x < g.L2 + 2 * Dm::kPad; x += kTThreads) {
     const int j = x - Dm::kPad;
     s2[j] = j >= 0 && j < g.L2 ? A.seq[P.s2_off + j] : (uint8_t)kTPadChar;
@@ -302,7 +363,7 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
 
   // a helper's share of chunk c: lane k, double step 8 c + (lane >> 2)
   auto produce = [&](int c) {
-    const int k = 4 * (warp - 1) + (lane & 3), v = lane >> 2, m = kTChunk * c + v;
+    const int k = 4 * (warp - 1 - warp / 4) + (lane & 3), v = lane >> 2, m = kTChunk * c + v;
     const int r0 = g.r0 + m - 2 * NQ * k, j0 = g.j0 + m + 2 * NQ * k;
     const uint8_t *pa = s1 + r0, *pb = s2 + j0;
     int b[2 * NQ + 1];
@@ -360,14 +421,14 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
       }
       S.aE[q] = S.aO[q] = 0;
     }
-  } else {
+  } else if (warp % 4) {
     produce(0);
   }
   __syncthreads();
   for (int c = 0; c < nch; ++c) {
-    if (warp != 0) {
+    if (warp % 4) {
       if (c + 1 < nch) produce(c + 1);
-    } else {
+    } else if (warp == 0) {
       const uint8_t *slot = team_sm + (c & 1) * Dm::kSlot;
       if (c + 1 < nch) {
 #pragma unroll
@@ -393,23 +454,29 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
     }
     __syncthreads();
   }
-  if (warp != 0) return;
-  if (lane == 0) {
+  if (tid == 0) {
     const int cc = (fcell % D) >> 1;
     const uint32_t v = (end[32 * (cc % NQ) + fk] >> (16 * (cc / NQ))) & 0xFFFFu;
     A.cost[id] = ((int)v - (int)tab[s1[0] * kTStride + s2[0]]) / sc;
   }
   if (MODE == kDpChoice) {
-    __syncwarp();
-    team_walk<D>(A.tb, med, id, P, A.dm + id * A.dm_stride, reinterpret_cast<uint4 *>(team_sm), s1,
-                 s2, lane);
+    __shared__ int s_n;
+    __shared__ int64_t scan[kTThreads / 32];
+    uint8_t *path = team_sm + Dm::path(g.L1 + g.L2);
+    if (warp == 0) {
+      const int n = team_walk<D>(P, swaped, slot_cap(g.L1, g.L2), A.dm + id * A.dm_stride,
+                                 reinterpret_cast<uint4 *>(team_sm), path, lane);
+      if (lane == 0) s_n = n;
+    }
+    __syncthreads();
+    team_write(A.tb, med, id, P, s1, s2, path, s_n, scan);
   }
 }
 
 template <int MODE, int D>
 int team_launch(const TeamArgs &A, int maxsum, cudaStream_t st) {
   static std::atomic<uint32_t> opted[64];
-  const uint32_t sm = TeamDim<D>::bytes(maxsum);
+  const uint32_t sm = TeamDim<D>::bytes(MODE, maxsum);
   int dev = 0;
   cudaGetDevice(&dev);
   if (opted[dev & 63].load() < sm) {
@@ -424,12 +491,13 @@ int team_launch(const TeamArgs &A, int maxsum, cudaStream_t st) {
 
 }  // namespace
 
-// Diagonals per lane for bands up to maxwd (one more for the parity), 0 when
-// the band or the sequences do not fit.
+// Diagonals per lane for bands up to maxwd (three more: the masked ends and the
+// parity), 0 when the band or the sequences do not fit.
 int lin_team_width(int maxwd, int maxsum) {
-  const int d = maxwd + 1 <= 256 ? 8 : maxwd + 1 <= 512 ? 16 : maxwd + 1 <= 1024 ? 32 : 0;
-  const uint32_t sm = d == 8 ? TeamDim<8>::bytes(maxsum) : d == 16 ? TeamDim<16>::bytes(maxsum)
-                    : d == 32 ? TeamDim<32>::bytes(maxsum) : 0;
+  const int d = maxwd + 3 <= 256 ? 8 : maxwd + 3 <= 512 ? 16 : maxwd + 3 <= 1024 ? 32 : 0;
+  const uint32_t sm = d == 8 ? TeamDim<8>::bytes(kDpChoice, maxsum)
+                    : d == 16 ? TeamDim<16>::bytes(kDpChoice, maxsum)
+                    : d == 32 ? TeamDim<32>::bytes(kDpChoice, maxsum) : 0;
   return sm <= kTeamSmemMax ? d : 0;
 }
 
