@@ -1,4 +1,6 @@
-// Affine-gap ("3 matrix", 4-state) banded DO on sm_103a.
+// Affine-gap ("3 matrix", 4-state) banded DO on sm_103a: plans, the row-wise
+// kernels (values past 16 bits, very wide bands) and the batch driver; the
+// others run by antidiagonals in affine_diag.cu.
 //
 // Restates algn_fill_plane_3_aff_nobt / algn_fill_plane_3_aff
 // (algn.c:2287-2548) with the FILL_* cell rules (algn.c:1740-1977) and
@@ -26,6 +28,7 @@
 #include <cstdlib>
 #include <numeric>
 #include <vector>
+#include "affine_diag.cuh"
 #include "affine_kernels.cuh"
 #include "back_writer.cuh"
 
@@ -52,17 +55,6 @@ constexpr int kAffWarps = 4;                // warps per block (24 per SM)
 constexpr uint32_t kCodeLeft = 2u | 4u | (3u << 5);   // DO_VERTICAL | END_VERTICAL
 constexpr uint32_t kCodeRight = 0u | 8u | (3u << 5);  // DO_HORIZONTAL | END_HORIZONTAL
 
-struct AffPlan {
-  int64_t si_off, sj_off;
-  int32_t leni, lenj;  // rows 0..leni (si), columns 0..lenj (sj)
-  int32_t e0, wd;
-  int32_t swap;        // 1: rows are the caller's b
-  int32_t nstrips, sblocks;  // sblocks: 4-step DM words per lane per strip
-  int32_t empty;
-  int32_t pad_[4];
-};
-static_assert(sizeof(AffPlan) == 64, "AffPlan layout");
-
 struct AffPlanArgs {
   int n;
   const uint8_t *seq;
@@ -73,12 +65,16 @@ struct AffPlanArgs {
   int gap;
   int dos_empty;
   long long maxc;
+  int scale, go;     // k_aff_diag's value scale (0: its 16 bits are out of the question)
+  int maxsub, maxext;  // largest substitution and extension cost
   AffPlan *plans;
   int64_t *dm_words;
-  int32_t *wd_out;
+  int32_t *wd_out;   // band width; kAffFits when k_aff_diag's values fit
+  int32_t *steps;    // leni + lenj
   int64_t *cells;
   int32_t *err;
 };
+constexpr int32_t kAffFits = 1 << 30;
 
 struct AffDpArgs {
   int n;
@@ -106,10 +102,14 @@ struct AffTbArgs {
   uint8_t *out;
   const int64_t *out_off;
   int32_t *out_len;
+  const int32_t *order;  // the pairs to walk
 };
 
-__global__ void k_aff_plan(AffPlanArgs A) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per pair: the scans of its sequences are coalesced (a thread per
+// pair took 381 us for 16,384 pairs of 100-5,000 bp).
+__global__ void __launch_bounds__(128) k_aff_plan(AffPlanArgs A) {
+  const int lane = threadIdx.x & 31;
+  const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (id >= A.n) return;
   const int la = A.a_len[id], lb = A.b_len[id];
   const int64_t ao = A.a_off[id], bo = A.b_off[id];
@@ -130,33 +130,56 @@ __global__ void k_aff_plan(AffPlanArgs A) {
   const int Spad = (S + 15) / 16 * 16;  // whole 16-step half blocks
   P.sblocks = Spad / 4;
   P.empty = 0;
-  if (A.dos_empty) {
-    bool ea = true, eb = true;
-    for (int x = 0; x < la && ea; ++x) ea = A.seq[ao + x] == A.gap;
-    for (int x = 0; x < lb && eb; ++x) eb = A.seq[bo + x] == A.gap;
-    P.empty = ea ? 1 : (eb ? 2 : 0);
+  // codes: any above 31 (they index 32-entry table rows), gap-bearing ones past
+  // position 0, all gaps
+  unsigned wide = 0, gaps = 0, rest_a = 0, rest_b = 0;
+  for (int x = lane; x < la; x += 32) {
+    const int c = A.seq[ao + x];
+    wide |= (unsigned)c;
+    gaps |= x ? c & 16 : 0;
+    rest_a |= c != A.gap;
   }
-  for (int t = 0; t < 4; ++t) P.pad_[t] = 0;
-  A.plans[id] = P;
-  A.dm_words[id] = (int64_t)P.nstrips * P.sblocks * kAffRows;
-  A.wd_out[id] = P.wd;
+  for (int x = lane; x < lb; x += 32) {
+    const int c = A.seq[bo + x];
+    wide |= (unsigned)c;
+    gaps |= x ? c & 16 : 0;
+    rest_b |= c != A.gap;
+  }
+  wide = __reduce_or_sync(kFullA, wide);
+  gaps = __reduce_or_sync(kFullA, gaps);
+  rest_a = __reduce_or_sync(kFullA, rest_a);
+  rest_b = __reduce_or_sync(kFullA, rest_b);
+  if (A.dos_empty) P.empty = !rest_a ? 1 : (!rest_b ? 2 : 0);
+  long long cells = 0;
   if (A.cells) {
-    long long c = lenj + 1;
-    for (int i = 1; i <= leni; ++i) {
+    for (int i = 1 + lane; i <= leni; i += 32) {
       const int s = i > kStart ? i - kStart + 1 : 1;
       int e = e0 + i - 1;
       if (e > lenj) e = lenj;
-      c += e - s + 1;
+      cells += e - s + 1;
     }
-    A.cells[id] = c;
+    for (int o = 16; o > 0; o >>= 1) cells += __shfl_xor_sync(kFullA, cells, o);
   }
-  if (la < 1 || lb < 1) atomicOr(A.err, 1);
-  unsigned wide = 0;  // codes index 32-entry table rows
-  for (int x = 0; x < la; ++x) wide |= A.seq[ao + x];
-  for (int x = 0; x < lb; ++x) wide |= A.seq[bo + x];
-  if (wide >> 5) atomicOr(A.err, 4);
+  if (lane != 0) return;
+  for (int t = 0; t < 4; ++t) P.pad_[t] = 0;
+  A.plans[id] = P;
+  A.dm_words[id] = (int64_t)P.nstrips * P.sblocks * kAffRows;
+  A.steps[id] = leni + lenj;
+  // k_aff_diag: a cell's value is at most that of the diagonal path and one gap
+  // to it (and a state's, one more opening and step); infinities grow by at
+  // most a band of extensions outside the matrix
+  const long long ext = A.maxext + A.go + 1LL, step = A.maxsub + 2 * ext;
+  const long long most = A.scale * ((long long)leni * A.maxsub + P.wd * ext + 4 * step);
+  const bool fits = A.scale && most < 0xC000 && A.scale * (ext * (P.wd + 8) + 4 * step) < 0x3000;
+  A.wd_out[id] = P.wd | (fits ? kAffFits : 0);
+  if (A.cells) A.cells[id] = cells + lenj + 1;
+  int err = 0;
+  if (la < 1 || lb < 1) err |= 1;
+  if (wide >> 5) err |= 4;
   // real costs must stay clear of the HIGH_NUM sentinel arithmetic
-  if (A.maxc * (long long)(la + lb + 2) >= (1 << 22)) atomicOr(A.err, 2);
+  if (A.maxc * (long long)(la + lb + 2) >= (1 << 22)) err |= 2;
+  if (gaps) err |= 16;  // not an error: k_aff_diag's general variant
+  if (err) atomicOr(A.err, err);
 }
 
 // Shared memory of one k_aff_dp block.
@@ -782,8 +805,9 @@ __global__ void __launch_bounds__(128) k_aff_traceback(AffTbArgs A) {
   __shared__ uint8_t med[1024];
   for (int t = threadIdx.x; t < 1024; t += blockDim.x) med[t] = A.tables->median[t];
   __syncthreads();
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= A.n) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= A.n) return;
+  const int id = A.order[t];
   const AffPlan P = A.plans[id];
   const int li = P.leni + 1, lj = P.lenj + 1;
   const int la = P.swap ? lj : li, lb = P.swap ? li : lj;
@@ -922,57 +946,145 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   if (rc) return rc;
   AffPlan *plans = (AffPlan *)ws_buffer(w, WS_AFF, sizeof(AffPlan) * (size_t)n);
   int64_t *dmw = (int64_t *)ws_buffer(w, WS_DMWORDS, sizeof(int64_t) * 2 * (size_t)n);
-  int32_t *wdb = (int32_t *)ws_buffer(w, WS_WD, sizeof(int32_t) * 2 * (size_t)n + 16);
-  int32_t *err = (int32_t *)ws_buffer(w, WS_ERR, 64);
-  if (!plans || !dmw || !wdb || !err) return fail(POYD_ENOMEM, "plan allocation failed");
+  // band widths, steps and the error word, read back together
+  int32_t *wdb = (int32_t *)ws_buffer(w, WS_WD, sizeof(int32_t) * (2 * (size_t)n + 1) + 16);
+  if (!plans || !dmw || !wdb) return fail(POYD_ENOMEM, "plan allocation failed");
+  int32_t *err = wdb + 2 * (size_t)n;
   CKA(cudaMemsetAsync(err, 0, 4, st));
+  // The packed kernels run when one step's largest add stays far below their
+  // 16-bit infinity (small cost tables; POYD_AFF_PACKED=0 keeps the 32-bit
+  // kernel).
+  const long long top = std::max(maxc, cm->gap_open);
+  bool packed = 4LL * (top + 2LL * cm->gap_open + 1) < 0x3000;
+  if (const char *e = std::getenv("POYD_AFF_PACKED")) packed = packed && std::atoi(e) != 0;
+  int maxsub = 0, maxext = 0;
+  bool negative = false;  // only entries of code 0 can be, which no constructor sets
+  for (int x = 0; x < 32; ++x) {
+    for (int y = 0; y < 16 && x < 16; ++y) {
+      maxsub = std::max(maxsub, cm->cost[x << 5 | y] & 0xffff);
+      negative |= cm->cost[x << 5 | y] < 0;
+    }
+    for (const int c : {cm->cost[x << 5 | 16], cm->cost[16 << 5 | x]}) {
+      maxext = std::max(maxext, c & 0xffff);
+      negative |= c < 0;
+    }
+  }
   AffPlanArgs PA;
   PA.n = n; PA.seq = seq; PA.a_off = a_off; PA.a_len = a_len; PA.b_off = b_off;
   PA.b_len = b_len; PA.gap = cm->gap; PA.dos_empty = (flags & POYD_FLAG_DOS_EMPTY) ? 1 : 0;
-  PA.maxc = std::max(maxc, cm->gap_open);
-  PA.plans = plans; PA.dm_words = dmw; PA.wd_out = wdb; PA.cells = cells; PA.err = err;
+  PA.maxc = top;
+  PA.scale = packed && !negative ? (want_align ? 4 : 1) : 0;
+  PA.maxsub = maxsub; PA.maxext = maxext;
+  PA.go = cm->gap_open;
+  PA.plans = plans; PA.dm_words = dmw; PA.wd_out = wdb; PA.steps = wdb + n; PA.cells = cells;
+  PA.err = err;
   {
     ProfScope ps("aff_plan", st);
-    k_aff_plan<<<(n + 127) / 128, 128, 0, st>>>(PA);
+    k_aff_plan<<<(unsigned)(((int64_t)n + 3) / 4), 128, 0, st>>>(PA);
   }
   CKA(cudaGetLastError());
-  std::vector<int64_t> hw((size_t)n);
-  std::vector<int32_t> hwd((size_t)n + 1);
-  CKA(cudaMemcpyAsync(hw.data(), dmw, sizeof(int64_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
-  CKA(cudaMemcpyAsync(hwd.data(), wdb, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
-  CKA(cudaMemcpyAsync(hwd.data() + n, err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  std::vector<int32_t> hwd(2 * (size_t)n + 1);
+  CKA(cudaMemcpyAsync(hwd.data(), wdb, sizeof(int32_t) * hwd.size(), cudaMemcpyDeviceToHost, st));
   CKA(cudaStreamSynchronize(st));
-  if (hwd[n] & 1) return fail(POYD_EINVAL, "sequences must have length >= 1 (the leading gap)");
-  if (hwd[n] & 2) return fail(POYD_ERANGE, "affine costs could reach the HIGH_NUM sentinel range");
-  if (hwd[n] & 4) return fail(POYD_EINVAL, "sequence codes must be below 32 (5-bit element masks)");
-  std::vector<int64_t> off((size_t)n);
-  int64_t total = 0;
-  int maxwd = 1;
-  for (int32_t t = 0; t < n; ++t) {
-    off[t] = total;
-    if (want_align) total += hw[t];
-    maxwd = std::max(maxwd, hwd[t]);
+  const int herr = hwd[2 * (size_t)n];
+  if (herr & 1) return fail(POYD_EINVAL, "sequences must have length >= 1 (the leading gap)");
+  if (herr & 2) return fail(POYD_ERANGE, "affine costs could reach the HIGH_NUM sentinel range");
+  if (herr & 4) return fail(POYD_EINVAL, "sequence codes must be below 32 (5-bit element masks)");
+
+  // Longest first; the pairs whose values fit go to k_aff_diag (affine_diag.cu)
+  // in tasks of one class (lanes x diagonals a lane), longest task first; the
+  // others run in rows.
+  std::vector<int64_t> key((size_t)n);
+  for (int32_t t = 0; t < n; ++t) key[t] = (int64_t)hwd[(size_t)n + t] << 7;  // longest_first's unit
+  std::vector<int32_t> order, rows_of, slots[kDiagClassN];
+  longest_first(key, order);
+  for (int32_t id : order) {
+    const int c = (hwd[id] & kAffFits) ? aff_diag_class((hwd[id] & ~kAffFits) - 41) : kDiagClassN;
+    if (c == kDiagClassN) rows_of.push_back(id);
+    else slots[c].push_back(id);
   }
-  std::vector<int32_t> order;
-  longest_first(hw, order);
+  struct Task {
+    int cls, at;  // the class and the first of its pairs in slots[cls]
+  };
+  std::vector<Task> tasks;
+  key.clear();
+  for (int c = 0; c < kDiagClassN; ++c) {
+    const int per = 32 / kDiagClasses[c].lanes;
+    for (int at = 0; at < (int)slots[c].size(); at += per) {
+      tasks.push_back({c, at});
+      key.push_back((int64_t)hwd[(size_t)n + slots[c][at]] * kDiagClasses[c].width << 3);
+    }
+  }
+  std::vector<int32_t> torder, all;
+  longest_first(key, torder);
+  std::vector<int64_t> task_word;
+  int64_t total = 0;
+  for (int32_t q : torder) {
+    const Task t = tasks[q];
+    const AffDiagClass c = kDiagClasses[t.cls];
+    task_word.push_back(aff_diag_task(total, c));
+    if (want_align) total += aff_diag_words(c.width, hwd[(size_t)n + slots[t.cls][t.at]]);
+    for (int g = 0; g < kDiagTask; ++g) {
+      const bool in = g < 32 / c.lanes && t.at + g < (int)slots[t.cls].size();
+      all.push_back(in ? slots[t.cls][t.at + g] : -1);
+    }
+  }
+  const int diag = (int)all.size(), rows = (int)rows_of.size();
+  all.insert(all.end(), rows_of.begin(), rows_of.end());
+  int maxwd = 1;
+  std::vector<int64_t> off, hw;
+  if (rows) {
+    hw.resize((size_t)n);
+    CKA(cudaMemcpyAsync(hw.data(), dmw, sizeof(int64_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
+    CKA(cudaStreamSynchronize(st));
+    off.assign((size_t)n, 0);
+    for (int32_t id : rows_of) {
+      off[id] = total;
+      if (want_align) total += hw[id];
+      maxwd = std::max(maxwd, hwd[id] & ~kAffFits);
+    }
+  }
+  // device lists: the order, then (8-byte aligned) the tasks' offsets
+  const size_t list = (all.size() + 1) & ~(size_t)1;
   int64_t *doff = dmw + n;
-  int32_t *dord = (int32_t *)ws_buffer(w, WS_ORDER, sizeof(int32_t) * (size_t)n);
+  int32_t *dord = (int32_t *)ws_buffer(w, WS_ORDER, 4 * list + 8 * task_word.size() + 16);
   int *counter = (int *)ws_buffer(w, WS_COUNTER, 64);
-  if (!dord || !counter) return fail(POYD_ENOMEM, "order allocation failed");
-  CKA(cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, st));
-  CKA(cudaMemcpyAsync(dord, order.data(), sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
-  CKA(cudaMemsetAsync(counter, 0, 4, st));
+  AffWhere *where = want_align ? (AffWhere *)ws_buffer(w, WS_CELLS, sizeof(AffWhere) * (size_t)n) : nullptr;
+  if (!dord || !counter || (want_align && !where)) return fail(POYD_ENOMEM, "order allocation failed");
+  all.resize(list, -1);
+  CKA(cudaMemcpyAsync(dord, all.data(), 4 * list, cudaMemcpyHostToDevice, st));
+  int64_t *dtask = (int64_t *)(dord + list);
+  if (diag)
+    CKA(cudaMemcpyAsync(dtask, task_word.data(), 8 * task_word.size(), cudaMemcpyHostToDevice, st));
+  CKA(cudaMemsetAsync(counter, 0, 64, st));
   uint32_t *dm = nullptr;
   if (want_align) {
     dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)std::max<int64_t>(total, 1));
     if (!dm) return fail(POYD_ENOMEM, "affine direction matrix allocation failed");
   }
-  // The packed kernel runs when one step's largest add stays far below its
-  // 16-bit infinity (small cost tables; POYD_AFF_PACKED=0 keeps the 32-bit
-  // kernel); a pair whose final cost is past its exact range sends the
-  // whole batch to the 32-bit kernel afterwards.
-  bool packed = 4LL * (PA.maxc + 2LL * cm->gap_open + 1) < 0x3000;
-  if (const char *e = std::getenv("POYD_AFF_PACKED")) packed = packed && std::atoi(e) != 0;
+  const char *name = want_align ? "aff_dp_dm" : "aff_dp_cost";
+  AffDiagArgs GA = {};
+  GA.seq = seq; GA.plans = plans; GA.order = dord; GA.tables = tabs; GA.go = cm->gap_open;
+  GA.dm = dm; GA.where = where; GA.cost = cost;
+  GA.one = 1; GA.m1 = ~0u; GA.k4 = 4; GA.k8 = 8; GA.k16 = 16; GA.k32 = 32; GA.k256 = 256;
+  if (diag) {
+    GA.tasks = (int)task_word.size(); GA.task = dtask; GA.counter = counter;
+    ProfScope ps(name, st);
+    if ((rc = launch_aff_diag(GA, want_align, (herr & 16) != 0, st))) return rc;
+  }
+  if (diag && want_align) {
+    AffWalkArgs WA;
+    WA.n = diag; WA.seq = seq; WA.plans = plans; WA.order = dord; WA.where = where;
+    WA.dm = dm; WA.tables = tabs; WA.out = out; WA.out_off = out_off; WA.out_len = out_len;
+    ProfScope ps("aff_traceback", st);
+    if ((rc = launch_aff_walk(WA, st))) return rc;
+  }
+  if (!rows) return POYD_OK;
+
+  // The rows kernels, two pairs per lane group in 16-bit halves or (large
+  // costs) one in 32 bits; a pair whose final cost is past the packed exact
+  // range sends its batch to the 32-bit kernel afterwards.
+  CKA(cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, st));
   for (int attempt = 0; attempt < 2; ++attempt) {
     const int blocks = aff_blocks(want_align, packed);
     const int64_t slab = maxwd + 8;
@@ -981,12 +1093,13 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
                                           kAffGroups);
     if (!scratch) return fail(POYD_ENOMEM, "scratch allocation failed");
     AffDpArgs DA;
-    DA.n = n; DA.seq = seq; DA.plans = plans; DA.dm_off = doff; DA.order = dord; DA.tables = tabs;
-    DA.go = cm->gap_open; DA.counter = counter; DA.scratch = scratch; DA.slab = slab; DA.dm = dm;
+    DA.n = rows; DA.seq = seq; DA.plans = plans; DA.dm_off = doff; DA.order = dord + diag;
+    DA.tables = tabs;
+    DA.go = cm->gap_open; DA.counter = counter + 1; DA.scratch = scratch; DA.slab = slab; DA.dm = dm;
     DA.cost = cost; DA.err = err;
-    if (attempt) CKA(cudaMemsetAsync(counter, 0, 4, st));
+    if (attempt) CKA(cudaMemsetAsync(counter + 1, 0, 4, st));
     {
-      ProfScope ps(want_align ? "aff_dp_dm" : "aff_dp_cost", st);
+      ProfScope ps(name, st);
       if (packed && want_align) k_aff_dp2<true><<<blocks, kAffWarps * 32, 0, st>>>(DA);
       else if (packed) k_aff_dp2<false><<<blocks, kAffWarps * 32, 0, st>>>(DA);
       else if (want_align) k_aff_dp<true><<<blocks, kAffWarps * 32, 0, st>>>(DA);
@@ -995,11 +1108,11 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
     CKA(cudaGetLastError());
     if (want_align) {
       AffTbArgs TA;
-      TA.n = n; TA.seq = seq; TA.plans = plans; TA.dm_off = doff; TA.dm = dm; TA.tables = tabs;
-      TA.out = out; TA.out_off = out_off; TA.out_len = out_len;
+      TA.n = rows; TA.seq = seq; TA.plans = plans; TA.dm_off = doff; TA.dm = dm; TA.tables = tabs;
+      TA.out = out; TA.out_off = out_off; TA.out_len = out_len; TA.order = dord + diag;
       {
         ProfScope ps("aff_traceback", st);
-        k_aff_traceback<<<(n + 127) / 128, 128, 0, st>>>(TA);
+        k_aff_traceback<<<(rows + 127) / 128, 128, 0, st>>>(TA);
       }
       CKA(cudaGetLastError());
     }
