@@ -689,38 +689,51 @@ __global__ void __launch_bounds__(kDpWarps * 32, 3) k_lin_dp(LinDpArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// Packing of batched align_2 results: one warp per pair copies the used tail
-// of each of its four right-aligned slots back to back.
+// Packing of batched align_2 results: a block per pair copies the used tail of
+// each of its four right-aligned slots back to back, 16 bytes a store.  A
+// store's source starts anywhere in a word: its five aligned words are
+// shifted together (only words that hold some of its bytes are read).
+// Measured: 65,536 pairs of 100-5,000 bp (670 MB) took 785 us with a warp per
+// pair copying bytes; one pair of 1,000 bp 25 us.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 16) k_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
-                                  const int32_t *a_len, const int32_t *b_len,
-                                  const int32_t *out_len, uint8_t *packed,
-                                  const int64_t *packed_off) {
-  const int lane = threadIdx.x & 31;
-  const int64_t id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (id >= n) return;
-  const int64_t cap = slot_cap(a_len[id], b_len[id]);
+constexpr int kPackThreads = 128;
+__device__ __forceinline__ void pack_copy(uint8_t *d, const uint8_t *s, int64_t len) {
+  const int64_t head = min(len, (int64_t)(-(intptr_t)d & 15));
+  if (threadIdx.x < head) d[threadIdx.x] = s[threadIdx.x];
+  d += head, s += head, len -= head;
+  const int64_t full = len >> 4;
+  const uint32_t *w = reinterpret_cast<const uint32_t *>((uintptr_t)s & ~(uintptr_t)3);
+  const unsigned sh = 8u * (unsigned)((uintptr_t)s & 3);
+  for (int64_t x = threadIdx.x; x < full; x += kPackThreads) {
+    const uint32_t *p = w + 4 * x;
+    const uint32_t a = p[0], b = p[1], c = p[2], e = p[3], f = sh ? p[4] : 0u;
+    reinterpret_cast<uint4 *>(d)[x] =
+        make_uint4(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh), __funnelshift_r(c, e, sh),
+                   __funnelshift_r(e, f, sh));
+  }
+  const int64_t at = (full << 4) + threadIdx.x;
+  if (threadIdx.x < 16 && at < len) d[at] = s[at];
+}
+
+// cap: every slot's sequence capacity, or null: from the pair's lengths
+__global__ void __launch_bounds__(kPackThreads, 12) k_pack_alignments(
+    const uint8_t *out, const int64_t *out_off, const int32_t *a_len, const int32_t *b_len,
+    const int64_t *caps, const int32_t *out_len, uint8_t *packed, const int64_t *packed_off) {
+  const int64_t id = blockIdx.x;
+  const int64_t cap = caps ? caps[id] : slot_cap(a_len[id], b_len[id]);
   const int64_t na = out_len[2 * id], nm = out_len[2 * id + 1];
   const uint8_t *src = out + out_off[id];
   uint8_t *dst = packed + packed_off[id];
-  for (int k = 0; k < 4; ++k) {
-    const int64_t len = k < 3 ? na : nm;
-    const uint8_t *s = src + (k + 1) * cap - len;
-    uint8_t *d = dst + (k < 3 ? k * na : 3 * na);
-    for (int64_t x = lane; x < len; x += 32) d[x] = s[x];
-  }
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) pack_copy(dst + k * na, src + (k + 1) * cap - na, na);
+  pack_copy(dst + 3 * na, src + 4 * cap - nm, nm);
 }
 
 void launch_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
-                            const int32_t *a_len, const int32_t *b_len,
+                            const int32_t *a_len, const int32_t *b_len, const int64_t *caps,
                             const int32_t *out_len, uint8_t *packed,
                             const int64_t *packed_off, cudaStream_t st) {
-  // 128-thread blocks (<= 32 registers each) fit in the registers a
-  // resident k_lin_dp grid leaves free on every SM, so a pipelined caller's
-  // pack runs beside the next chunk's DP instead of after it
-  const int threads = 128;
-  const int64_t blocks = ((int64_t)n * 32 + threads - 1) / threads;
-  k_pack_alignments<<<(unsigned)blocks, threads, 0, st>>>(n, out, out_off, a_len, b_len,
+  k_pack_alignments<<<(unsigned)n, kPackThreads, 0, st>>>(out, out_off, a_len, b_len, caps,
                                                           out_len, packed, packed_off);
 }
 

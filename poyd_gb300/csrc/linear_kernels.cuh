@@ -116,7 +116,7 @@ int launch_lin_team(const LinDpArgs &D, int mode, int width, int64_t dm_stride, 
                     cudaStream_t st);
 void launch_lin_traceback(const LinTbArgs &A, cudaStream_t st);
 void launch_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
-                            const int32_t *a_len, const int32_t *b_len,
+                            const int32_t *a_len, const int32_t *b_len, const int64_t *caps,
                             const int32_t *out_len, uint8_t *packed,
                             const int64_t *packed_off, cudaStream_t st);
 

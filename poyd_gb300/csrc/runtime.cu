@@ -481,7 +481,7 @@ extern "C" int poyd_pack_alignments(int32_t n, const uint8_t *out, const int64_t
     return fail(POYD_EINVAL, "poyd_pack_alignments: null argument");
   if (n == 0) return POYD_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  { ProfScope ps("pack_alignments", st); launch_pack_alignments(n, out, out_off, a_len, b_len, out_len, packed, packed_off, st); }
+  { ProfScope ps("pack_alignments", st); launch_pack_alignments(n, out, out_off, a_len, b_len, nullptr, out_len, packed, packed_off, st); }
   CK(cudaGetLastError());
   return POYD_OK;
 }
