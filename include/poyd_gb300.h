@@ -471,14 +471,13 @@ typedef struct poyd_node_store {
 /* ---------------------------------------------------------------------
  * Autotuner (no counterpart in the reference).  The batched linear DP
  * (poyd_cost_2_batch, poyd_align_2_batch, poyd_align_2_host and every
- * caller of them) has launch variants with identical results: the packed
- * kernel when its 16-bit bound holds or the 32-bit kernel, a persistent
- * grid of 1 to the maximum resident blocks per SM, and for batches with a
- * warp per pair the whole-warp or the batched traceback walk.  A variant
+ * caller of them) has launch variants with identical results: the default
+ * (-1: where 16 bits hold a block per pair or the antidiagonal kernel, by the
+ * batch's size), the packed warp-per-pair kernel or the 32-bit kernel, of
+ * these a persistent grid of 1 to the maximum resident blocks per SM, and for
+ * batches with a warp per pair the whole-warp or the batched traceback walk.  A variant
  * is kept per shape class: (device, align 0/1, floor(log2 pairs),
- * floor(log2 widest band)).  Without an entry the defaults apply (packed
- * when it can, the maximum grid, the whole-warp walk when every pair has
- * its own warp).  The band is always the reference's.
+ * floor(log2 widest band)).  Without an entry the defaults apply.  The band is always the reference's.
  * ------------------------------------------------------------------- */
 typedef struct poyd_tune_result {
   int32_t packed, blocks_per_sm, solo; /* the variant kept (-1: default) */

@@ -44,9 +44,9 @@ struct LinTbArgs {
 
 // Runtime multipliers of the DP's multiply-add arithmetic (see linear.cu).
 struct DpK {
-  int one, m1, four, m64k;
+  int one, m1, four, m64k, k64;
 };
-inline DpK dp_constants() { return DpK{1, -1, 4, -65536}; }
+inline DpK dp_constants() { return DpK{1, -1, 4, -65536, 65536}; }
 
 struct LinDpArgs {
   int n;
@@ -114,6 +114,66 @@ int lin_team_width(int maxwd, int maxsum);
 int64_t lin_team_words(int width, int maxsum);
 int launch_lin_team(const LinDpArgs &D, int mode, int width, int64_t dm_stride, int maxsum,
                     cudaStream_t st);
+// Throughput DP (linear_diag.cu): 8, 16 or 32 lanes a pair, the band in
+// registers, for large batches that k_lin_dp4 could run.  A class is (lanes,
+// diagonals a lane), widest band first; wider pairs stay with k_lin_dp4.
+struct LinDiagClass {
+  int lanes, width;
+};
+constexpr int kLinDiagClasses = 18, kLinDiagBuckets = 128;
+__host__ __device__ __forceinline__ LinDiagClass lin_diag_class(int c) {
+  return LinDiagClass{32 >> (c / 6), 28 - 4 * (c % 6)};
+}
+// idx = j - i + off: the least even off that leaves idx 0 below the band
+__host__ __device__ __forceinline__ int lin_diag_off(int dlo) { return (2 - dlo) & ~1; }
+// The class of fewest diagonals that holds the band, the fewest lanes among
+// equals (kLinDiagClasses: none).
+__host__ __device__ __forceinline__ int lin_diag_class_of(int dlo, int wd, int min_lanes) {
+  const int need = dlo + lin_diag_off(dlo) + wd;
+  int best = kLinDiagClasses, slots = 1 << 30;
+  for (int c = 0; c < kLinDiagClasses; ++c) {
+    const LinDiagClass k = lin_diag_class(c);
+    const int s = k.lanes * k.width;
+    if (k.lanes >= min_lanes && s >= need && s <= slots) best = c, slots = s;
+  }
+  return best;
+}
+// Double steps whose moves share a direction word: those a lane unrolls.
+__host__ __device__ constexpr int lin_diag_block(int width) {
+  return width > 12 ? width / 4 : width / 2;
+}
+// Direction words of a pair of l1 + l2 = sum.
+__host__ __device__ __forceinline__ int64_t lin_diag_words(int c, int sum) {
+  const LinDiagClass k = lin_diag_class(c);
+  return (int64_t)((sum > 2 ? (sum - 2) / 2 : 0) / lin_diag_block(k.width) + 1) * (k.width / 2) * k.lanes;
+}
+struct LinDiagOrder {
+  int hist[(kLinDiagClasses + 1) * kLinDiagBuckets];  // pairs per bucket, then cursors
+  // read back in one piece:
+  int base[kLinDiagClasses + 1];     // first position of each class; the pairs of none last
+  unsigned long long total, total4;  // direction words: this kernel's classes, k_lin_dp4 alone
+  int maxwd, err;
+  int counter;
+};
+struct LinDiagArgs {
+  int base[kLinDiagClasses + 1], tasks[kLinDiagClasses + 1];
+  const uint8_t *seq;
+  const LinPlan *plans;
+  const int32_t *order;
+  const int64_t *dm_off;
+  const DevTables *tables;
+  int *counter;
+  uint32_t *dm;
+  int32_t *cost;
+  LinTbArgs tb;
+  DpK k;
+};
+int lin_diag_min_lanes(int n, int sms, bool bt);
+void launch_lin_diag_order(int n, int min_lanes, bool bt, const LinPlan *plans,
+                           const int64_t *dm_words, int64_t *dm_off, LinDiagOrder *os,
+                           int32_t *order, cudaStream_t st);
+int launch_lin_diag(LinDiagArgs &A, bool bt, const int *base, cudaStream_t st);
+int launch_lin_diag_walk(const LinDiagArgs &A, cudaStream_t st);  // after it, the same arguments
 void launch_lin_traceback(const LinTbArgs &A, cudaStream_t st);
 void launch_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
                             const int32_t *a_len, const int32_t *b_len, const int64_t *caps,

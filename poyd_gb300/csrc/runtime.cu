@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -185,19 +186,20 @@ constexpr int kTuneMax = 8;  // variants timed per batch (poyd_tune_result)
 // ---------------------------------------------------------------------------
 // Autotuner (no counterpart in the reference, whose C code has one kernel per
 // operation).  The batched linear DP has several implementations that give
-// identical results: the packed kernel (k_lin_dp4, when the plan finds every
-// value fits 16 bits) or the 32-bit one (k_lin_dp), a persistent grid of 1 to
-// the kernel's maximum resident blocks per SM, and, for batches with a warp
+// identical results: for values that fit 16 bits a block per pair (k_lin_team) or
+// the antidiagonal kernel (k_lin_diag), by the batch's size, or a warp per pair
+// (k_lin_dp4); the 32-bit one (k_lin_dp); of the latter two a persistent grid of 1
+// to the kernel's maximum resident blocks per SM, and, for batches with a warp
 // per pair, the whole-warp small-batch walk or the batched one.  Which is
 // fastest depends on the batch's shape; poyd_autotune_batch times each on a
 // caller's batch and records the winner for the batch's shape class (device,
 // mode, log2 of the pair count, log2 of the widest band), and every later
-// batch of that class launches it.  Without an entry the defaults apply
-// (packed when eligible, the maximum resident grid, the solo walk when
+// batch of that class launches it.  Without an entry the defaults apply (the
+// first two when they can, else the maximum resident grid and the solo walk when
 // every pair has its own warp).  The band itself is always the reference's.
 // ---------------------------------------------------------------------------
 struct LinVariant {
-  int packed;         // 1 packed when eligible, 0 the 32-bit kernel, -1 default
+  int packed;         // 1 k_lin_dp4 when eligible, 0 the 32-bit kernel, -1 default
   int blocks_per_sm;  // 0: the maximum resident
   int solo;           // 1 / 0 small-batch walk on / off, -1 default
 };
@@ -221,6 +223,11 @@ static int sm_count() {
 }
 
 constexpr int kTeamPairsPerSm = 3;
+// k_lin_diag's batches start where its throughput pays: below, a lone warp's steps
+// take longer than k_lin_dp4's.  Costs of 1,500 bp: 700 pairs 408 and 356 us,
+// 1,300 pairs 410 and 470; alignments of 100-1,500 bp: 1,300 pairs 849 and 796 us,
+// 2,600 pairs 1,015 and 1,734.
+constexpr int kDiagPairsPerSm[2] = {8, 12};  // costs, alignments
 
 static int ilog2_64(int64_t x) {
   int r = 0;
@@ -243,13 +250,13 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   LinPlan *plans = (LinPlan *)ws_buffer(w, WS_PLANS, sizeof(LinPlan) * (size_t)n);
   int64_t *dmw = (int64_t *)ws_buffer(w, WS_DMWORDS, sizeof(int64_t) * 2 * (size_t)n);
   int32_t *wdb = (int32_t *)ws_buffer(w, WS_WD, sizeof(int32_t) * 2 * (size_t)n + 16);
-  LinOrderScratch *os = (LinOrderScratch *)ws_buffer(w, WS_ORDSCR, sizeof(LinOrderScratch));
+  // the order scratches of k_lin_diag's batches and of the others
+  LinDiagOrder *dg = (LinDiagOrder *)ws_buffer(w, WS_ORDSCR, sizeof(LinDiagOrder) + sizeof(LinOrderScratch));
   int32_t *dord = (int32_t *)ws_buffer(w, WS_ORDER, sizeof(int32_t) * (size_t)n);
   int *counter = (int *)ws_buffer(w, WS_COUNTER, 64);
-  if (!plans || !dmw || !wdb || !os || !dord || !counter)
+  if (!plans || !dmw || !wdb || !dg || !dord || !counter)
     return fail(POYD_ENOMEM, "plan allocation failed");
-  int32_t *err = &os->pad;  // the plan's error bits travel with the order totals
-  CK(cudaMemsetAsync(os, 0, sizeof(LinOrderScratch), st));
+  LinOrderScratch *os = (LinOrderScratch *)(dg + 1);
   LinPlanArgs PA;
   PA.n = n; PA.seq = seq; PA.a_off = a_off; PA.a_len = a_len; PA.b_off = b_off; PA.b_len = b_len;
   PA.policy = policy; PA.deltaw = deltaw; PA.gap = cm->gap; PA.maxc = maxc;
@@ -257,6 +264,13 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   // keeps only the chosen moves (values x4 must fit the 16-bit profile); the
   // single-pair protocol (out == nullptr) keeps the full direction sets.
   const int mode = !want_align ? kDpCost : ((out && maxc < 16384) ? kDpChoice : kDpSets);
+  // Large batches are ordered for k_lin_diag; the others, and those that prove to
+  // need another kernel, as those want it.
+  const bool diag_order = mode != kDpSets && !ls && n > kDiagPairsPerSm[want_align] * sm_count();
+  // the plan's error bits travel with the order totals
+  int32_t *err = diag_order ? &dg->err : &os->pad;
+  if (diag_order) CK(cudaMemsetAsync(dg, 0, sizeof(LinDiagOrder), st));
+  else CK(cudaMemsetAsync(os, 0, sizeof(LinOrderScratch), st));
   PA.with_dm = mode; PA.dos_empty = (flags & POYD_FLAG_DOS_EMPTY) ? 1 : 0;
   PA.plans = plans; PA.dm_words = dmw; PA.wd_out = wdb; PA.cells = cells; PA.err = err;
   { ProfScope ps("lin_plan", st); launch_lin_plan(PA, st); }
@@ -277,10 +291,13 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   }
   // small batches take pairs in id order (the kernel also zeroes the DP's
   // counters); the others the bucketed longest-first order
-  const bool small = n <= kOrderSmall && !ls;
+  const bool small = n <= kOrderSmall && !ls && !diag_order;
   {
     ProfScope ps("lin_order", st);
-    if (small) launch_lin_order_small(n, plans, dmw, doff, os, counter, batch_done, nbatch, st);
+    if (diag_order)
+      launch_lin_diag_order(n, lin_diag_min_lanes(n, sm_count(), want_align), want_align, plans, dmw, doff, dg,
+                            dord, st);
+    else if (small) launch_lin_order_small(n, plans, dmw, doff, os, counter, batch_done, nbatch, st);
     else launch_lin_order(n, plans, dmw, doff, os, dord, st);
   }
   CK(cudaGetLastError());
@@ -289,13 +306,53 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     int maxwd, err, maxsum, pad;
   } tl;
   static_assert(sizeof(tl) == 24, "order read-back");
-  CK(cudaMemcpyAsync(&tl, &os->total, sizeof tl, cudaMemcpyDeviceToHost, st));
+  struct {
+    int base[kLinDiagClasses + 1];
+    unsigned long long total, total4;
+    int maxwd, err;
+  } dt;
+  static_assert(sizeof(dt) == offsetof(LinDiagOrder, counter) - offsetof(LinDiagOrder, base),
+                "order read-back");
+  if (diag_order) CK(cudaMemcpyAsync(&dt, dg->base, sizeof dt, cudaMemcpyDeviceToHost, st));
+  else CK(cudaMemcpyAsync(&tl, &os->total, sizeof tl, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (diag_order) {
+    tl.total = dt.total4;
+    tl.maxwd = dt.maxwd;
+    tl.err = dt.err;
+    tl.maxsum = 0;
+  }
   if (tl.err & 1) return fail(POYD_EINVAL, "sequences must have length >= 1 (the leading gap)");
   if (tl.err & 2) return fail(POYD_ERANGE, "alignment costs could exceed the 2^24 range of the kernels");
   if (tl.err & 4) return fail(POYD_EINVAL, "sequence codes must be below 32 (5-bit element masks)");
   const int maxwd = std::max(1, tl.maxwd);
-  const int64_t need = want_align ? (int64_t)tl.total : 0;
+  // The packed kernel (four rows per lane in 16-bit halves) runs the batch
+  // when the plan found every pair's values to fit (no err bit 16);
+  // POYD_PACKED=0 keeps the 32-bit kernel.
+  bool packed = !(tl.err & 16) && mode != kDpSets;
+  if (const char *e = std::getenv("POYD_PACKED")) packed = packed && std::atoi(e) != 0;
+  // the launch variant of this batch's shape class (autotuner)
+  LinVariant var{-1, 0, -1};
+  {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    g_last_key = TuneKey(dev, mode == kDpChoice ? 1 : 0, ilog2_64(n), ilog2_64(maxwd));
+    g_last_eligible = packed;
+    if (g_force) {
+      var = *g_force;
+    } else if (mode != kDpSets) {
+      std::lock_guard<std::mutex> lk(g_tune_mu);
+      auto it = g_tune.find(g_last_key);
+      if (it != g_tune.end()) var = it->second;
+    }
+  }
+  if (var.packed == 0) packed = false;
+  // k_lin_diag runs the pairs that its classes hold, unless a tuned variant
+  // asks for another kernel (or the batch is streamed, its results wanted as
+  // they come: k_lin_dp4 walks its pairs on the way).
+  const int diag_n = diag_order ? dt.base[kLinDiagClasses] : 0;
+  bool diag = packed && diag_n > 0 && var.packed < 0 && var.blocks_per_sm == 0 && var.solo < 0;
+  int64_t need = !want_align ? 0 : (int64_t)(diag ? dt.total : tl.total);
   // Waves: consecutive runs of a longest-first order whose direction
   // matrices fit the device-memory budget, one persistent launch each; one
   // wave, with the device order, when the whole batch fits (the usual
@@ -310,6 +367,16 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
       cudaMemGetInfo(&freeb, &totb);
       budget = std::max<int64_t>((int64_t)((double)(freeb + w->size[WS_DM]) * 0.8) / 4, 1);
     }
+  }
+  if (diag && need > budget) {  // the other kernels' waves
+    diag = false;
+    need = (int64_t)tl.total;
+  }
+  if (diag_order && !diag) {
+    CK(cudaMemsetAsync(os, 0, sizeof(LinOrderScratch), st));
+    ProfScope ps("lin_order", st);
+    launch_lin_order(n, plans, dmw, doff, os, dord, st);
+    CK(cudaGetLastError());
   }
   const bool host_waves = need > budget;
   std::vector<int32_t> order;
@@ -360,27 +427,6 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     if (!dm) return fail(POYD_ENOMEM, "direction matrix allocation (%lld bytes) failed",
                          (long long)(max_words * 4));
   }
-  // The packed kernel (four rows per lane in 16-bit halves) runs the batch
-  // when the plan found every pair's values to fit (no err bit 16);
-  // POYD_PACKED=0 keeps the 32-bit kernel.
-  bool packed = !(tl.err & 16) && mode != kDpSets;
-  if (const char *e = std::getenv("POYD_PACKED")) packed = packed && std::atoi(e) != 0;
-  // the launch variant of this batch's shape class (autotuner)
-  LinVariant var{-1, 0, -1};
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    g_last_key = TuneKey(dev, mode == kDpChoice ? 1 : 0, ilog2_64(n), ilog2_64(maxwd));
-    g_last_eligible = packed;
-    if (g_force) {
-      var = *g_force;
-    } else if (mode != kDpSets) {
-      std::lock_guard<std::mutex> lk(g_tune_mu);
-      auto it = g_tune.find(g_last_key);
-      if (it != g_tune.end()) var = it->second;
-    }
-  }
-  if (var.packed == 0) packed = false;
   // A small batch takes a block per pair (k_lin_team) unless a tuned variant
   // says otherwise: up to three pairs an SM, beyond which a warp per pair
   // keeps the SMs busier.
@@ -412,6 +458,25 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)max_words);
     if (!dm) return fail(POYD_ENOMEM, "direction matrix allocation (%lld bytes) failed",
                          (long long)(max_words * 4));
+  }
+  if (diag) {
+    LinDiagArgs GA = {};
+    GA.seq = seq; GA.plans = plans; GA.order = dord; GA.dm_off = doff; GA.tables = tabs;
+    GA.counter = &dg->counter; GA.dm = dm; GA.cost = cost; GA.k = dp_constants();
+    GA.tb.n = n; GA.tb.seq = seq; GA.tb.plans = plans; GA.tb.dm_off = doff; GA.tb.dm = dm;
+    GA.tb.tables = tabs; GA.tb.gap = cm->gap; GA.tb.out = out; GA.tb.out_off = out_off;
+    GA.tb.out_len = out_len; GA.tb.swaped = -1; GA.tb.mode = mode; GA.tb.order = dord;
+    {
+      ProfScope ps(want_align ? "lin_dp_dm" : "lin_dp_cost", st);
+      rc = launch_lin_diag(GA, want_align, dt.base, st);
+    }
+    if (!rc && want_align) {
+      ProfScope ps("lin_traceback", st);
+      rc = launch_lin_diag_walk(GA, st);
+    }
+    if (rc) return rc;
+    if (diag_n == n) return POYD_OK;
+    wave_at.assign({diag_n, n});  // the pairs of wider bands
   }
   int blocks = packed ? lin_dp4_blocks(mode) : lin_dp_blocks(mode);
   if (var.blocks_per_sm > 0) {
@@ -824,6 +889,7 @@ extern "C" int poyd_autotune_batch(const poyd_cm *cm, int32_t align, int32_t n,
   sms = std::max(sms, 1);
   const int mode = align ? kDpChoice : kDpCost;
   std::vector<LinVariant> cands;
+  if (eligible) cands.push_back(dflt);  // k_lin_diag or k_lin_team, which no other variant runs
   for (int pk = eligible ? 1 : 0; pk >= 0; --pk) {
     const int maxb = (pk ? lin_dp4_blocks(mode) : lin_dp_blocks(mode)) / sms;
     for (int b = std::max(maxb, 1); b >= 1 && (int)cands.size() < kTuneMax; --b) {
