@@ -169,6 +169,26 @@ int poyd_pack_alignments(int32_t n, const uint8_t *out, const int64_t *out_off,
                          const int32_t *out_len, uint8_t *packed,
                          const int64_t *packed_off, void *stream);
 
+/* The layouts of such calls (no reference counterpart), from device arrays;
+ * each waits for `stream`.
+ *   poyd_slot_layout: slots of four sequences of cap[i] = len0[i] + len1[i]
+ *     (+ len2[i], unless null) + extra bytes, rounded up to a multiple of 4:
+ *     extra is 2 for poyd_align_2_batch, 0 for the three-sequence calls.
+ *     out_off[i] is the sum of 4 cap[j] over j < i, *total (host) over all.
+ *   poyd_pack_layout: packed_off as poyd_pack_alignments wants it, *total
+ *     (host) the packed bytes, *least (host) the least out_len (negative: a
+ *     traceback that failed).
+ *   poyd_pack_slots: poyd_pack_alignments with the sequences' capacities in
+ *     the place of the lengths; asynchronous. */
+int poyd_slot_layout(int32_t n, const int32_t *len0, const int32_t *len1, const int32_t *len2,
+                     int32_t extra, int64_t *out_off, int64_t *cap, int64_t *total,
+                     void *stream);
+int poyd_pack_layout(int32_t n, const int32_t *out_len, int64_t *packed_off, int64_t *total,
+                     int64_t *least, void *stream);
+int poyd_pack_slots(int32_t n, const uint8_t *out, const int64_t *out_off, const int64_t *cap,
+                    const int32_t *out_len, uint8_t *packed, const int64_t *packed_off,
+                    void *stream);
+
 /* Column operations on aligned pairs (a_i and b_i both len[i] bytes, the
  * output of an alignment), the DP-free externals of sequence.ml:453-758:
  *   median_2_with_gaps: algn_CAML_median_2_with_gaps (algn.c:4011-4024)

@@ -85,6 +85,30 @@ def _stream_handle(stream):
     return C.c_void_p(stream.cuda_stream)
 
 
+def _native_ok(dtype, *tensors) -> bool:
+    """Whether a kernel on the current device can read the tensors as they are."""
+    return all(t.is_cuda and t.dtype == dtype and t.is_contiguous() and
+               t.device.index == torch.cuda.current_device() for t in tensors)
+
+
+def slot_layout(lens, extra: int):
+    """(offsets, total bytes, capacities) of output slots of 4 sequences of
+    capacity sum(lens) + extra, rounded up to a multiple of 4."""
+    n = int(lens[0].numel())
+    if n and all(t.dim() == 1 and t.numel() == n for t in lens) and _native_ok(torch.int32, *lens):
+        off = torch.empty(n, dtype=torch.int64, device=lens[0].device)
+        cap, total = torch.empty_like(off), C.c_int64()
+        check(lib().poyd_slot_layout(
+            n, lens[0].data_ptr(), lens[1].data_ptr(), lens[2].data_ptr() if len(lens) > 2 else None,
+            extra, off.data_ptr(), cap.data_ptr(), C.byref(total), _stream_handle(None)))
+        return off, total.value, cap
+    cap = (sum(t.to(torch.int64) for t in lens) + extra + 3) // 4 * 4
+    sizes = 4 * cap
+    off = torch.zeros_like(sizes)
+    off[1:] = torch.cumsum(sizes, 0)[:-1]
+    return off, int((off[-1] + sizes[-1]).item()) if n else 0, cap
+
+
 class PairBatch:
     """Pairs (a_i, b_i) packed in one device byte buffer.
 
@@ -135,11 +159,7 @@ class PairBatch:
     def out_layout(self):
         """Per-pair output slot offsets: 4 sequences of cap = la + lb + 2
         rounded up to a multiple of 4 (the library's slot_cap)."""
-        cap = (self.a_len.to(torch.int64) + self.b_len.to(torch.int64) + 2 + 3) // 4 * 4
-        sizes = 4 * cap
-        off = torch.zeros_like(sizes)
-        off[1:] = torch.cumsum(sizes, 0)[:-1]
-        return off, int((off[-1] + sizes[-1]).item()) if self.n else 0, cap
+        return slot_layout((self.a_len, self.b_len), 2)
 
 
 def cost_2(batch: PairBatch, cm: CostMatrix, deltaw=None, band_cells: bool = False,
@@ -209,6 +229,20 @@ class AlignResult:
         only the bytes that hold results."""
         n = self.cost.numel()
         dev = self.cost.device
+        if n and _native_ok(torch.int32, self.out_len) and \
+                _native_ok(torch.int64, self.out_off, self.cap) and \
+                self.out_len.numel() == 2 * n and self.cap.numel() == n == self.out_off.numel():
+            off = torch.empty(n, dtype=torch.int64, device=dev)
+            total, least = C.c_int64(), C.c_int64()
+            check(lib().poyd_pack_layout(n, self.out_len.data_ptr(), off.data_ptr(), C.byref(total),
+                                         C.byref(least), _stream_handle(None)))
+            if least.value >= 0:
+                packed = torch.empty(max(total.value, 16), dtype=torch.uint8, device=dev)
+                check(lib().poyd_pack_slots(
+                    n, self.out.data_ptr(), self.out_off.data_ptr(), self.cap.data_ptr(),
+                    self.out_len.data_ptr(), packed.data_ptr(), off.data_ptr(),
+                    _stream_handle(stream)))
+                return PackedAlignments(self.cost, packed[:total.value], self.out_len)
         ln = self.out_len.view(-1, 2).to(torch.int64)
         sizes = 3 * ln[:, 0] + ln[:, 1]
         off = torch.cumsum(sizes, 0) - sizes

@@ -82,6 +82,8 @@ extern "C" int poyd_workspace_release(void) {
   return POYD_OK;
 }
 
+size_t ws_size(const Workspace *w, int slot) { return w->size[slot]; }
+
 void *ws_buffer(Workspace *w, int slot, size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (w->size[slot] >= bytes) return w->ptr[slot];

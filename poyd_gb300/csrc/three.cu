@@ -190,11 +190,54 @@ __global__ void __launch_bounds__(kP3Threads) k_p3(const __grid_constant__ P3Arg
   }
 }
 
+// Cost_matrix.Three_D.of_two_dim_comb (cost_matrix.ml:803-851): the median
+// of (i, j, k) is the lowest single state l with the least
+// cost[l][i] + cost[l][j] + cost[l][k]; the gap takes part only for metric
+// matrices or when two of i, j, k hold it.  The reference seeds each entry
+// with OCaml's max_int, which fits a C int on a 32-bit OCaml only (on a
+// 64-bit one it truncates to -1 and no entry is ever set); this follows the
+// 32-bit reading.
+static uint8_t median3_of(const poyd_cm *cm, int i, int j, int k) {
+  int64_t best = INT64_MAX;
+  int med = 0;
+  for (int l = 0; l < cm->lcm; ++l) {
+    const int x = 1 << l;
+    const int shared = ((i & x) != 0) + ((j & x) != 0) + ((k & x) != 0);
+    int64_t c = INT64_MAX;
+    if (cm->is_metric || shared >= 2 || x != cm->gap)
+      c = (int64_t)cm->cost[(x << 5) + i] + cm->cost[(x << 5) + j] + cm->cost[(x << 5) + k];
+    if (c < best) {
+      best = c;
+      med = x;
+    } else if (c == best) {
+      med |= x;
+    }
+  }
+  return (uint8_t)(med & -med);
+}
+static void median3_table(const poyd_cm *cm, uint8_t *tab) {
+  std::memset(tab, 0, 32768);
+  for (int i = 1; i < 32; ++i)
+    for (int j = 1; j < 32; ++j)
+      for (int k = 1; k < 32; ++k) tab[(i << 10) | (j << 5) | k] = median3_of(cm, i, j, k);
+}
+
+// The lengths side by side, for one copy to the host.
+__global__ void k_p3_lens(int n, const int32_t *a, const int32_t *b, const int32_t *c,
+                          const int32_t *d, int32_t *out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[i] = a[i];
+  out[n + i] = b[i];
+  out[2 * (int64_t)n + i] = c[i];
+  if (d) out[3 * (int64_t)n + i] = d[i];
+}
+
 // Host side shared by the two batched entry points.
 static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const off[4],
                   const int32_t *const len[4], int mm, int go, int ge, int gap,
-                  const uint8_t *median3, int32_t *cost, uint8_t *out, const int64_t *out_off,
-                  int32_t *out_len, int32_t *changed, cudaStream_t st) {
+                  const uint8_t *median3, const poyd_cm *median_cm, int32_t *cost, uint8_t *out,
+                  const int64_t *out_off, int32_t *out_len, int32_t *changed, cudaStream_t st) {
   if (n < 0) return fail(POYD_EINVAL, "three-sequence batch: n < 0");
   if (n == 0) return POYD_OK;
   if (!seq || !cost || !out || !out_off || !out_len || (mode == 1 && !changed))
@@ -204,12 +247,18 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   const int nq = mode == 1 ? 4 : 3;
   for (int q = 0; q < nq; ++q)
     if (!off[q] || !len[q]) return fail(POYD_EINVAL, "three-sequence batch: null argument");
-  std::vector<int32_t> hl[4];
-  for (int q = 0; q < nq; ++q) {
-    hl[q].resize(n);
-    CK3(cudaMemcpyAsync(hl[q].data(), len[q], sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
-  }
+  Workspace *w = workspace(st);
+  // the lengths to the host, in one copy
+  int32_t *dlen = (int32_t *)ws_buffer(w, WS_P3_LENS, sizeof(int32_t) * (size_t)n * nq);
+  if (!dlen) return fail(POYD_ENOMEM, "three-sequence workspace");
+  k_p3_lens<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, len[0], len[1], len[2],
+                                                        nq == 4 ? len[3] : nullptr, dlen);
+  CK3(cudaGetLastError());
+  std::vector<int32_t> all_len((size_t)n * nq);
+  CK3(cudaMemcpyAsync(all_len.data(), dlen, sizeof(int32_t) * (size_t)n * nq, cudaMemcpyDeviceToHost, st));
   CK3(cudaStreamSynchronize(st));
+  const int32_t *hl[4];
+  for (int q = 0; q < 4; ++q) hl[q] = all_len.data() + (size_t)n * std::min(q, nq - 1);
   int64_t ring_max = 0, dir_max = 0, lin_plane = 0, lin_dir = 0;
   int64_t open_plane = 0, open_dir = 0;
   int smax = 16, max_b = 1;
@@ -243,14 +292,23 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   int dev = 0, sms = 0;
   CK3(cudaGetDevice(&dev));
   CK3(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  size_t fr = 0, tot = 0;
-  CK3(cudaMemGetInfo(&fr, &tot));
-  // the choices dominate: one set per resident block, sized for the largest
-  // triple; by default at most 60 % of the free memory, 120 GiB
-  int64_t budget = std::min<int64_t>((int64_t)(fr * 0.6), 120LL << 30);
-  if (const char *e = getenv("POYD_P3_BUDGET_MB")) budget = std::max<int64_t>(1, atoll(e)) << 20;
-
-  Workspace *w = workspace(st);
+  // Blocks of a launch whose buffers take ring + dir bytes each.  The choices
+  // dominate: one set per resident block, sized for the largest triple; by default
+  // at most 60 % of the free memory, 120 GiB (asked for only where the buffers do
+  // not hold the launch already).
+  auto fit = [&](int64_t want, int64_t ring, int64_t dir) -> int64_t {
+    int64_t budget;
+    if (const char *e = getenv("POYD_P3_BUDGET_MB")) {
+      budget = std::max<int64_t>(1, atoll(e)) << 20;
+    } else {
+      if ((size_t)(ring * want) <= ws_size(w, WS_P3_RING) && (size_t)(dir * want) <= ws_size(w, WS_P3_DIR))
+        return want;
+      size_t fr = 0, tot = 0;
+      if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return 1;
+      budget = std::min<int64_t>((int64_t)(fr * 0.6), 120LL << 30);
+    }
+    return std::min(want, std::max<int64_t>(1, budget / (ring + dir)));
+  };
   int32_t *meta = (int32_t *)ws_buffer(w, WS_P3_META, sizeof(int32_t) * ((size_t)n + 4));
   if (!meta) return fail(POYD_ENOMEM, "three-sequence workspace");
   order.push_back(0);  // counter
@@ -278,14 +336,15 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   A.go = go;
   A.ge = ge;
   A.gap = gap;
-  A.has_med = median3 ? 1 : 0;
+  A.has_med = median3 || median_cm ? 1 : 0;
   {
     static const int st5[5] = {1, 2, 4, 8, 16};
     for (int x = 0; x < 5; ++x)
       for (int y = 0; y < 5; ++y)
         for (int z = 0; z < 5; ++z)
           A.med[25 * x + 5 * y + z] =
-              median3 ? median3[(st5[x] << 10) | (st5[y] << 5) | st5[z]] : (uint8_t)gap;
+              median_cm ? median3_of(median_cm, st5[x], st5[y], st5[z])
+              : median3 ? median3[(st5[x] << 10) | (st5[y] << 5) | st5[z]] : (uint8_t)gap;
   }
   A.smax = smax;
   // the launch's error bits; bit 2: an optimum reached the 16-bit clamp, the
@@ -320,9 +379,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     int warps = 1;
     const int most = (int64_t)n * 4 >= 8LL * sms ? 4 : 16;
     while (2 * warps <= most && 2 * warps * kP3LinLag <= longest + 40) warps *= 2;
-    const int64_t per = lin_plane + lin_dir;
-    const int blocks = (int)std::min<int64_t>(
-        {(int64_t)n, (int64_t)p3_linear_blocks(warps, longest), std::max<int64_t>(1, budget / per)});
+    const int blocks = (int)fit(std::min<int64_t>(n, p3_linear_blocks(warps, longest)), lin_plane, lin_dir);
     uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(lin_plane * blocks));
     uint8_t *dirb = (uint8_t *)ws_buffer(w, WS_P3_DIR, (size_t)(lin_dir * blocks));
     if (!plane || !dirb) return fail(POYD_ENOMEM, "three-sequence workspace (%d blocks)", blocks);
@@ -343,8 +400,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     int csize = ce && ce[0] == '0' ? 1 : (int)std::min<int64_t>(
         {8, (useful + p3_open_warps() - 1) / p3_open_warps(), std::max<int64_t>(1, sms / n)});
     while (csize > 1 && p3_open_clusters(csize) < n) --csize;
-    const int64_t per = open_plane + open_dir;
-    int blocks = (int)std::min<int64_t>({(int64_t)n, 2LL * sms, std::max<int64_t>(1, budget / per)});
+    int blocks = (int)fit(std::min<int64_t>(n, 2LL * sms), open_plane, open_dir);
     uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(open_plane * blocks));
     uint8_t *dirb = (uint8_t *)ws_buffer(w, WS_P3_DIR, (size_t)(open_dir * blocks));
     if (!plane || !dirb) return fail(POYD_ENOMEM, "three-sequence workspace (%d blocks)", blocks);
@@ -356,8 +412,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     rc = finish(&redo);
     if (rc || !redo) return rc;
   }
-  const int64_t per_block = ring_max * 4 + dir_max * 8;
-  const int64_t blocks = std::min<int64_t>({(int64_t)n, 3LL * sms, std::max<int64_t>(1, budget / per_block)});
+  const int64_t blocks = fit(std::min<int64_t>(n, 3LL * sms), ring_max * 4, dir_max * 8);
   A.ring = (int32_t *)ws_buffer(w, WS_P3_RING, (size_t)(ring_max * 4 * blocks));
   A.dir = (uint64_t *)ws_buffer(w, WS_P3_DIR, (size_t)(dir_max * 8 * blocks));
   if (!A.ring || !A.dir)
@@ -371,37 +426,6 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   }
   bool redo = false;
   return finish(&redo);
-}
-
-// Cost_matrix.Three_D.of_two_dim_comb (cost_matrix.ml:803-851): the median
-// of (i, j, k) is the lowest single state l with the least
-// cost[l][i] + cost[l][j] + cost[l][k]; the gap takes part only for metric
-// matrices or when two of i, j, k hold it.  The reference seeds each entry
-// with OCaml's max_int, which fits a C int on a 32-bit OCaml only (on a
-// 64-bit one it truncates to -1 and no entry is ever set); this follows the
-// 32-bit reading.
-static void median3_table(const poyd_cm *cm, uint8_t *tab) {
-  std::memset(tab, 0, 32768);
-  for (int i = 1; i < 32; ++i)
-    for (int j = 1; j < 32; ++j)
-      for (int k = 1; k < 32; ++k) {
-        int64_t best = INT64_MAX;
-        int med = 0;
-        for (int l = 0; l < cm->lcm; ++l) {
-          const int x = 1 << l;
-          const int shared = ((i & x) != 0) + ((j & x) != 0) + ((k & x) != 0);
-          int64_t c = INT64_MAX;
-          if (cm->is_metric || shared >= 2 || x != cm->gap)
-            c = (int64_t)cm->cost[(x << 5) + i] + cm->cost[(x << 5) + j] + cm->cost[(x << 5) + k];
-          if (c < best) {
-            best = c;
-            med = x;
-          } else if (c == best) {
-            med |= x;
-          }
-        }
-        tab[(i << 10) | (j << 5) | k] = (uint8_t)(med & -med);
-      }
 }
 
 }  // namespace poyd
@@ -424,7 +448,7 @@ extern "C" int poyd_powell_3d_batch(int32_t n, const uint8_t *seq, const int64_t
                                     const int64_t *out_off, int32_t *out_len, void *stream) {
   const int64_t *off[4] = {a_off, b_off, c_off, nullptr};
   const int32_t *len[4] = {a_len, b_len, c_len, nullptr};
-  return p3_run(0, n, seq, off, len, mm, go, ge, 16, median3, cost, out, out_off, out_len,
+  return p3_run(0, n, seq, off, len, mm, go, ge, 16, median3, nullptr, cost, out, out_off, out_len,
                 nullptr, (cudaStream_t)stream);
 }
 
@@ -441,11 +465,9 @@ extern "C" int poyd_readjust_3d_batch(const poyd_cm *cm, int32_t n, const uint8_
   // align_3_powell_inter's parameters (sequence.ml:1091-1102)
   const int mm = cm->cost[(1 << 5) + 2], ge = cm->cost[(1 << 5) + 16];
   const int go = cm->cost_model == 1 ? cm->gap_open : 0;
-  static thread_local uint8_t tab[32768];
-  median3_table(cm, tab);
   const int64_t *off[4] = {s1_off, s2_off, p_off, m_off};
   const int32_t *len[4] = {s1_len, s2_len, p_len, m_len};
-  return p3_run(1, n, seq, off, len, mm, go, ge, cm->gap, tab, cost, out, out_off, out_len,
+  return p3_run(1, n, seq, off, len, mm, go, ge, cm->gap, nullptr, cm, cost, out, out_off, out_len,
                 changed, (cudaStream_t)stream);
 }
 

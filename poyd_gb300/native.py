@@ -81,10 +81,11 @@ EXPORTED = (
     "poyd_nonadd16_median_3_batch", "poyd_nonadd16_median_batch",
     "poyd_nonadd32_distance_batch", "poyd_nonadd32_median_3_batch",
     "poyd_nonadd32_median_batch", "poyd_nonadd8_distance_batch", "poyd_nonadd8_median_3_batch",
-    "poyd_nonadd8_median_batch", "poyd_pack_alignments", "poyd_powell_3D_align",
+    "poyd_nonadd8_median_batch", "poyd_pack_alignments", "poyd_pack_layout", "poyd_pack_slots",
+    "poyd_powell_3D_align",
     "poyd_powell_3d_batch", "poyd_profile_enable", "poyd_profile_read", "poyd_readjust_3d_batch",
     "poyd_relu_grad_bf16", "poyd_sank_distance_batch",
-    "poyd_sank_median_3_batch", "poyd_sank_median_batch", "poyd_to_bf16", "poyd_verify_2_batch", "poyd_version",
+    "poyd_sank_median_3_batch", "poyd_sank_median_batch", "poyd_slot_layout", "poyd_to_bf16", "poyd_verify_2_batch", "poyd_version",
     "poyd_workspace_release", "poyd_worst_2_batch",
 )
 
@@ -115,6 +116,10 @@ SIGNATURES = [
     ("poyd_launch_count", C.c_longlong, []),
     ("poyd_pack_alignments", C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                        C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    ("poyd_slot_layout", C.c_int, [_i32, _vp, _vp, _vp, _i32, _vp, _vp, C.POINTER(C.c_int64), _vp]),
+    ("poyd_pack_layout", C.c_int, [_i32, _vp, _vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64),
+                                   _vp]),
+    ("poyd_pack_slots", C.c_int, [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     ("poyd_align_2_host", C.c_int, [_cmp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                     C.c_int64, _vp, _vp, _i32]),
     ("poyd_algn_align_2d", C.c_int, [_vp, _i32, _vp, _i32, _cmp, _vp, _vp, _vp, _i32, _vp, _i32,

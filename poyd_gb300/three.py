@@ -13,7 +13,7 @@ import ctypes as C
 import numpy as np
 import torch
 
-from .align import CostMatrix, _stream_handle
+from .align import CostMatrix, _stream_handle, slot_layout
 from .native import check, lib
 
 
@@ -55,14 +55,8 @@ class TripleBatch:
     def out_layout(self):
         """Slots of 4 sequences of cap = a + b + c (first three lengths)
         rounded up to a multiple of 4."""
-        tot = self.lens[0].to(torch.int64) + self.lens[1].to(torch.int64)
-        tot = tot + (self.lens[3] if len(self.lens) == 4 else self.lens[2]).to(torch.int64)
-        cap = (tot + 3) // 4 * 4
-        sizes = 4 * cap
-        off = torch.zeros_like(sizes)
-        if self.n:
-            off[1:] = torch.cumsum(sizes, 0)[:-1]
-        return off, int((off[-1] + sizes[-1]).item()) if self.n else 0, cap
+        third = self.lens[3] if len(self.lens) == 4 else self.lens[2]
+        return slot_layout((self.lens[0], self.lens[1], third), 0)
 
 
 class ThreeResult:
