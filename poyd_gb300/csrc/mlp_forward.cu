@@ -3,20 +3,26 @@
 // with the activations written out, the training forward.
 //
 // A CTA keeps all three weight matrices in shared memory (208 KB, staged once)
-// and runs 128-row tiles through the layers.  Per tile:
-//   * layer 1: A = the tile's bf16 inputs in shared memory, D in TMEM columns
-//     0-255 (region 0);
-//   * the epilogue reads a row's sums with tcgen05.ld (one thread per row and
-//     half of the columns), adds the bias, applies ReLU, rounds to bf16 and
+// and runs 128-row tiles through the layers.  TMEM is two regions of 256 columns,
+// P and Q, which change places from tile to tile.  Per tile:
+//   * layer 1: A = the tile's bf16 inputs in shared memory, D in P;
+//   * the epilogue reads a row's sums with tcgen05.ld (sixteen warps, a thread per
+//     row and 32 columns of each half of the layer), adds the bias, applies ReLU, rounds to bf16 and
 //     writes the packed values back with tcgen05.st over columns it has read:
 //     the next layer's A operand never leaves TMEM, which is what leaves the
 //     shared memory to the weights;
-//   * layer 2: A from region 0, D in region 1; layer 3: A from region 1, D in
-//     region 0; then the 128 -> 1 head from registers.
-// Measured: 984,102 rows from fp32 in 0.29 ms (0.72 PFLOP/s) where the
-// mma.sync kernel with its weights in L2 took 1.21 ms, the input's conversion
-// and the weights' transposes 33 us more.  What bounds it: the chain of a
-// tile's products and epilogues, which share the one set of TMEM columns.
+//   * layer 2: A from P, D in Q; layer 3: A from Q, D in P's first half.  A
+//     layer's products over the first half of its k start when that half of its A
+//     is ready and run beside the other half's epilogue;
+//   * the 128 -> 1 head from registers by four warps of its own, while the others
+//     take the next tile's layer 1, whose sums go to Q.
+// Measured: 984,102 rows from fp32 in 0.227 ms (0.93 PFLOP/s) where eight warps
+// with one tile's products and epilogues in turn took 0.29 ms, and the mma.sync
+// kernel with its weights in L2 1.21 ms, the input's conversion and the weights'
+// transposes 33 us more.  What bounds it: the chain of a tile, 0.144 ms of it the
+// products and the waits around them (0.11 at the tensor cores' rate); a second
+// tile's products beside it would want 1,024 TMEM columns.  Layer 2 in halves of
+// n, its first half's epilogue beside the second's products, took 0.238 ms.
 //
 // Every layer accumulates k in ascending chunks of 16 from zero and the head
 // sums as k_head_forward does (lane-strided, then the xor butterfly's tree).
@@ -32,7 +38,7 @@
 namespace poyd {
 namespace {
 
-constexpr int kMRows = 128, kMThreads = 256;
+constexpr int kMRows = 128, kMMain = 512, kMThreads = kMMain + 128;
 constexpr int kMIn = 32, kMH1 = 256, kMH2 = 256, kMH3 = 128;
 __host__ __device__ constexpr int m_sbo(int k) { return k / 8 * 128 + 16; }
 constexpr uint32_t kMW1 = 0;
@@ -41,9 +47,9 @@ constexpr uint32_t kMW3 = kMW2 + kMH2 / 8 * m_sbo(kMH1);
 constexpr uint32_t kMX = kMW3 + kMH3 / 8 * m_sbo(kMH2);
 constexpr uint32_t kMBias = kMX + kMRows / 8 * m_sbo(kMIn);  // b1, b2, b3, w4 (fp32)
 constexpr uint32_t kMBar = kMBias + 4 * (kMH1 + kMH2 + 2 * kMH3);
-constexpr uint32_t kMSmem = kMBar + 32 + 128;  // + alignment slack
+constexpr uint32_t kMSmem = kMBar + 48 + 128;  // + alignment slack
 static_assert(kMSmem <= 227 * 1024, "weights, inputs and biases fit one CTA");
-constexpr int kMWaitMax = 1 << 22;  // mbarrier polls before a wait gives up
+constexpr int kMWaitMax = 1 << 20;  // waits of a microsecond before one gives up
 
 struct MlpFwdArgs {
   const void *X;
@@ -91,10 +97,10 @@ __device__ __forceinline__ bool m_wait(uint32_t bar, uint32_t parity) {
   for (int i = 0; i < kMWaitMax; ++i) {
     uint32_t ok;
     asm volatile(
-        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
         "selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(1000)
         : "memory");
     if (ok) return true;
   }
@@ -128,12 +134,33 @@ __device__ __forceinline__ void m_before() {
 __device__ __forceinline__ void m_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ uint32_t m_relu2(float lo, float hi) {
-  lo = lo > 0.f ? lo : 0.f;
-  hi = hi > 0.f ? hi : 0.f;
+__device__ __forceinline__ uint32_t m_relu2(float lo, float hi) {  // NaN becomes 0
+  lo = fmaxf(lo, 0.f);
+  hi = fmaxf(hi, 0.f);
   uint32_t d;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
+}
+// {a, b} + {x, y}, ReLU, bf16
+__device__ __forceinline__ uint32_t m_bias_relu(uint32_t a, uint32_t b, float x, float y) {
+  float lo, hi;
+  asm("{\n.reg .b64 s, t;\nmov.b64 s, {%2, %3};\nmov.b64 t, {%4, %5};\nadd.rn.f32x2 s, s, t;\n"
+      "mov.b64 {%0, %1}, s;\n}\n"
+      : "=f"(lo), "=f"(hi)
+      : "r"(a), "r"(b), "f"(x), "f"(y));
+  return m_relu2(lo, hi);
+}
+// Barrier of the sixteen warps of the hidden layers; whether any of them saw `bad`
+// (the same answer for all).
+__device__ __forceinline__ bool m_main_sync(int bad) {
+  int any;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\n"
+      "selp.s32 %0, 1, 0, q;\n}\n"
+      : "=r"(any)
+      : "r"(bad), "n"(kMMain)
+      : "memory");
+  return any != 0;
 }
 
 // Stages a K x N weight matrix as the K-major B operand at `dst`.
@@ -178,41 +205,85 @@ __device__ __forceinline__ void m_stage_w(uint8_t *dst, const uint16_t *W, int K
   }
 }
 
-// Eight inputs (one core matrix row) of row m, zero past M.
-__device__ __forceinline__ uint4 m_load_x(const MlpFwdArgs &A, int64_t m, int kc) {
-  if (m >= A.M) return make_uint4(0, 0, 0, 0);
-  if (!A.x32) return *reinterpret_cast<const uint4 *>((const uint16_t *)A.X + m * kMIn + kc * 8);
-  const float4 *p = reinterpret_cast<const float4 *>((const float *)A.X + m * kMIn + kc * 8);
-  const float4 u = p[0], v = p[1];
-  uint4 r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.x) : "f"(u.y), "f"(u.x));
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.y) : "f"(u.w), "f"(u.z));
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.z) : "f"(v.y), "f"(v.x));
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.w) : "f"(v.w), "f"(v.z));
-  return r;
+// Eight inputs (one core matrix row) of row m as they lie in memory, zero past M.
+struct MlpX {
+  uint4 u, v;
+};
+__device__ __forceinline__ MlpX m_load_x(const MlpFwdArgs &A, int64_t m, int kc) {
+  MlpX x;
+  x.u = x.v = make_uint4(0, 0, 0, 0);
+  if (m >= A.M) return x;
+  if (A.x32) {
+    const uint4 *p = reinterpret_cast<const uint4 *>((const float *)A.X + m * kMIn + kc * 8);
+    x.u = p[0], x.v = p[1];
+  } else {
+    x.u = *reinterpret_cast<const uint4 *>((const uint16_t *)A.X + m * kMIn + kc * 8);
+  }
+  return x;
+}
+__device__ __forceinline__ uint4 m_bf16_x(const MlpFwdArgs &A, const MlpX &x) {
+  if (!A.x32) return x.u;
+  auto two = [](uint32_t lo, uint32_t hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+    return d;
+  };
+  return make_uint4(two(x.u.x, x.u.y), two(x.u.z, x.u.w), two(x.v.x, x.v.y), two(x.v.z, x.v.w));
 }
 
-// One hidden layer's epilogue for this thread's row and half of 256 columns:
-// the sums at `reg` become the next layer's packed A operand in place (and,
-// when H is given, row-major activations).
+// A hidden layer's epilogue for this thread's row and 32 columns: the sums at
+// `reg` become the next layer's packed A operand in place (and, when h is
+// given, row-major activations).
 __device__ __forceinline__ void m_epilogue(uint32_t reg, const float *bias, uint16_t *h) {
+  uint32_t r[32], p[16];
+  m_ld32(r, reg);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 bb = *reinterpret_cast<const float4 *>(bias + 4 * q);
+    p[2 * q] = m_bias_relu(r[4 * q], r[4 * q + 1], bb.x, bb.y);
+    p[2 * q + 1] = m_bias_relu(r[4 * q + 2], r[4 * q + 3], bb.z, bb.w);
+  }
+  m_st16(reg, p);
+  if (h) {
+    uint4 *o = reinterpret_cast<uint4 *>(h);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o[q] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// The third layer's epilogue and the head of this thread's row: s[l] sums
+// columns l, l + 32, l + 64, l + 96, then the butterfly's tree over l.
+__device__ __forceinline__ float m_head(uint32_t reg, const float *b3, const float *w4, uint16_t *h) {
+  float s[32];
+#pragma unroll
+  for (int l = 0; l < 32; ++l) s[l] = 0.f;
 #pragma unroll 1
   for (int c = 0; c < 4; ++c) {
-    uint32_t r[32], p[16];
+    uint32_t r[32];
     m_ld32(r, reg + 32 * c);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const float2 bb = *reinterpret_cast<const float2 *>(bias + 32 * c + 2 * q);
-      p[q] = m_relu2(__uint_as_float(r[2 * q]) + bb.x, __uint_as_float(r[2 * q + 1]) + bb.y);
+    for (int q = 0; q < 8; ++q) {
+      const float4 bb = *reinterpret_cast<const float4 *>(b3 + 32 * c + 4 * q);
+      const float4 ww = *reinterpret_cast<const float4 *>(w4 + 32 * c + 4 * q);
+      r[2 * q] = m_bias_relu(r[4 * q], r[4 * q + 1], bb.x, bb.y);
+      r[2 * q + 1] = m_bias_relu(r[4 * q + 2], r[4 * q + 3], bb.z, bb.w);
+      s[4 * q] = fmaf(__uint_as_float(r[2 * q] << 16), ww.x, s[4 * q]);
+      s[4 * q + 1] = fmaf(__uint_as_float(r[2 * q] & 0xFFFF0000u), ww.y, s[4 * q + 1]);
+      s[4 * q + 2] = fmaf(__uint_as_float(r[2 * q + 1] << 16), ww.z, s[4 * q + 2]);
+      s[4 * q + 3] = fmaf(__uint_as_float(r[2 * q + 1] & 0xFFFF0000u), ww.w, s[4 * q + 3]);
     }
-    m_st16(reg + 16 * c, p);
     if (h) {
       uint4 *o = reinterpret_cast<uint4 *>(h + 32 * c);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+      for (int q = 0; q < 4; ++q) o[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
     }
   }
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int l = 0; l < o; ++l) s[l] += s[l + o];
+  return s[0];
 }
 
 __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_constant__ MlpFwdArgs A) {
@@ -220,19 +291,24 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
   uint8_t *sm = mlp_raw + ((128 - ((uint32_t)__cvta_generic_to_shared(mlp_raw) & 127)) & 127);
   const uint32_t sb = (uint32_t)__cvta_generic_to_shared(sm);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int half = warp >> 2;                       // columns 128 half ..
+  const int quarter = warp >> 2;                    // columns 32 quarter .. of a half; 4: the head
   const int row = (warp & 3) * 32 + lane;           // this thread's TMEM lane
   float *bias = reinterpret_cast<float *>(sm + kMBias);
-  const uint32_t bar = sb + kMBar;
-  uint32_t *slot = reinterpret_cast<uint32_t *>(sm + kMBar + 16);
+  // mbarriers: layers 1, 2, 3 done; the head has read its sums
+  const uint32_t bar1 = sb + kMBar, bar2 = bar1 + 8, bar3 = bar1 + 16, bar_head = bar1 + 24;
+  uint32_t *slot = reinterpret_cast<uint32_t *>(sm + kMBar + 32);
+  volatile int *dead = reinterpret_cast<volatile int *>(sm + kMBar + 40);
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sb + kMBar + 16)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sb + kMBar + 32)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    for (int q = 0; q < 4; ++q)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar1 + 8 * q), "r"(q == 3 ? 4 : 1)
+                   : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *dead = 0;
   }
   m_stage_w(sm + kMW1, A.W[0], kMIn, kMH1, A.trans);
   m_stage_w(sm + kMW2, A.W[1], kMH1, kMH2, A.trans);
@@ -241,124 +317,113 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
     bias[i] = i < 256 ? A.b[0][i] : i < 512 ? A.b[1][i - 256] : i < 640 ? A.b[2][i - 512]
               : __uint_as_float((uint32_t)A.w4[i - 640] << 16);
   const int tiles = (A.M + kMRows - 1) / kMRows;
-  // a thread's two core matrix rows of an input tile
-  auto put_x = [&](int e, uint4 v) {
-    const int r = (e & 7) | e >> 5 << 3, kc = e >> 3 & 3;
-    *reinterpret_cast<uint4 *>(sm + kMX + (r >> 3) * m_sbo(kMIn) + kc * 128 + (r & 7) * 16) = v;
+  // a main thread's core matrix row of an input tile
+  auto put_x = [&](const MlpX &x) {
+    const int r = (tid & 7) | tid >> 5 << 3, kc = tid >> 3 & 3;
+    *reinterpret_cast<uint4 *>(sm + kMX + (r >> 3) * m_sbo(kMIn) + kc * 128 + (r & 7) * 16) = m_bf16_x(A, x);
   };
-  auto get_x = [&](int t, int e) {
-    return m_load_x(A, (int64_t)t * kMRows + ((e & 7) | e >> 5 << 3), e >> 3 & 3);
+  auto get_x = [&](int t) {
+    return m_load_x(A, (int64_t)t * kMRows + ((tid & 7) | tid >> 5 << 3), tid >> 3 & 3);
   };
-  int t = blockIdx.x;
-  if (t < tiles) {
-    put_x(tid, get_x(t, tid));
-    put_x(tid + kMThreads, get_x(t, tid + kMThreads));
-  }
+  if (tid < kMMain && (int)blockIdx.x < tiles) put_x(get_x(blockIdx.x));
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // staged operands
   m_before();
   __syncthreads();
   m_after();
   const uint32_t tm = *slot;
   const uint32_t lane_base = (uint32_t)(warp & 3) << 21;  // TMEM lane 32 (warp % 4) in bits 16-
-  const uint32_t mine = tm + lane_base + 128 * half;
-  uint32_t parity = 0;
-  bool dead = false;
-  // all threads: wait for the committed products (bounded)
-  auto wait_mma = [&]() {
-    const bool ok = m_wait(bar, parity);
-    parity ^= 1;
-    dead = __syncthreads_or(!ok);
+  auto layer1 = [&](uint32_t d) {
+    for (int k = 0; k < kMIn / 16; ++k)
+      m_mma_ss(d, m_desc(sb + kMX + 256 * k, m_sbo(kMIn)), m_desc(sb + kMW1 + 256 * k, m_sbo(kMIn)),
+               m_idesc(kMH1), k);
+    m_commit(bar1);
+  };
+  // n columns of a layer over half h of its k.  Its packed A: 16 columns of each 32
+  // that the sums had
+  auto half = [&](uint32_t d, uint32_t a, uint32_t w, int h, int n) {
+#pragma unroll
+    for (int k = 8 * h; k < 8 * h + 8; ++k)
+      m_mma_ts(d, a + 32 * (k >> 1) + 8 * (k & 1), m_desc(sb + w + 256 * k, m_sbo(kMH1)), m_idesc(n), k);
+  };
+  // A wait that runs out marks the CTA; the main warps leave together after the
+  // next barrier, the head's before their next tile.
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (!m_wait(bar, parity)) *dead = 1;
     m_after();
   };
-  for (; t < tiles && !dead; t += gridDim.x) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // staged operands
-    m_before();
-    __syncthreads();
-    if (tid == 0) {
-      m_after();
-      for (int k = 0; k < kMIn / 16; ++k)
-        m_mma_ss(tm, m_desc(sb + kMX + 256 * k, m_sbo(kMIn)), m_desc(sb + kMW1 + 256 * k, m_sbo(kMIn)),
-                 m_idesc(kMH1), k);
-      m_commit(bar);
-    }
-    // the next tile's inputs travel while this one computes
-    const int tn = t + gridDim.x;
-    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
-    if (tn < tiles) {
-      x0 = get_x(tn, tid);
-      x1 = get_x(tn, tid + kMThreads);
-    }
-    wait_mma();
-    if (dead) break;
-    put_x(tid, x0);
-    put_x(tid + kMThreads, x1);
-    const int64_t m = (int64_t)t * kMRows + row;
-    const bool in = m < A.M;
-    m_epilogue(mine, bias + 128 * half, in && A.H[0] ? A.H[0] + m * kMH1 + 128 * half : nullptr);
-    m_before();
-    __syncthreads();
-    if (tid == 0) {
-      m_after();
-      for (int k = 0; k < kMH1 / 16; ++k)  // A: columns 8 k of each half's 64
-        m_mma_ts(tm + 256, tm + 8 * k + (k >= 8 ? 64 : 0), m_desc(sb + kMW2 + 256 * k, m_sbo(kMH1)),
-                 m_idesc(kMH2), k);
-      m_commit(bar);
-    }
-    wait_mma();
-    if (dead) break;
-    m_epilogue(mine + 256, bias + 256 + 128 * half,
-               in && A.H[1] ? A.H[1] + m * kMH2 + 128 * half : nullptr);
-    m_before();
-    __syncthreads();
-    if (tid == 0) {
-      m_after();
-      for (int k = 0; k < kMH2 / 16; ++k)
-        m_mma_ts(tm, tm + 256 + 8 * k + (k >= 8 ? 64 : 0),
-                 m_desc(sb + kMW3 + 256 * k, m_sbo(kMH2)), m_idesc(kMH3), k);
-      m_commit(bar);
-    }
-    wait_mma();
-    if (dead) break;
-    if (half == 0) {
-      // the third layer's epilogue and the head: s[l] sums columns l, l + 32,
-      // l + 64, l + 96, then the butterfly's tree over l
-      float s[32];
-#pragma unroll
-      for (int l = 0; l < 32; ++l) s[l] = 0.f;
-      uint16_t *h = in && A.H[2] ? A.H[2] + m * kMH3 : nullptr;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32], p[16];
-        m_ld32(r, mine + 32 * c);
-        const float *b3 = bias + 512 + 32 * c, *w4 = bias + 640 + 32 * c;
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const float2 bb = *reinterpret_cast<const float2 *>(b3 + 2 * q);
-          const float2 ww = *reinterpret_cast<const float2 *>(w4 + 2 * q);
-          p[q] = m_relu2(__uint_as_float(r[2 * q]) + bb.x, __uint_as_float(r[2 * q + 1]) + bb.y);
-          s[2 * q] = fmaf(__uint_as_float(p[q] << 16), ww.x, s[2 * q]);
-          s[2 * q + 1] = fmaf(__uint_as_float(p[q] & 0xFFFF0000u), ww.y, s[2 * q + 1]);
-        }
-        if (h) {
-          uint4 *o = reinterpret_cast<uint4 *>(h + 32 * c);
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            o[q] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
-        }
+  uint32_t i = 0;  // tiles done: the barriers' phases, the regions' places
+  if (quarter < 4) {
+    if (tid == 0 && (int)blockIdx.x < tiles) layer1(tm);
+    // the next tile's inputs travel for a whole tile, unconverted
+    MlpX x = get_x(blockIdx.x + gridDim.x);
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
+      const uint32_t P = tm + 256 * (i & 1), Q = tm + 256 * (~i & 1);
+      const uint32_t mine = lane_base + 32 * quarter;
+      const float *b1 = bias + 32 * quarter, *b2 = b1 + 256;
+      const int tn = t + gridDim.x;
+      const int64_t m = (int64_t)t * kMRows + row;
+      const bool in = m < A.M;
+      uint16_t *h1 = in && A.H[0] ? A.H[0] + m * kMH1 + 32 * quarter : nullptr;
+      uint16_t *h2 = in && A.H[1] ? A.H[1] + m * kMH2 + 32 * quarter : nullptr;
+      wait(bar1, i & 1);
+      put_x(x);
+      x = get_x(tn + gridDim.x);
+      m_epilogue(P + mine, b1, h1);
+      m_before();
+      if (m_main_sync(*dead)) break;
+      if (tid == 0) {
+        if (i) wait(bar_head, ~i & 1);  // the last tile's sums are in Q
+        m_after();
+        half(Q, P, kMW2, 0, kMH2);
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int l = 0; l < o; ++l) s[l] += s[l + o];
-      if (in) A.y[m] = s[0] + A.b4[0];
+      m_epilogue(P + mine + 128, b1 + 128, h1 ? h1 + 128 : nullptr);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next inputs
+      m_before();
+      if (m_main_sync(*dead)) break;
+      if (tid == 0) {
+        m_after();
+        half(Q, P, kMW2, 1, kMH2);
+        m_commit(bar2);
+      }
+      wait(bar2, i & 1);
+      m_epilogue(Q + mine, b2, h2);
+      m_before();
+      if (m_main_sync(*dead)) break;
+      if (tid == 0) {
+        m_after();
+        half(P, Q, kMW3, 0, kMH3);
+      }
+      m_epilogue(Q + mine + 128, b2 + 128, h2 ? h2 + 128 : nullptr);
+      m_before();
+      if (m_main_sync(*dead)) break;
+      if (tid == 0) {
+        m_after();
+        half(P, Q, kMW3, 1, kMH3);
+        m_commit(bar3);
+        wait(bar3, i & 1);
+        if (tn < tiles) layer1(Q);
+      }
+    }
+  } else {
+    for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++i) {
+      const uint32_t P = tm + 256 * (i & 1);
+      const int64_t m = (int64_t)t * kMRows + row;
+      const bool in = m < A.M;
+      wait(bar3, i & 1);
+      const float s = m_head(P + lane_base, bias + 512, bias + 640,
+                             in && A.H[2] ? A.H[2] + m * kMH3 : nullptr);
+      m_before();
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_head) : "memory");
+      if (in) A.y[m] = s + A.b4[0];
     }
   }
-  if (dead)  // a product never completed: no prediction may pass for one
-    for (; t < tiles; t += gridDim.x) {
-      const int64_t m = (int64_t)t * kMRows + row;
-      if (half == 0 && m < A.M) A.y[m] = __int_as_float(0x7FFFFFFF);
-    }
   m_before();
   __syncthreads();
+  if (*dead)  // a product never completed: no prediction may pass for one
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x)
+      if (quarter == 4 && t * kMRows + row < A.M) A.y[t * kMRows + row] = __int_as_float(0x7FFFFFFF);
   if (warp == 0) {
     m_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm) : "memory");
