@@ -13,7 +13,8 @@
 //     them.  An even step updates E from O, an odd one O from E: a cell's
 //     align predecessor is its own diagonal's last value, insert the diagonal
 //     below, delete the one above; only the lane's edge needs a shuffle and a
-//     byte permute, so a step is one short dependency chain whatever D is.
+//     byte permute, so a step is one short dependency chain whatever D is (up to
+//     D = 16 one exchange serves two steps, see team_step).
 //   * the helpers look up the costs of the next 8 double steps, one (lane,
 //     double step) each, and lay them out in shared memory as the main warp
 //     reads them: the align costs of every register, and the one new insert
@@ -25,8 +26,10 @@
 // condition are k_lin_dp4's, see linear4.cu; the band and results the
 // reference's (algn.c:375-968, 3551-3666).
 //
-// Bound: the latency of a step (shuffle, permute, add-min, clear), L1 + L2 of
-// them.
+// Bound: the latency of a double step (shuffle, then permute, add-min and clear
+// twice: 55 cycles, 82 measured with 8 diagonals a lane and 107 with 16), L1 + L2
+// halves of them.  An exchange and late costs at each step took 93 and 126: one
+// alignment of 1,500 bp 174 us, now 146.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
@@ -120,6 +123,7 @@ struct TeamState {
   uint32_t E[NQ], O[NQ], gi[NQ], gd[NQ];
   uint32_t kE[NQ], iE[NQ], kO[NQ], iO[NQ];  // masks: bits kept, infinity forced
   uint32_t aE[NQ], aO[NQ];                  // the moves of 8 steps
+  uint32_t hE, kH, iH;  // high half: the next lane's first cell, its masks
 };
 
 // Appends a register's moves (the two low bits of x's halves; y is x with them
@@ -132,32 +136,65 @@ __device__ __forceinline__ uint32_t team_move(uint32_t acc, uint32_t x, uint32_t
   return t_mad(y, (uint32_t)K.m1, t_mad(acc, (uint32_t)K.four, x));
 }
 
-// One double step.  cap: the final cell is in this one (0 even, 1 odd step):
-// its registers go to `end`.
-template <int MODE, int D>
-__device__ __forceinline__ void team_step(TeamState<MODE, D> &S, const uint4 *cv, uint2 g, int lane,
-                                          const DpK &K, int cap, uint32_t *end) {
-  constexpr int NQ = D / 4;
-  uint32_t W[2 * NQ];
+// A lane's costs of one double step, as the helpers left them.
+template <int D>
+struct TeamCost {
+  uint32_t W[D / 2], hW;
+  uint2 g;
+};
+template <int D>
+__device__ __forceinline__ void team_load(TeamCost<D> &C, const uint8_t *step, int lane) {
+  const uint4 *cv = reinterpret_cast<const uint4 *>(step) + lane;
 #pragma unroll
   for (int v = 0; v < D / 8; ++v) {
     const uint4 x = cv[32 * v];
-    W[4 * v] = x.x, W[4 * v + 1] = x.y, W[4 * v + 2] = x.z, W[4 * v + 3] = x.w;
+    C.W[4 * v] = x.x, C.W[4 * v + 1] = x.y, C.W[4 * v + 2] = x.z, C.W[4 * v + 3] = x.w;
   }
+  C.hW = reinterpret_cast<const uint32_t *>(cv)[4];  // the next lane's; lane 31: any (masked)
+  C.g = reinterpret_cast<const uint2 *>(step + D / 8 * 512)[lane];
+}
+
+// One double step.  A lane also computes the next lane's first even cell, which
+// its last odd one reads, so that all it needs of others is their odd cells of
+// the double step before: one shuffle latency for two steps (not with 32
+// diagonals a lane, which fill the two by themselves: the costs of a pair of
+// 4,000 bp take 347 us, 384 with the extra cell).  cap: the final cell is in this
+// one (0 even, 1 odd step): its registers go to `end`.
+template <int MODE, int D>
+__device__ __forceinline__ void team_step(TeamState<MODE, D> &S, const TeamCost<D> &C, int lane,
+                                          const DpK &K, int cap, uint32_t *end) {
+  constexpr int NQ = D / 4;
+  const uint32_t(&W)[2 * NQ] = C.W;
+  const uint2 g = C.g;
+  const uint32_t hW = C.hW;
+  const uint32_t below = __shfl_sync(kTFull, S.O[NQ - 1], lane + 31);  // lane - 1, in a ring
+  constexpr bool kHalo = D < 32;
+  const uint32_t above = kHalo ? __shfl_sync(kTFull, S.O[0], lane + 1) : 0u;
   const uint32_t one = (uint32_t)K.one;
+  const uint32_t hd = S.gd[NQ - 1];
 #pragma unroll
   for (int q = NQ - 1; q > 0; --q) S.gd[q] = S.gd[q - 1];
   S.gd[0] = g.y;
+  uint32_t rw;
   {
-    const uint32_t recv = __shfl_sync(kTFull, S.O[NQ - 1], lane + 31);  // lane - 1, in a ring
-    const uint32_t lw = t_prmt(recv, S.O[NQ - 1], 0x5432);
+    // the next lane's first cell, in the high half (the low one holds anything)
+    uint32_t h = t_mad(hW, (uint32_t)K.k64, S.hE);
+    h = __viaddmin_u16x2(S.O[NQ - 1], g.x, h);
+    h = __viaddmin_u16x2(t_mad(above, (uint32_t)K.k64, 0), hd, h);
+    h = (h & S.kH) | S.iH;
+    const uint32_t lw = t_prmt(below, S.O[NQ - 1], 0x5432);
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      uint32_t x = __viaddmin_u16x2(S.E[q], W[q], t_mad(S.O[q], one, S.gd[q]));
+    for (int e = 0; e < NQ; ++e) {
+      const int q = kHalo ? NQ - 1 - e : e;  // what waits for a shuffle last, or goes into one first
+      uint32_t x = kHalo ? __viaddmin_u16x2(S.O[q], S.gd[q], t_mad(S.E[q], one, W[q]))
+                         : __viaddmin_u16x2(S.E[q], W[q], t_mad(S.O[q], one, S.gd[q]));
       x = __viaddmin_u16x2(q ? S.O[q - 1] : lw, S.gi[q], x);
       S.E[q] = (x & S.kE[q]) | S.iE[q];
       if (MODE == kDpChoice) S.aE[q] = team_move(S.aE[q], x, S.E[q], q, K);
     }
+    const uint32_t next = __shfl_sync(kTFull, S.E[0], lane + 1);
+    if (kHalo) S.hE = t_mad(next, (uint32_t)K.k64, 0);
+    rw = kHalo ? t_prmt(S.E[0], h, 0x7632) : t_prmt(S.E[0], next, 0x5432);
   }
   if (cap == 0) {
 #pragma unroll
@@ -166,16 +203,13 @@ __device__ __forceinline__ void team_step(TeamState<MODE, D> &S, const uint4 *cv
 #pragma unroll
   for (int q = 0; q + 1 < NQ; ++q) S.gi[q] = S.gi[q + 1];
   S.gi[NQ - 1] = g.x;
-  {
-    const uint32_t recv = __shfl_sync(kTFull, S.E[0], lane + 1);
-    const uint32_t rw = t_prmt(S.E[0], recv, 0x5432);
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      uint32_t x = __viaddmin_u16x2(S.O[q], W[NQ + q], t_mad(S.E[q], one, S.gi[q]));
-      x = __viaddmin_u16x2(q + 1 < NQ ? S.E[q + 1] : rw, S.gd[q], x);
-      S.O[q] = (x & S.kO[q]) | S.iO[q];
-      if (MODE == kDpChoice) S.aO[q] = team_move(S.aO[q], x, S.O[q], q, K);
-    }
+  for (int q = 0; q < NQ; ++q) {
+    uint32_t x = kHalo ? __viaddmin_u16x2(S.E[q], S.gi[q], t_mad(S.O[q], one, W[NQ + q]))
+                       : __viaddmin_u16x2(S.O[q], W[NQ + q], t_mad(S.E[q], one, S.gi[q]));
+    x = __viaddmin_u16x2(q + 1 < NQ ? S.E[q + 1] : rw, S.gd[q], x);
+    S.O[q] = (x & S.kO[q]) | S.iO[q];
+    if (MODE == kDpChoice) S.aO[q] = team_move(S.aO[q], x, S.O[q], q, K);
   }
   if (cap == 1) {
 #pragma unroll
@@ -421,6 +455,11 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
       }
       S.aE[q] = S.aO[q] = 0;
     }
+    const int ih = D * lane + D;
+    const bool eh = ih >= g.lo && ih < g.hi;
+    S.kH = eh ? keep << 16 : 0u;
+    S.iH = eh ? 0u : 0xC0000000u;
+    S.hE = __shfl_sync(kTFull, S.E[0], lane + 1) << 16;
   } else if (warp % 4) {
     produce(0);
   }
@@ -431,17 +470,22 @@ __global__ void __launch_bounds__(kTThreads) k_lin_team(const __grid_constant__ 
     } else if (warp == 0) {
       const uint8_t *slot = team_sm + (c & 1) * Dm::kSlot;
       if (c + 1 < nch) {
+        constexpr int kAhead = D < 32 ? 1 : 0;  // double steps a cost is read ahead
+        TeamCost<D> C[2];
+        if (kAhead) team_load<D>(C[0], slot, lane);
 #pragma unroll
-        for (int v = 0; v < kTChunk; ++v)
-          team_step<MODE, D>(S, reinterpret_cast<const uint4 *>(slot + v * Dm::kStep) + lane,
-                             reinterpret_cast<const uint2 *>(slot + v * Dm::kStep + NV * 512)[lane],
-                             lane, A.k, -1, end);
+        for (int v = 0; v < kTChunk; ++v) {
+          const int x = v + kAhead;
+          if (x < kTChunk) team_load<D>(C[x & 1], slot + x * Dm::kStep, lane);
+          team_step<MODE, D>(S, C[v & 1], lane, A.k, -1, end);
+        }
       } else {
 #pragma unroll 1
-        for (int v = 0; v < kTChunk; ++v)
-          team_step<MODE, D>(S, reinterpret_cast<const uint4 *>(slot + v * Dm::kStep) + lane,
-                             reinterpret_cast<const uint2 *>(slot + v * Dm::kStep + NV * 512)[lane],
-                             lane, A.k, v == g.me % kTChunk ? (fcell & 1) : -1, end);
+        for (int v = 0; v < kTChunk; ++v) {
+          TeamCost<D> C;
+          team_load<D>(C, slot + v * Dm::kStep, lane);
+          team_step<MODE, D>(S, C, lane, A.k, v == g.me % kTChunk ? (fcell & 1) : -1, end);
+        }
       }
       if (MODE == kDpChoice) {
         uint32_t w[2 * NQ];
