@@ -996,10 +996,14 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   // others run in rows.
   std::vector<int64_t> key((size_t)n);
   for (int32_t t = 0; t < n; ++t) key[t] = (int64_t)hwd[(size_t)n + t] << 7;  // longest_first's unit
+  int dev = 0, sms = 1;
+  CKA(cudaGetDevice(&dev));
+  CKA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool spread = want_align && n <= kDiagSpreadPerSm * sms;
   std::vector<int32_t> order, rows_of, slots[kDiagClassN];
   longest_first(key, order);
   for (int32_t id : order) {
-    const int c = (hwd[id] & kAffFits) ? aff_diag_class((hwd[id] & ~kAffFits) - 41) : kDiagClassN;
+    const int c = (hwd[id] & kAffFits) ? aff_diag_class((hwd[id] & ~kAffFits) - 41, spread) : kDiagClassN;
     if (c == kDiagClassN) rows_of.push_back(id);
     else slots[c].push_back(id);
   }
@@ -1070,7 +1074,7 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   if (diag) {
     GA.tasks = (int)task_word.size(); GA.task = dtask; GA.counter = counter;
     ProfScope ps(name, st);
-    if ((rc = launch_aff_diag(GA, want_align, (herr & 16) != 0, st))) return rc;
+    if ((rc = launch_aff_diag(GA, want_align, (herr & 16) != 0, spread, st))) return rc;
   }
   if (diag && want_align) {
     AffWalkArgs WA;

@@ -7,7 +7,7 @@
 // boundary test per cell (82 instructions a cell); here the band lives in
 // registers:
 //   * eight lanes take a pair, four pairs a warp (16 or 32 lanes where the band is
-//     wider than 128 or 256).  Lane k owns the D diagonals
+//     wider than 128 or 256, 16 in small batches with directions).  Lane k owns the D diagonals
 //     idx = D k .. D k + D - 1 of the band (idx = d + 40, d = j - i), each
 //     register two cells of one parity: E[q] idx 2q in the low half and 2q + D/2
 //     in the high half, O[q] the odd ones above.  Step t updates the cells i + j
@@ -474,7 +474,9 @@ __device__ __forceinline__ void diag_task(const AffDiagArgs &A, const DiagSmem &
   if (has && k == 0) A.cost[id] = (int)(res >> (16 * (fc / NQ)) & 0xFFFFu) / sc;
 }
 
-template <bool BT, bool GAPS>
+// SPREAD: the classes of a small batch with directions (a kernel of its own: the
+// code for 8 diagonals a lane costs the others 2 %).
+template <bool BT, bool GAPS, bool SPREAD>
 __global__ void __launch_bounds__(kDWarps * 32, GAPS ? 3 : 4) k_aff_diag(const __grid_constant__ AffDiagArgs A) {
   extern __shared__ __align__(16) uint8_t diag_sm[];
   DiagSmem &sm = *reinterpret_cast<DiagSmem *>(diag_sm);
@@ -498,7 +500,8 @@ __global__ void __launch_bounds__(kDWarps * 32, GAPS ? 3 : 4) k_aff_diag(const _
     const int64_t word = A.task[t];
     const int64_t off = word & 0xFFFFFFFFFFFFll;
     const int lanes = (int)(word >> 56), width = (int)(word >> 48) & 0xFF;
-    if (width == 12) diag_task<BT, GAPS, 12>(A, sm, rings, t, off, lanes, lane);
+    if (SPREAD && width == 8) diag_task<BT, GAPS, 8>(A, sm, rings, t, off, lanes, lane);
+    else if (width == 12) diag_task<BT, GAPS, 12>(A, sm, rings, t, off, lanes, lane);
     else diag_task<BT, GAPS, 16>(A, sm, rings, t, off, lanes, lane);
   }
 }
@@ -536,7 +539,8 @@ __global__ void __launch_bounds__(128) k_aff_walk(const __grid_constant__ AffWal
   }
   uint8_t *ri = P.swap ? ob : oa, *rj = P.swap ? oa : ob;
   const AffWhere W = A.where[id];
-  const int D = W.width, NQ = D / 4, dsh = D == 12 ? 0 : 4;
+  const int D = W.width, NQ = D / 4;
+  const unsigned inv = 0xFFFFFFFFu / (unsigned)D + 1;  // idx / D
   const uint32_t *dm = A.dm + W.off + 2 * W.lane0;
   int i = P.leni, j = P.lenj, nr = 0, nm = 0, mode = 0, last_m = -1;
   bool bad = false;
@@ -562,7 +566,7 @@ __global__ void __launch_bounds__(128) k_aff_walk(const __grid_constant__ AffWal
       bad = true;
       break;
     }
-    const int k = dsh ? idx >> dsh : idx / 12, c = (idx - k * D) >> 1;
+    const int k = (int)__umulhi((unsigned)idx, inv), c = (idx - k * D) >> 1;
     const int qq = c < NQ ? c : c - NQ, half = c < NQ ? 0 : 16;
     const int w = ((idx & 1) ? NQ : 0) + qq;
     // lane l: cell (i - l, j - l)
@@ -625,7 +629,7 @@ __global__ void __launch_bounds__(128) k_aff_walk(const __grid_constant__ AffWal
   }
 }
 
-template <bool BT, bool GAPS>
+template <bool BT, bool GAPS, bool SPREAD = false>
 void diag_launch(const AffDiagArgs &A, cudaStream_t st) {
   static std::atomic<int> cache[64];  // resident blocks of the device
   constexpr uint32_t sm = diag_smem<GAPS>();
@@ -634,18 +638,20 @@ void diag_launch(const AffDiagArgs &A, cudaStream_t st) {
   int c = cache[dev & 63].load();
   if (!c) {
     int per = 0, sms = 0;
-    cudaFuncSetAttribute(k_aff_diag<BT, GAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aff_diag<BT, GAPS>, kDWarps * 32, sm);
+    cudaFuncSetAttribute(k_aff_diag<BT, GAPS, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aff_diag<BT, GAPS, SPREAD>, kDWarps * 32, sm);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cache[dev & 63].store(c = std::max(per, 1) * std::max(sms, 1));
   }
-  k_aff_diag<BT, GAPS><<<std::min((A.tasks + kDWarps - 1) / kDWarps, c), kDWarps * 32, sm, st>>>(A);
+  k_aff_diag<BT, GAPS, SPREAD><<<std::min((A.tasks + kDWarps - 1) / kDWarps, c), kDWarps * 32, sm, st>>>(A);
 }
 
 }  // namespace
 
-int launch_aff_diag(const AffDiagArgs &A, bool bt, bool gaps, cudaStream_t st) {
-  if (bt && gaps) diag_launch<true, true>(A, st);
+int launch_aff_diag(const AffDiagArgs &A, bool bt, bool gaps, bool spread, cudaStream_t st) {
+  if (spread && gaps) diag_launch<true, true, true>(A, st);
+  else if (spread) diag_launch<true, false, true>(A, st);
+  else if (bt && gaps) diag_launch<true, true>(A, st);
   else if (bt) diag_launch<true, false>(A, st);
   else if (gaps) diag_launch<false, true>(A, st);
   else diag_launch<false, false>(A, st);

@@ -53,26 +53,39 @@ struct AffWalkArgs {
 };
 
 // A task is a warp's pairs: 32 / lanes of them, `lanes` lanes each with `width`
-// diagonals (8 x 12 diagonals up to 32 x 16).
+// diagonals (8 x 12 diagonals up to 32 x 16; 8 a lane in small batches with
+// directions alone).
 constexpr int kDiagTask = 4;
 struct AffDiagClass {
   int lanes, width;
 };
-constexpr AffDiagClass kDiagClasses[] = {{8, 12}, {8, 16}, {16, 12}, {16, 16}, {32, 12}, {32, 16}};
-constexpr int kDiagClassN = 6;
-// Smallest class for a band of e0 (kDiagClassN: wider than all).
-inline int aff_diag_class(int e0) {
-  int c = 0;
-  while (c < kDiagClassN && kDiagClasses[c].lanes * kDiagClasses[c].width < e0 + 41) ++c;
-  return c;
+constexpr AffDiagClass kDiagClasses[] = {{8, 12},  {8, 16},  {16, 8}, {16, 12},
+                                         {16, 16}, {32, 12}, {32, 16}};
+constexpr int kDiagClassN = 7;
+// Smallest class for a band of e0 (kDiagClassN: wider than all).  `spread`: of 16
+// lanes at least (the fewer diagonals a lane, the shorter a pair's own time).
+inline int aff_diag_class(int e0, bool spread) {
+  int best = kDiagClassN, slots = 1 << 30;
+  for (int c = 0; c < kDiagClassN; ++c) {
+    const int s = kDiagClasses[c].lanes * kDiagClasses[c].width;
+    if (spread ? kDiagClasses[c].lanes < 16 : kDiagClasses[c].width < 12) continue;
+    if (s >= e0 + 41 && s < slots) best = c, slots = s;
+  }
+  return best;
 }
+// Batches with directions are spread up to eight pairs an SM: 200 pairs of
+// 100-5,000 bp take 0.81 ms instead of 1.53, 1,300 of 1,000 bp 0.26 instead of 0.34;
+// 2,600 of 1,000 bp would take 0.36 instead of 0.32.  Costs alone gain nothing
+// (200 pairs of 1,000 bp: 0.21 ms both ways).
+constexpr int kDiagSpreadPerSm = 8;
 // Task word: direction words' offset, lanes and width; the words of a task
 // whose longest pair has leni + lenj = steps.
 inline int64_t aff_diag_task(int64_t off, AffDiagClass c) {
   return off | (int64_t)c.lanes << 56 | (int64_t)c.width << 48;
 }
 inline int64_t aff_diag_words(int width, int64_t steps) { return (steps / 4 + 1) * 16 * width; }
-int launch_aff_diag(const AffDiagArgs &A, bool bt, bool gaps, cudaStream_t st);
+// spread: with directions, of classes chosen as such
+int launch_aff_diag(const AffDiagArgs &A, bool bt, bool gaps, bool spread, cudaStream_t st);
 int launch_aff_walk(const AffWalkArgs &A, cudaStream_t st);
 
 }  // namespace poyd
