@@ -259,7 +259,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   CK3(cudaStreamSynchronize(st));
   const int32_t *hl[4];
   for (int q = 0; q < 4; ++q) hl[q] = all_len.data() + (size_t)n * std::min(q, nq - 1);
-  int64_t ring_max = 0, dir_max = 0, lin_plane = 0, lin_dir = 0;
+  int64_t ring_max = 0, dir_max = 0, lin_plane = 0, lin_dir = 0, lin_steps = 0;
   int64_t open_plane = 0, open_dir = 0;
   int smax = 16, max_b = 1;
   std::vector<int64_t> work(n);
@@ -277,6 +277,7 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     smax = std::max<int>(smax, (int)std::max(la, std::max(lb, lc)));
     work[i] = la * lb * lc;
     const P3LinearPlan lp = p3_linear_plan(la, lb, lc);
+    lin_steps += p3_linear_steps(la, lb, lc);
     lin_plane = std::max(lin_plane, lp.plane);
     lin_dir = std::max(lin_dir, lp.dir);
     const P3OpenPlan op = p3_open_plan(la, lb, lc);
@@ -371,14 +372,26 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
   const bool packed = !(pk && pk[0] == '0') && 48LL * go + 15 < 0x4000 &&
                 16LL * (2LL * mm + 3LL * ge) < 0x4000;
   if (packed && go == 0) {
-    // Warps per triple: consecutive strips run kP3LinLag steps apart, so a
-    // triple feeds about (steps of a strip) / kP3LinLag warps.  A batch that
-    // fills the SMs takes at most 4 (more blocks per SM share the issue
-    // slots alike, and its shorter triples waste fewer warps); a small one
-    // takes what its longest triple can use.
+    // Warps per triple: twice as many while the largest triple's own steps get
+    // fewer by three tenths (its strips follow one another kP3LinLag steps apart,
+    // so that a strip feeds steps / kP3LinLag warps; 20 triples of 150-200 bp, a
+    // fifth fewer steps, take 1.15 ms with 4 warps and 1.37 with more) and its own
+    // time, at four warps a scheduler, is more than three quarters of what the
+    // whole batch's instructions take.
+    // Up to two triples an SM, then twice as many where that costs no step: a
+    // block an SM, whose waiting warps leave the others the issue slots.
+    // Measured with 2, 4, 8 and 16 warps: 1,216 triples of 100-300 bp 17.6, 10.1,
+    // 8.9 and 11.4 ms, of 200 bp 6.6, 6.1, 9.0 and 10.7; 304 of 100-300 bp 6.5,
+    // 5.4, 5.3 and 3.1.
+    const int big = order[0];
+    const int64_t bl[3] = {hl[0][big], hl[1][big], hl[2][big]};
+    auto chain = [&](int w) { return p3_linear_chain(bl[0], bl[1], bl[2], w); };
+    const double batch = 280.0 * (double)lin_steps / (4.0 * sms);
     int warps = 1;
-    const int most = (int64_t)n * 4 >= 8LL * sms ? 4 : 16;
-    while (2 * warps <= most && 2 * warps * kP3LinLag <= longest + 40) warps *= 2;
+    while (warps < 16 && 10 * chain(2 * warps) <= 7 * chain(warps) &&
+           1100.0 * (double)chain(warps) > 0.75 * batch)
+      warps *= 2;
+    if (n <= 2 * sms && warps == 8 && chain(16) <= chain(8)) warps = 16;
     const int blocks = (int)fit(std::min<int64_t>(n, p3_linear_blocks(warps, longest)), lin_plane, lin_dir);
     uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(lin_plane * blocks));
     uint8_t *dirb = (uint8_t *)ws_buffer(w, WS_P3_DIR, (size_t)(lin_dir * blocks));

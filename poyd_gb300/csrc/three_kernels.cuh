@@ -292,6 +292,9 @@ struct P3LinearPlan {
 };
 P3LinearPlan p3_linear_plan(int64_t la, int64_t lb, int64_t lc);
 int p3_linear_blocks(int warps, int longest);  // resident blocks of the device
+// Warp steps of a triple in all, and of the longest of its `warps` warps.
+int64_t p3_linear_steps(int64_t la, int64_t lb, int64_t lc);
+int64_t p3_linear_chain(int64_t la, int64_t lb, int64_t lc, int warps);
 int launch_p3_linear(const P3Args &A, int warps, int longest, int blocks, uint8_t *plane,
                      int64_t plane_stride, uint8_t *dir, int64_t dir_stride, cudaStream_t st);
 constexpr int kP3LinLag = 48;  // steps between consecutive strips

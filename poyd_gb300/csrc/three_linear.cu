@@ -15,7 +15,8 @@
 // Bound: integer issue (7 add-mins, the mismatch terms and the choice bits
 // per two cells: about 8 instructions a cell); the choices are 0.5 bytes a
 // cell, the strip boundaries about 1.  Measured: 1,216 triples of 100-300 bp
-// in 10.8 ms where k_p3 with all 16 x 16 state pairs took 339 ms.
+// in 9.0 ms (10.1 with at most four warps a triple) where k_p3 with all 16 x 16
+// state pairs took 339 ms.
 //
 // Layout.  The axes are the sequences by length: A the shortest, C the
 // longest.  A thread owns a 4 x 4 tile of (A, B) and marches along C; its
@@ -382,6 +383,17 @@ P3LinearPlan p3_linear_plan(int64_t la, int64_t lb, int64_t lc) {
   const int64_t TB = std::max<int64_t>((l[1] + 3) / 4, kMinTB), F = (l[0] + 3) / 4 * TB;
   const int64_t U = (F + 31) / 32, R = (TB + 31) / 32 + 2, NS = (l[2] + 32 + 7) & ~(int64_t)7;
   return {R * NS * (256 + 16), U * NS * 256};
+}
+
+int64_t p3_linear_steps(int64_t la, int64_t lb, int64_t lc) {
+  const P3LinearPlan p = p3_linear_plan(la, lb, lc);
+  return p.dir / 256;
+}
+
+int64_t p3_linear_chain(int64_t la, int64_t lb, int64_t lc, int warps) {
+  const P3LinearPlan p = p3_linear_plan(la, lb, lc);
+  const int64_t NS = (std::max({la, lb, lc}) + 32 + 7) & ~(int64_t)7, U = p.dir / 256 / NS;
+  return (U - 1) / warps * std::max<int64_t>(NS, kP3LinLag * warps) + (U - 1) % warps * kP3LinLag + NS;
 }
 
 int p3_linear_blocks(int warps, int longest) {
