@@ -92,13 +92,67 @@ __device__ __forceinline__ void t_chain(const __nv_bfloat16 *in, const __nv_bflo
       }
 }
 
+// The output bias's gradient and the loss, summed row after row as
+// poyd_mlp_head_backward sums them: the residuals cancel, so that another order's
+// rounding would show in the sixth digit of the one number.  Two threads add what
+// the others have staged, 1,024 rows a turn, by a block of its own beside the chain
+// (4,096 rows: 9 of the launch's 22 us).
+__device__ __forceinline__ void t_head_sums(const MlpBwdArgs &A, float *buf) {
+  constexpr int kTurn = 1024;
+  const int tid = threadIdx.x;
+  auto stage = [&](int m0, int first, int step) {
+    float *d = buf + (m0 / kTurn & 1) * 2 * kTurn, *e = d + kTurn;
+    for (int x = first; x < kTurn; x += step) {
+      const int m = m0 + x;
+      const float r = m < A.M ? A.y[m] - A.target[m] : 0.f;
+      e[x] = r;
+      d[x] = 2.f * r / (float)A.M;
+    }
+  };
+  stage(0, tid, kTThreads);
+  __syncthreads();
+  float s = 0.f;
+  for (int m0 = 0; m0 < A.M; m0 += kTurn) {
+    const float4 *v = reinterpret_cast<const float4 *>(buf + ((m0 / kTurn & 1) * 2 + tid / 32) * kTurn);
+    if (tid >= 64) {
+      if (m0 + kTurn < A.M) stage(m0 + kTurn, tid - 64, kTThreads - 64);
+    } else if (tid == 0) {
+#pragma unroll 8
+      for (int x = 0; x < kTurn / 4; ++x) {
+        const float4 f = v[x];
+        s += f.x;
+        s += f.y;
+        s += f.z;
+        s += f.w;
+      }
+    } else if (tid == 32) {
+#pragma unroll 8
+      for (int x = 0; x < kTurn / 4; ++x) {
+        const float4 f = v[x];
+        s = fmaf(f.x, f.x, s);
+        s = fmaf(f.y, f.y, s);
+        s = fmaf(f.z, f.z, s);
+        s = fmaf(f.w, f.w, s);
+      }
+    }
+    __syncthreads();
+  }
+  if (tid == 0) A.gb[3][0] = s;
+  if (tid == 32) A.loss[0] = s / (float)A.M;
+}
+
 // dZ3 = dy w4 masked, dZ2 = dZ3 W3^T masked, dZ1 = dZ2 W2^T masked, for 32
-// rows a block.
+// rows a block; the first block takes t_head_sums.
 __global__ void __launch_bounds__(kTThreads) k_mlp_chain(const __grid_constant__ MlpBwdArgs A) {
   __shared__ __align__(16) __nv_bfloat16 z3[kTRows * (kTH3 + kTPad)];
   __shared__ __align__(16) __nv_bfloat16 z2[kTRows * (kTH2 + kTPad)];
+  static_assert(sizeof(z2) >= 4 * 1024 * sizeof(float), "t_head_sums stages over z2");
+  if (blockIdx.x == 0) {
+    t_head_sums(A, reinterpret_cast<float *>(z2));
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int m0 = blockIdx.x * kTRows;
+  const int m0 = (blockIdx.x - 1) * kTRows;
   __shared__ float dy[kTRows];
   if (threadIdx.x < kTRows) {
     const int m = m0 + threadIdx.x;
@@ -140,8 +194,8 @@ __global__ void __launch_bounds__(kTThreads) k_mlp_chain(const __grid_constant__
 // the rows; the partial tiles meet in distributed shared memory and are
 // summed in rank order (the same sum every time).  Tiles 0-1: layer 1 (its 32
 // rows fill half a tile), 2-9: layer 2, 10-13: layer 3; the tile with input
-// row 0 also sums dZ's columns (the bias gradient).  Tile 14: the head's dw,
-// db and the loss.  Measured at 4,096 rows against one reduction over the
+// row 0 also sums dZ's columns (the bias gradient).  Tile 14: the head's dw.
+// Measured at 4,096 rows against one reduction over the
 // whole batch per tile: 8-64 blocks were busy for most of 1.5 ms.
 constexpr int kGSplit = 8, kGTiles = 15;
 constexpr int kGM = 64, kGN = 128, kGK = 32;  // tile and staged rows
@@ -165,19 +219,13 @@ __global__ void __cluster_dims__(kGSplit, 1, 1) __launch_bounds__(kTThreads)
   const int r0 = min(A.M, rank * chunk), r1 = min(A.M, r0 + chunk);
   int rows = kGM;  // gradient rows of the tile
   if (tile == kGTiles - 1) {
-    // [0, 128): dw; [128] db, [129] loss.  256 rows a pass: their dy into
-    // shared memory, then eight columns a thread over every 16th row.
+    // [0, 128): dw.  256 rows a pass: their dy into shared memory, then eight
+    // columns a thread over every 16th row.
     float *dyv = part + 16 * 128;
     const int c8 = (tid & 15) * 8, rg = tid >> 4;
-    float sw[8] = {}, sd = 0.f, se = 0.f;
+    float sw[8] = {};
     for (int m = r0; m < r1; m += kTThreads) {
-      float d = 0.f;
-      if (m + tid < r1) {
-        const float e = A.y[m + tid] - A.target[m + tid];
-        d = 2.f * e / (float)A.M;
-        sd += d;
-        se += e * e;
-      }
+      const float d = m + tid < r1 ? t_dy(A, m + tid) : 0.f;
       __syncthreads();
       dyv[tid] = d;
       __syncthreads();
@@ -194,19 +242,12 @@ __global__ void __cluster_dims__(kGSplit, 1, 1) __launch_bounds__(kTThreads)
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) part[rg * 128 + c8 + j] = sw[j];
-    for (int o = 16; o > 0; o >>= 1) {
-      sd += __shfl_xor_sync(0xffffffffu, sd, o);
-      se += __shfl_xor_sync(0xffffffffu, se, o);
-    }
-    __syncthreads();  // dyv's readers are done
-    if (lane == 0) dyv[warp] = sd, dyv[8 + warp] = se;
+    __syncthreads();
     float t = 0.f;
     if (tid < 128)
       for (int g = 0; g < 16; ++g) t += part[g * 128 + tid];
     __syncthreads();
-    if (tid >= 128 && tid < 130)
-      for (int w = 0; w < 8; ++w) t += dyv[8 * (tid - 128) + w];
-    if (tid < 130) part[tid] = t;
+    if (tid < 128) part[tid] = t;
   } else {
     const int layer = tile < 2 ? 0 : tile < 10 ? 1 : 2;
     const int lt = tile - (layer == 0 ? 0 : layer == 1 ? 2 : 10);
@@ -293,11 +334,7 @@ __global__ void __cluster_dims__(kGSplit, 1, 1) __launch_bounds__(kTThreads)
     return s;
   };
   if (tile == kGTiles - 1) {
-    if (rank == 0) {
-      if (tid < 128) A.gW[3][tid] = total(tid);
-      if (tid == 128) A.gb[3][0] = total(128);
-      if (tid == 129) A.loss[0] = total(129) / (float)A.M;
-    }
+    if (rank == 0 && tid < 128) A.gW[3][tid] = total(tid);
   } else {
     const int layer = tile < 2 ? 0 : tile < 10 ? 1 : 2;
     const int lt = tile - (layer == 0 ? 0 : layer == 1 ? 2 : 10);
@@ -377,7 +414,7 @@ extern "C" int poyd_mlp_backward(const void *X, int32_t M, const void *H1, const
   cudaStream_t st = (cudaStream_t)stream;
   {
     ProfScope ps("mlp_chain", st);
-    k_mlp_chain<<<(M + kTRows - 1) / kTRows, kTThreads, 0, st>>>(A);
+    k_mlp_chain<<<(M + kTRows - 1) / kTRows + 1, kTThreads, 0, st>>>(A);
   }
   {
     ProfScope ps("mlp_grads", st);
