@@ -320,7 +320,8 @@ int poyd_algn_align_affine_3(const uint8_t *si, int32_t li, const uint8_t *sj,
  * GPU keeps, from the end, the lowest-numbered final state and at every
  * column the lowest-numbered previous state (Powell's recursion can return
  * another optimal one).  Each sequence is at most 4,096 elements; the
- * choice cube needs 8 bytes per cell of la x lb x lc.
+ * choice cube needs half a byte per cell of la x lb x lc without gap
+ * openings, else 8.
  * ------------------------------------------------------------------- */
 /* powell_3D_align(sa, sb, sc, ra, rb, rc, mm, go, ge) (ukkCommon.c:111-143)
  * with host buffers: the aligned rows, leading gap column first, are
