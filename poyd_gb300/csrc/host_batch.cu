@@ -8,9 +8,10 @@
 // host-mapped memory as each batch of 32 pairs is written, so the finished
 // slots form a growing prefix of the output.  The host follows that prefix
 // and copies it down on a second stream while the DP runs; only the slots
-// of the last (shortest) pairs are copied after it.  Cutting the batch into
-// separate launches was measured slower: each launch gives up part of the
-// longest-first schedule's load balance.
+// of the last (shortest) pairs are copied after it.  (Cutting that launch into
+// several was slower: each gives up part of the schedule's load balance.)
+// k_lin_diag's batches run in one to four parts instead, by the bytes of their
+// results, and raise the flags of a part once its sequences are written.
 #include <algorithm>
 #include <chrono>
 #include <cstdio>

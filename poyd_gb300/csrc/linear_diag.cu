@@ -426,7 +426,7 @@ struct DiagPair {
   int id, lanes, width;
   int64_t words;
 };
-// The pair of position p.
+// The pair of position p (of those from A.base[0]).
 __device__ __forceinline__ DiagPair diag_pair(const LinDiagArgs &A, int p) {
   int c = 0;
   while (p >= A.base[c + 1]) ++c;
@@ -440,7 +440,7 @@ __device__ __forceinline__ DiagPair diag_pair(const LinDiagArgs &A, int p) {
 // Bound: the memory latency of a step.
 __global__ void __launch_bounds__(64) k_diag_path(const __grid_constant__ LinDiagArgs A, int per) {
   const int lane = threadIdx.x & 31;
-  const int p = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per + lane;
+  const int p = A.base[0] + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per + lane;
   if (lane >= per || p >= A.base[kLinDiagClasses]) return;
   const DiagPair D = diag_pair(A, p);
   const LinPlan P = A.plans[D.id];
@@ -515,7 +515,8 @@ __global__ void __launch_bounds__(128) k_diag_write(const __grid_constant__ LinD
   __shared__ uint8_t med[1024];
   for (int e = threadIdx.x; e < 1024; e += blockDim.x) med[e] = A.tables->median[e];
   __syncthreads();
-  const int lane = threadIdx.x & 31, p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const int p = A.base[0] + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (p >= A.base[kLinDiagClasses]) return;
   const DiagPair D = diag_pair(A, p);
   const LinPlan P = A.plans[D.id];
@@ -684,6 +685,11 @@ __global__ void __launch_bounds__(128) k_diag_scatter(int n, int min_lanes, cons
   if (ok) order[at] = id;
 }
 
+__global__ void k_diag_flags(int *done, int b0, int b1) {
+  const int b = b0 + blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < b1) *(volatile int *)(done + b) = 1;
+}
+
 template <bool BT>
 int diag_blocks() {
   static std::atomic<int> cache[64];
@@ -734,7 +740,7 @@ int launch_lin_diag(LinDiagArgs &A, bool bt, const int *base, cudaStream_t st) {
 }
 
 int launch_lin_diag_walk(const LinDiagArgs &A, cudaStream_t st) {
-  const unsigned n = (unsigned)A.base[kLinDiagClasses];
+  const unsigned n = (unsigned)(A.base[kLinDiagClasses] - A.base[0]);
   // four pairs a warp: the fewer, the fewer wait for another's memory (32: 1.5 ms
   // for 608 pairs of 5,000 bp, 16: 0.58, 8: 0.50, 4: 0.45, their writing included)
   const int per = 4;
@@ -742,6 +748,12 @@ int launch_lin_diag_walk(const LinDiagArgs &A, cudaStream_t st) {
   k_diag_write<<<(n + 3) / 4, 128, 0, st>>>(A);
   const cudaError_t e = cudaGetLastError();
   return e != cudaSuccess ? cuda_fail(e, "k_diag_write") : POYD_OK;
+}
+
+int launch_lin_diag_flags(int *done, int b0, int b1, cudaStream_t st) {
+  k_diag_flags<<<(b1 - b0 + 255) / 256, 256, 0, st>>>(done, b0, b1);
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? cuda_fail(e, "k_diag_flags") : POYD_OK;
 }
 
 }  // namespace poyd

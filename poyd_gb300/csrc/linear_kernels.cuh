@@ -174,6 +174,8 @@ void launch_lin_diag_order(int n, int min_lanes, bool bt, const LinPlan *plans,
                            int32_t *order, cudaStream_t st);
 int launch_lin_diag(LinDiagArgs &A, bool bt, const int *base, cudaStream_t st);
 int launch_lin_diag_walk(const LinDiagArgs &A, cudaStream_t st);  // after it, the same arguments
+// done[b0 .. b1 - 1] = 1 (host-mapped), once what was launched before is written
+int launch_lin_diag_flags(int *done, int b0, int b1, cudaStream_t st);
 void launch_lin_traceback(const LinTbArgs &A, cudaStream_t st);
 void launch_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
                             const int32_t *a_len, const int32_t *b_len, const int64_t *caps,

@@ -268,7 +268,7 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   const int mode = !want_align ? kDpCost : ((out && maxc < 16384) ? kDpChoice : kDpSets);
   // Large batches are ordered for k_lin_diag; the others, and those that prove to
   // need another kernel, as those want it.
-  const bool diag_order = mode != kDpSets && !ls && n > kDiagPairsPerSm[want_align] * sm_count();
+  const bool diag_order = mode != kDpSets && n > kDiagPairsPerSm[want_align] * sm_count();
   // the plan's error bits travel with the order totals
   int32_t *err = diag_order ? &dg->err : &os->pad;
   if (diag_order) CK(cudaMemsetAsync(dg, 0, sizeof(LinDiagOrder), st));
@@ -350,10 +350,10 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   }
   if (var.packed == 0) packed = false;
   // k_lin_diag runs the pairs that its classes hold, unless a tuned variant
-  // asks for another kernel (or the batch is streamed, its results wanted as
-  // they come: k_lin_dp4 walks its pairs on the way).
+  // asks for another kernel (a streamed batch's flags need one kernel for all).
   const int diag_n = diag_order ? dt.base[kLinDiagClasses] : 0;
-  bool diag = packed && diag_n > 0 && var.packed < 0 && var.blocks_per_sm == 0 && var.solo < 0;
+  bool diag = packed && diag_n > 0 && var.packed < 0 && var.blocks_per_sm == 0 && var.solo < 0 &&
+              !(ls && diag_n < n);
   int64_t need = !want_align ? 0 : (int64_t)(diag ? dt.total : tl.total);
   // Waves: consecutive runs of a longest-first order whose direction
   // matrices fit the device-memory budget, one persistent launch each; one
@@ -468,15 +468,40 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     GA.tb.n = n; GA.tb.seq = seq; GA.tb.plans = plans; GA.tb.dm_off = doff; GA.tb.dm = dm;
     GA.tb.tables = tabs; GA.tb.gap = cm->gap; GA.tb.out = out; GA.tb.out_off = out_off;
     GA.tb.out_len = out_len; GA.tb.swaped = -1; GA.tb.mode = mode; GA.tb.order = dord;
-    {
-      ProfScope ps(want_align ? "lin_dp_dm" : "lin_dp_cost", st);
-      rc = launch_lin_diag(GA, want_align, dt.base, st);
+    // A streamed batch runs in parts, whose results the caller downloads while the
+    // next ones are computed; the last is small, since nothing hides its download.
+    // A part gives up some of the schedule's balance (about 0.5 ms), as long as 100
+    // MB of results take.
+    std::vector<int32_t> cuts{0, diag_n};
+    if (ls) {
+      const int32_t last = order[(size_t)n - 1];
+      const int64_t bytes = ls->out_off_host[last] + 4 * slot_cap(ls->a_len_h[last], ls->b_len_h[last]);
+      std::vector<double> at;
+      if (bytes >= (int64_t)128 << 20) at = {0.4, 0.7, 0.9};
+      else if (bytes >= (int64_t)16 << 20) at = {0.7};
+      int32_t p = 0;
+      for (const double f : at) {
+        while (p < n && (double)ls->out_off_host[order[p]] < f * (double)bytes) p += kLanes;
+        if (p > cuts[cuts.size() - 2] && p < n) cuts.insert(cuts.end() - 1, p);
+      }
     }
-    if (!rc && want_align) {
-      ProfScope ps("lin_traceback", st);
-      rc = launch_lin_diag_walk(GA, st);
+    for (size_t c = 0; c + 1 < cuts.size(); ++c) {
+      int base[kLinDiagClasses + 1];
+      for (int k = 0; k <= kLinDiagClasses; ++k)
+        base[k] = std::min(std::max(dt.base[k], cuts[c]), cuts[c + 1]);
+      if (c) CK(cudaMemsetAsync(GA.counter, 0, sizeof(int), st));
+      {
+        ProfScope ps(want_align ? "lin_dp_dm" : "lin_dp_cost", st);
+        rc = launch_lin_diag(GA, want_align, base, st);
+      }
+      if (!rc && want_align) {
+        ProfScope ps("lin_traceback", st);
+        rc = launch_lin_diag_walk(GA, st);
+      }
+      if (!rc && ls)
+        rc = launch_lin_diag_flags(ls->done, cuts[c] / kLanes, (cuts[c + 1] + kLanes - 1) / kLanes, st);
+      if (rc) return rc;
     }
-    if (rc) return rc;
     if (diag_n == n) return POYD_OK;
     wave_at.assign({diag_n, n});  // the pairs of wider bands
   }
