@@ -53,17 +53,18 @@ __global__ void k_fitch_distance(const uint8_t *nodes, int64_t stride, int len, 
   const int nv = (len + 15) >> 4;
   constexpr int kBatch = 4;
   int cnt = 0;
-  for (int v0 = lane; v0 < nv; v0 += 32 * kBatch) {
+  for (int base = 0; base < nv; base += 32 * kBatch) {
     uint4 x[kBatch], y[kBatch];
 #pragma unroll
     for (int e = 0; e < kBatch; ++e) {
-      const int v = v0 + 32 * e;
+      const int v = base + 32 * e + lane;
       x[e] = y[e] = make_uint4(0, 0, 0, 0);
       if (v < nv) x[e] = a[v], y[e] = b[v];
     }
 #pragma unroll
     for (int e = 0; e < kBatch; ++e) {
-      const int valid = min(max(len - 16 * (v0 + 32 * e), 0), 16);
+      if (base + 32 * e >= nv) break;  // short rows: nothing past the warp's last vector
+      const int valid = min(max(len - 16 * (base + 32 * e + lane), 0), 16);
       uint32_t n0 = nzbits(x[e].x & y[e].x), n1 = nzbits(x[e].y & y[e].y);
       uint32_t n2 = nzbits(x[e].z & y[e].z), n3 = nzbits(x[e].w & y[e].w);
       if (valid < 16) {
