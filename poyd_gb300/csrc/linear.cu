@@ -179,6 +179,9 @@ __global__ void __launch_bounds__(128, 16) k_lin_plan(LinPlanArgs A) {
     if (la < 1 || lb < 1) atomicOr(A.err, 1);
     if (wide) atomicOr(A.err, 4);  // codes index 32-entry table rows
     if ((long long)A.maxc * (l1 + l2 + 2) >= kMaxCost) atomicOr(A.err, 2);
+    // A negative deltaw[i] can leave the first or the final cell outside the band;
+    // k_lin_team and k_lin_diag size their tables by a path through it.
+    if (dlo > l2 - l1 || dhi < 0) atomicOr(A.err, kPlanNoPath);
   }
 }
 

@@ -97,6 +97,8 @@ void launch_lin_order_small(int n, const LinPlan *plans, const int64_t *dm_words
                             int64_t *dm_off, LinOrderScratch *os, int *counter, int *batch_done,
                             int nbatch, cudaStream_t st);
 
+// LinPlanArgs::err: some pair's band does not hold both ends of a path.
+constexpr int kPlanNoPath = 32;
 void launch_lin_plan(const LinPlanArgs &A, cudaStream_t st);
 int lin_dp_blocks(int mode);
 void launch_lin_dp(const LinDpArgs &A, int mode, int blocks, cudaStream_t st);

@@ -349,10 +349,11 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     }
   }
   if (var.packed == 0) packed = false;
+  const bool path = !(tl.err & kPlanNoPath);  // else k_lin_dp4 or the 32-bit kernel
   // k_lin_diag runs the pairs that its classes hold, unless a tuned variant
   // asks for another kernel (a streamed batch's flags need one kernel for all).
   const int diag_n = diag_order ? dt.base[kLinDiagClasses] : 0;
-  bool diag = packed && diag_n > 0 && var.packed < 0 && var.blocks_per_sm == 0 && var.solo < 0 &&
+  bool diag = packed && path && diag_n > 0 && var.packed < 0 && var.blocks_per_sm == 0 && var.solo < 0 &&
               !(ls && diag_n < n);
   int64_t need = !want_align ? 0 : (int64_t)(diag ? dt.total : tl.total);
   // Waves: consecutive runs of a longest-first order whose direction
@@ -432,7 +433,7 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   // A small batch takes a block per pair (k_lin_team) unless a tuned variant
   // says otherwise: up to three pairs an SM, beyond which a warp per pair
   // keeps the SMs busier.
-  const int team = packed && small && !host_waves && var.packed < 0 && var.blocks_per_sm == 0 &&
+  const int team = packed && path && small && !host_waves && var.packed < 0 && var.blocks_per_sm == 0 &&
                            var.solo < 0 && n <= kTeamPairsPerSm * sm_count()
                        ? lin_team_width(maxwd, tl.maxsum) : 0;
   if (team) {
