@@ -170,7 +170,7 @@ int poyd_pack_alignments(int32_t n, const uint8_t *out, const int64_t *out_off,
                          const int64_t *packed_off, void *stream);
 
 /* The layouts of such calls (no reference counterpart), from device arrays;
- * each waits for `stream`.
+ * each waits for `stream`.  Calls of the first two may overlap on a stream.
  *   poyd_slot_layout: slots of four sequences of cap[i] = len0[i] + len1[i]
  *     (+ len2[i], unless null) + extra bytes, rounded up to a multiple of 4:
  *     extra is 2 for poyd_align_2_batch, 0 for the three-sequence calls.

@@ -5,6 +5,7 @@
 // seq block per call.
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <mutex>
 #include "poyd_internal.h"
 #include "linear_kernels.cuh"
 
@@ -92,9 +93,13 @@ __global__ void __launch_bounds__(kLayThreads) k_layout(const LayoutArgs A) {
   }
 }
 
+// Unlike other calls, layouts of several threads may overlap on a stream: a caller
+// whose batches have streams of their own sizes them on the current one.
 int layout(const LayoutArgs &in, bool pack, int64_t *total, int64_t *least, cudaStream_t st) {
   LayoutArgs A = in;
-  A.total = (int64_t *)ws_buffer(workspace(st), WS_LAYOUT, 2 * sizeof(int64_t));
+  Workspace *w = workspace(st);
+  std::lock_guard<std::mutex> lk(ws_layout_mutex(w));
+  A.total = (int64_t *)ws_buffer(w, WS_LAYOUT, 2 * sizeof(int64_t));
   if (!A.total) return fail(POYD_ENOMEM, "layout allocation failed");
   if (pack) k_layout<true><<<1, kLayThreads, 0, st>>>(A);
   else k_layout<false><<<1, kLayThreads, 0, st>>>(A);

@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <cstddef>
 #include <cuda_runtime.h>
+#include <mutex>
 #include <vector>
 #include "poyd_gb300.h"
 
@@ -85,6 +86,7 @@ Workspace *workspace(cudaStream_t st = nullptr);  // per (current device, stream
 // Grow-only device buffer `slot` of at least `bytes`; returns nullptr on failure.
 void *ws_buffer(Workspace *w, int slot, size_t bytes);
 size_t ws_size(const Workspace *w, int slot);  // bytes it holds now
+std::mutex &ws_layout_mutex(Workspace *w);     // held from a layout's launch to its read-back
 enum WsSlot {
   WS_TABLES = 0, WS_PLANS, WS_DMWORDS, WS_WD, WS_ORDER, WS_DM, WS_SCRATCH,
   WS_COUNTER, WS_CELLS, WS_AFF, WS_ERR, WS_SEQ, WS_META, WS_OUT, WS_BATCH, WS_ORDSCR,

@@ -45,6 +45,7 @@ struct Workspace {
   size_t size[WS_NSLOTS] = {};
   poyd_cm last_cm;
   bool have_cm = false;
+  std::mutex layout;  // WS_LAYOUT: layouts may overlap on a stream
 };
 
 static std::mutex g_ws_mu;
@@ -83,6 +84,7 @@ extern "C" int poyd_workspace_release(void) {
 }
 
 size_t ws_size(const Workspace *w, int slot) { return w->size[slot]; }
+std::mutex &ws_layout_mutex(Workspace *w) { return w->layout; }
 
 void *ws_buffer(Workspace *w, int slot, size_t bytes) {
   if (bytes == 0) bytes = 16;
