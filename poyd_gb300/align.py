@@ -91,9 +91,25 @@ def _native_ok(dtype, *tensors) -> bool:
                t.device.index == torch.cuda.current_device() for t in tensors)
 
 
-def slot_layout(lens, extra: int):
+def _order_after(stream):
+    """What the current stream does next waits for what `stream` has been given."""
+    if stream is not None and stream != torch.cuda.current_stream():
+        torch.cuda.current_stream().wait_stream(stream)
+
+
+def _keep_for(stream, *temporaries):
+    """The tensors' memory is not reused before `stream` has done with them."""
+    if stream is not None:
+        for t in temporaries:
+            if t.numel():
+                t.record_stream(stream)
+
+
+def slot_layout(lens, extra: int, stream=None):
     """(offsets, total bytes, capacities) of output slots of 4 sequences of
-    capacity sum(lens) + extra, rounded up to a multiple of 4."""
+    capacity sum(lens) + extra, rounded up to a multiple of 4; made on the current
+    stream, after what `stream` has been given."""
+    _order_after(stream)
     n = int(lens[0].numel())
     if n and all(t.dim() == 1 and t.numel() == n for t in lens) and _native_ok(torch.int32, *lens):
         off = torch.empty(n, dtype=torch.int64, device=lens[0].device)
@@ -156,10 +172,10 @@ class PairBatch:
              for x in parts]
         return cls(*t)
 
-    def out_layout(self):
+    def out_layout(self, stream=None):
         """Per-pair output slot offsets: 4 sequences of cap = la + lb + 2
         rounded up to a multiple of 4 (the library's slot_cap)."""
-        return slot_layout((self.a_len, self.b_len), 2)
+        return slot_layout((self.a_len, self.b_len), 2, stream)
 
 
 def cost_2(batch: PairBatch, cm: CostMatrix, deltaw=None, band_cells: bool = False,
@@ -226,7 +242,9 @@ class AlignResult:
     def pack(self, stream=None) -> "PackedAlignments":
         """The results packed back to back on the device (aligned a, aligned
         b, median with gaps, median per pair), ready for one download of
-        only the bytes that hold results."""
+        only the bytes that hold results.  With `stream`, after what that stream
+        has been given; the lengths are read on the current stream."""
+        _order_after(stream)
         n = self.cost.numel()
         dev = self.cost.device
         if n and _native_ok(torch.int32, self.out_len) and \
@@ -242,6 +260,7 @@ class AlignResult:
                     n, self.out.data_ptr(), self.out_off.data_ptr(), self.cap.data_ptr(),
                     self.out_len.data_ptr(), packed.data_ptr(), off.data_ptr(),
                     _stream_handle(stream)))
+                _keep_for(stream, off)
                 return PackedAlignments(self.cost, packed[:total.value], self.out_len)
         ln = self.out_len.view(-1, 2).to(torch.int64)
         sizes = 3 * ln[:, 0] + ln[:, 1]
@@ -256,9 +275,12 @@ class AlignResult:
         packed = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
         a_len = (self.cap - 2).to(torch.int32)  # slot_cap(cap - 2, 0) == cap
         zeros = torch.zeros_like(a_len)
+        if stream is not None:
+            stream.wait_stream(torch.cuda.current_stream())
         check(lib().poyd_pack_alignments(
             n, self.out.data_ptr(), self.out_off.data_ptr(), a_len.data_ptr(), zeros.data_ptr(),
             self.out_len.data_ptr(), packed.data_ptr(), off.data_ptr(), _stream_handle(stream)))
+        _keep_for(stream, off, a_len, zeros)
         return PackedAlignments(self.cost, packed[:total], self.out_len)
 
 
@@ -300,7 +322,7 @@ def align_2(batch: PairBatch, cm: CostMatrix, dos_empty: bool = False,
     output layout (out_off, total, cap) the caller computed from host
     copies of the lengths, saving the device read-back of the total."""
     dev = batch.seq.device
-    out_off, total, cap = batch.out_layout() if layout is None else layout
+    out_off, total, cap = batch.out_layout(stream) if layout is None else layout
     out = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
     cost = torch.empty(batch.n, dtype=torch.int32, device=dev)
     out_len = torch.empty(2 * batch.n, dtype=torch.int32, device=dev)
@@ -324,7 +346,7 @@ def autotune(batch: PairBatch, cm: CostMatrix, align: bool = True, deltaw=None,
     cost = torch.empty(batch.n, dtype=torch.int32, device=dev)
     out = out_off = out_len = None
     if align:
-        out_off, total, _ = batch.out_layout()
+        out_off, total, _ = batch.out_layout(stream)
         out = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
         out_len = torch.empty(2 * batch.n, dtype=torch.int32, device=dev)
     pol = native.DELTAW_DOS_DISTANCE if deltaw == "dos" else native.DELTAW_DEFAULT
@@ -384,7 +406,7 @@ def closest(batch: PairBatch, cm: CostMatrix, dos_empty: bool = True,
     empty rules with `dos_empty`, seqCS.ml:730-745); ``cost`` is the
     alignment cost of the pair."""
     dev = batch.seq.device
-    out_off, total, cap = batch.out_layout()
+    out_off, total, cap = batch.out_layout(stream)
     out = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
     cost = torch.empty(batch.n, dtype=torch.int32, device=dev)
     out_len = torch.empty(2 * batch.n, dtype=torch.int32, device=dev)

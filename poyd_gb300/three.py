@@ -52,11 +52,11 @@ class TripleBatch:
                    [torch.from_numpy(x).to(device) for x in offs],
                    [torch.from_numpy(x).to(device) for x in lens])
 
-    def out_layout(self):
+    def out_layout(self, stream=None):
         """Slots of 4 sequences of cap = a + b + c (first three lengths)
         rounded up to a multiple of 4."""
         third = self.lens[3] if len(self.lens) == 4 else self.lens[2]
-        return slot_layout((self.lens[0], self.lens[1], third), 0)
+        return slot_layout((self.lens[0], self.lens[1], third), 0, stream)
 
 
 class ThreeResult:
@@ -105,7 +105,7 @@ def align_3_powell(batch: TripleBatch, mm: int, go: int, ge: int, cm: CostMatrix
     """Batched ``align_3_powell`` (sequence.ml:1078-1087); with `cm`, also
     the median ``align_3_powell_inter`` builds (sequence.ml:1103-1115)."""
     dev = batch.seq.device
-    out_off, total, cap = batch.out_layout()
+    out_off, total, cap = batch.out_layout(stream)
     out = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
     cost = torch.empty(batch.n, dtype=torch.int32, device=dev)
     out_len = torch.empty(2 * batch.n, dtype=torch.int32, device=dev)
@@ -125,7 +125,7 @@ def readjust_3d(batch: TripleBatch, cm: CostMatrix, stream=None) -> ThreeResult:
     if len(batch.lens) != 4:
         raise ValueError("readjust_3d items are (s1, s2, m, p)")
     dev = batch.seq.device
-    out_off, total, cap = batch.out_layout()  # slots sized by s1 + s2 + p
+    out_off, total, cap = batch.out_layout(stream)  # slots sized by s1 + s2 + p
     out = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
     cost = torch.empty(batch.n, dtype=torch.int32, device=dev)
     out_len = torch.empty(2 * batch.n, dtype=torch.int32, device=dev)
