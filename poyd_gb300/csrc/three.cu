@@ -47,7 +47,6 @@ namespace poyd {
 
 constexpr int kP3Threads = 256;
 constexpr int kP3Inf = 1 << 30;      // x16 domain
-constexpr int kP3MaxLen = 4096;
 
 // The same tables for indices known only at run time (traceback, table
 // setup): constant memory rather than a local copy.

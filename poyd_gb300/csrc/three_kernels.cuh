@@ -7,6 +7,7 @@
 namespace poyd {
 
 constexpr int kP3States = 16;
+constexpr int kP3MaxLen = 4096;  // elements of a sequence that the entry points take
 
 // Powell's column states (ukkCommon.c:206-262): per sequence match (M),
 // delete (D) or insert (I), at least one M and at most one I, numbered in

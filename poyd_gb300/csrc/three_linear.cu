@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(32 * kW) k_p3_linear(const __grid_constant__ L
   }
 }
 
-size_t lin3_smem(int warps, int longest) {
+constexpr size_t lin3_smem(int warps, int longest) {
   return (size_t)warps * 2 * 8 * (32 * 8 + 16) + 2 * ((size_t)longest + 40 + 48);
 }
 
@@ -368,8 +368,11 @@ int lin3_blocks(int longest) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t sm = lin3_smem(kW, longest);
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_p3_linear<kW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // The same request for every batch: it is one value per kernel and device, which
+  // a thread with shorter sequences would lower under another's launch.
+  constexpr size_t most = lin3_smem(kW, kP3MaxLen);
+  if (most > 48 * 1024)
+    cudaFuncSetAttribute(k_p3_linear<kW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_p3_linear<kW>, 32 * kW, sm) != cudaSuccess)
     per = 1;
   return std::max(per, 1) * std::max(sms, 1);

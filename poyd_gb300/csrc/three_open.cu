@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(32 * kOpenWarps, 2) k_p3_open(const __grid_con
   }
 }
 
-size_t open_smem(int longest) {
+constexpr size_t open_smem(int longest) {
   return (size_t)kOpenWarps * 2 * 8 * (32 + 2) * 16 + 2 * ((size_t)longest + 40 + 48);
 }
 
@@ -444,9 +444,10 @@ int launch_p3_open(const P3Args &A, bool clamp, int longest, int blocks, int csi
   const cudaLaunchConfig_t cfg = open_config(blocks, csize, longest, &at, st);
   auto kern = csize > 1 ? (clamp ? k_p3_open<true, true> : k_p3_open<true, false>)
                         : (clamp ? k_p3_open<false, true> : k_p3_open<false, false>);
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)cfg.dynamicSmemBytes);
+  // the same request for every batch (one value per kernel and device, which a
+  // thread with shorter sequences would lower under another's launch)
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(csize > 1 ? kOpenClusterSmem : open_smem(kP3MaxLen)));
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_p3_open)");
   ProfScope ps("p3", st);
   e = cudaLaunchKernelEx(&cfg, kern, B);

@@ -1,13 +1,14 @@
 """Calls of several host threads, each with a stream of its own, while torch's
 current stream stays the default one: the layouts of their results, which run on
-the current stream, do not see each other's totals."""
+the current stream, do not see each other's totals, and a batch of short triples
+does not take from a batch of long ones the shared memory that it asked for."""
 import threading
 
 import numpy as np
 import pytest
 import torch
 
-from poyd_gb300 import align, synth
+from poyd_gb300 import align, synth, three
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +63,25 @@ def test_alignments_and_packs_overlap():
         return f
 
     run_threads([worker(b, w) for b, w in zip(batches, want)])
+
+
+# with openings a block a triple; without, sixteen warps for both shapes
+@pytest.mark.parametrize("go,shapes", [(3, ((2, 1, 2), (300, 1, 300))),
+                                       (0, ((4, 600, 900), (4, 600, 1200)))])
+def test_triples_of_different_lengths_overlap(monkeypatch, go, shapes):
+    monkeypatch.setenv("POYD_P3_CLUSTER", "0")
+    rng = np.random.default_rng(go)
+
+    def worker(lens):
+        T = [synth.with_gap(synth.random_dna(rng, n)) for n in lens]
+        b = three.TripleBatch.from_host([tuple(T)])
+        want = three.align_3_powell(b, 1, go, 2).cost.item()
+        s = torch.cuda.Stream()
+        def f():
+            for _ in range(1500):
+                r = three.align_3_powell(b, 1, go, 2, stream=s)
+                s.synchronize()
+            assert r.cost.item() == want
+        return f
+
+    run_threads([worker(n) for n in shapes for _ in range(2)])
