@@ -16,7 +16,8 @@
 //     is ready and run beside the other half's epilogue;
 //   * the 128 -> 1 head from registers by four warps of its own, while the others
 //     take the next tile's layer 1, whose sums go to Q.
-// Measured: 984,102 rows from fp32 in 0.227 ms (0.93 PFLOP/s) where eight warps
+// Measured: 984,102 rows from fp32 in 0.203 ms (1.03 PFLOP/s; 0.226 where the code
+// that keeps activations was not a kernel of its own) where eight warps
 // with one tile's products and epilogues in turn took 0.29 ms, and the mma.sync
 // kernel with its weights in L2 1.21 ms, the input's conversion and the weights'
 // transposes 33 us more.  What bounds it: the chain of a tile, 0.144 ms of it the
@@ -106,6 +107,10 @@ __device__ __forceinline__ bool m_wait(uint32_t bar, uint32_t parity) {
   }
   return false;
 }
+// The .aligned instructions, the main warps' barrier among them, want the whole
+// warp.  Lanes part in waits, in what one thread does alone and in loads of rows
+// past M: a __syncwarp() follows each of these (0.8 % of 984,102 rows' time; one
+// before every such instruction 1.5 %).  Activations are stored by predicate.
 __device__ __forceinline__ void m_ld32(uint32_t (&r)[32], uint32_t addr) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -126,6 +131,13 @@ __device__ __forceinline__ void m_st16(uint32_t addr, const uint32_t (&r)[16]) {
       "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
       "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// 16 bytes at p unless it is null, without a branch.
+__device__ __forceinline__ void m_keep(void *p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.u64 p, %0, 0;\n@p st.global.v4.b32 [%0], {%1, %2, %3, %4};\n}\n" ::"l"(p),
+      "r"(a), "r"(b), "r"(c), "r"(d)
       : "memory");
 }
 __device__ __forceinline__ void m_before() {
@@ -232,8 +244,9 @@ __device__ __forceinline__ uint4 m_bf16_x(const MlpFwdArgs &A, const MlpX &x) {
 }
 
 // A hidden layer's epilogue for this thread's row and 32 columns: the sums at
-// `reg` become the next layer's packed A operand in place (and, when h is
+// `reg` become the next layer's packed A operand in place (KEEP: and, when h is
 // given, row-major activations).
+template <bool KEEP>
 __device__ __forceinline__ void m_epilogue(uint32_t reg, const float *bias, uint16_t *h) {
   uint32_t r[32], p[16];
   m_ld32(r, reg);
@@ -244,16 +257,15 @@ __device__ __forceinline__ void m_epilogue(uint32_t reg, const float *bias, uint
     p[2 * q + 1] = m_bias_relu(r[4 * q + 2], r[4 * q + 3], bb.z, bb.w);
   }
   m_st16(reg, p);
-  if (h) {
-    uint4 *o = reinterpret_cast<uint4 *>(h);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) o[q] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
-  }
+  for (int q = 0; KEEP && q < 4; ++q)
+    m_keep(h ? h + 8 * q : nullptr, p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // The third layer's epilogue and the head of this thread's row: s[l] sums
 // columns l, l + 32, l + 64, l + 96, then the butterfly's tree over l.
+template <bool KEEP>
 __device__ __forceinline__ float m_head(uint32_t reg, const float *b3, const float *w4, uint16_t *h) {
   float s[32];
 #pragma unroll
@@ -273,11 +285,9 @@ __device__ __forceinline__ float m_head(uint32_t reg, const float *b3, const flo
       s[4 * q + 2] = fmaf(__uint_as_float(r[2 * q + 1] << 16), ww.z, s[4 * q + 2]);
       s[4 * q + 3] = fmaf(__uint_as_float(r[2 * q + 1] & 0xFFFF0000u), ww.w, s[4 * q + 3]);
     }
-    if (h) {
-      uint4 *o = reinterpret_cast<uint4 *>(h + 32 * c);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-    }
+    for (int q = 0; KEEP && q < 4; ++q)
+      m_keep(h ? h + 32 * c + 8 * q : nullptr, r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
@@ -286,6 +296,8 @@ __device__ __forceinline__ float m_head(uint32_t reg, const float *b3, const flo
   return s[0];
 }
 
+// KEEP: the hidden layers' activations are wanted.
+template <bool KEEP>
 __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_constant__ MlpFwdArgs A) {
   extern __shared__ unsigned char mlp_raw[];
   uint8_t *sm = mlp_raw + ((128 - ((uint32_t)__cvta_generic_to_shared(mlp_raw) & 127)) & 127);
@@ -368,7 +380,8 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
       wait(bar1, i & 1);
       put_x(x);
       x = get_x(tn + gridDim.x);
-      m_epilogue(P + mine, b1, h1);
+      __syncwarp();
+      m_epilogue<KEEP>(P + mine, b1, h1);
       m_before();
       if (m_main_sync(*dead)) break;
       if (tid == 0) {
@@ -376,7 +389,8 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
         m_after();
         half(Q, P, kMW2, 0, kMH2);
       }
-      m_epilogue(P + mine + 128, b1 + 128, h1 ? h1 + 128 : nullptr);
+      __syncwarp();
+      m_epilogue<KEEP>(P + mine + 128, b1 + 128, h1 ? h1 + 128 : nullptr);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next inputs
       m_before();
       if (m_main_sync(*dead)) break;
@@ -386,14 +400,16 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
         m_commit(bar2);
       }
       wait(bar2, i & 1);
-      m_epilogue(Q + mine, b2, h2);
+      __syncwarp();
+      m_epilogue<KEEP>(Q + mine, b2, h2);
       m_before();
       if (m_main_sync(*dead)) break;
       if (tid == 0) {
         m_after();
         half(P, Q, kMW3, 0, kMH3);
       }
-      m_epilogue(Q + mine + 128, b2 + 128, h2 ? h2 + 128 : nullptr);
+      __syncwarp();
+      m_epilogue<KEEP>(Q + mine + 128, b2 + 128, h2 ? h2 + 128 : nullptr);
       m_before();
       if (m_main_sync(*dead)) break;
       if (tid == 0) {
@@ -405,12 +421,14 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
       }
     }
   } else {
-    for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++i) {
+    // a warp leaves as one: its lanes may read the mark at different times
+    for (int t = blockIdx.x; t < tiles && !__any_sync(0xffffffffu, *dead); t += gridDim.x, ++i) {
       const uint32_t P = tm + 256 * (i & 1);
       const int64_t m = (int64_t)t * kMRows + row;
       const bool in = m < A.M;
       wait(bar3, i & 1);
-      const float s = m_head(P + lane_base, bias + 512, bias + 640,
+      __syncwarp();
+      const float s = m_head<KEEP>(P + lane_base, bias + 512, bias + 640,
                              in && A.H[2] ? A.H[2] + m * kMH3 : nullptr);
       m_before();
       __syncwarp();
@@ -426,6 +444,7 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
       if (quarter == 4 && t * kMRows + row < A.M) A.y[t * kMRows + row] = __int_as_float(0x7FFFFFFF);
   if (warp == 0) {
     m_after();
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm) : "memory");
   }
 }
@@ -441,13 +460,14 @@ int mlp_forward(const MlpFwdArgs &A, cudaStream_t st) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  auto kern = A.H[0] || A.H[1] || A.H[2] ? k_mlp_forward<true> : k_mlp_forward<false>;
   const cudaError_t e =
-      cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kMSmem);
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMSmem);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_mlp_forward)");
   const int tiles = (A.M + kMRows - 1) / kMRows;
   {
     ProfScope ps("mlp_forward", st);
-    k_mlp_forward<<<tiles < sms ? tiles : sms, kMThreads, kMSmem, st>>>(A);
+    kern<<<tiles < sms ? tiles : sms, kMThreads, kMSmem, st>>>(A);
   }
   const cudaError_t l = cudaGetLastError();
   return l != cudaSuccess ? cuda_fail(l, "k_mlp_forward") : POYD_OK;
