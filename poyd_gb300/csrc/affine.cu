@@ -109,7 +109,8 @@ struct AffTbArgs {
 // pair took 381 us for 16,384 pairs of 100-5,000 bp).
 __global__ void __launch_bounds__(128) k_aff_plan(AffPlanArgs A) {
   const int lane = threadIdx.x & 31;
-  const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // (a thread's own number would pass 32 bits at 2^27 pairs)
+  const int id = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   if (id >= A.n) return;
   const int la = A.a_len[id], lb = A.b_len[id];
   const int64_t ao = A.a_off[id], bo = A.b_off[id];

@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(128) k_aff_walk(const __grid_constant__ AffWal
     med[t] = A.tables->median[(t >> 4) << 5 | (t & 15)];
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int p = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   if (p >= A.n) return;
   const int id = A.order[p];
   if (id < 0) return;  // a task's missing pair
