@@ -65,6 +65,9 @@ struct MlpFwdArgs {
   float *y;
 };
 
+__host__ __device__ constexpr int m_tiles(int rows) {
+  return (int)(((int64_t)rows + kMRows - 1) / kMRows);
+}
 __device__ __forceinline__ uint64_t m_desc(uint32_t addr, uint32_t sbo) {
   return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(128 >> 4) << 16 |
          (uint64_t)(sbo >> 4) << 32 | 1ull << 46;
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(kMThreads, 1) k_mlp_forward(const __grid_const
   for (int i = tid; i < kMH1 + kMH2 + 2 * kMH3; i += kMThreads)
     bias[i] = i < 256 ? A.b[0][i] : i < 512 ? A.b[1][i - 256] : i < 640 ? A.b[2][i - 512]
               : __uint_as_float((uint32_t)A.w4[i - 640] << 16);
-  const int tiles = (A.M + kMRows - 1) / kMRows;
+  const int tiles = m_tiles(A.M);
   // a main thread's core matrix row of an input tile
   auto put_x = [&](const MlpX &x) {
     const int r = (tid & 7) | tid >> 5 << 3, kc = tid >> 3 & 3;
@@ -464,7 +467,7 @@ int mlp_forward(const MlpFwdArgs &A, cudaStream_t st) {
   const cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMSmem);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_mlp_forward)");
-  const int tiles = (A.M + kMRows - 1) / kMRows;
+  const int tiles = m_tiles(A.M);
   {
     ProfScope ps("mlp_forward", st);
     kern<<<tiles < sms ? tiles : sms, kMThreads, kMSmem, st>>>(A);
