@@ -426,43 +426,40 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
     ls->order = order;
     ls->waves = (int)wave_at.size() - 1;
   }
+  // A small batch takes a block per pair (k_lin_team) unless a tuned variant
+  // says otherwise: up to three pairs an SM, beyond which a warp per pair
+  // keeps the SMs busier.
+  int team = packed && path && small && !host_waves && var.packed < 0 && var.blocks_per_sm == 0 &&
+                     var.solo < 0 && n <= kTeamPairsPerSm * sm_count()
+                 ? lin_team_width(maxwd, tl.maxsum) : 0;
+  const int64_t team_words = team && want_align ? lin_team_words(team, tl.maxsum) : 0;
+  // One allocation, of what the kernel at hand needs: a buffer that grows waits for
+  // the device, other streams' work included.
   uint32_t *dm = nullptr;
-  if (want_align) {
+  if (team && want_align) {
+    if (team_words * n <= budget)
+      dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)(team_words * n));
+    if (!dm) team = 0;  // its matrix could not be had: the other kernels' is smaller
+  }
+  if (want_align && !team) {
     dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)max_words);
     if (!dm) return fail(POYD_ENOMEM, "direction matrix allocation (%lld bytes) failed",
                          (long long)(max_words * 4));
   }
-  // A small batch takes a block per pair (k_lin_team) unless a tuned variant
-  // says otherwise: up to three pairs an SM, beyond which a warp per pair
-  // keeps the SMs busier.
-  const int team = packed && path && small && !host_waves && var.packed < 0 && var.blocks_per_sm == 0 &&
-                           var.solo < 0 && n <= kTeamPairsPerSm * sm_count()
-                       ? lin_team_width(maxwd, tl.maxsum) : 0;
   if (team) {
-    const int64_t words = want_align ? lin_team_words(team, tl.maxsum) : 0;
-    uint32_t *tdm = dm;
-    if (want_align && words * n > max_words)
-      tdm = words * n <= budget ? (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)(words * n))
-                                : nullptr;
-    if (tdm || !want_align) {
-      LinDpArgs DA = {};
-      DA.n = n; DA.seq = seq; DA.plans = plans; DA.tables = tabs; DA.gap = cm->gap;
-      DA.dm = tdm; DA.cost = cost; DA.k = dp_constants();
-      DA.tb.n = n; DA.tb.seq = seq; DA.tb.plans = plans; DA.tb.tables = tabs; DA.tb.gap = cm->gap;
-      DA.tb.out = out; DA.tb.out_off = out_off; DA.tb.out_len = out_len;
-      DA.tb.swaped = -1; DA.tb.mode = mode;
-      {
-        ProfScope ps(want_align ? "lin_dp_dm" : "lin_dp_cost", st);
-        rc = launch_lin_team(DA, mode, team, words, tl.maxsum, st);
-      }
-      if (rc) return rc;
-      CK(cudaGetLastError());
-      return POYD_OK;
+    LinDpArgs DA = {};
+    DA.n = n; DA.seq = seq; DA.plans = plans; DA.tables = tabs; DA.gap = cm->gap;
+    DA.dm = dm; DA.cost = cost; DA.k = dp_constants();
+    DA.tb.n = n; DA.tb.seq = seq; DA.tb.plans = plans; DA.tb.tables = tabs; DA.tb.gap = cm->gap;
+    DA.tb.out = out; DA.tb.out_off = out_off; DA.tb.out_len = out_len;
+    DA.tb.swaped = -1; DA.tb.mode = mode;
+    {
+      ProfScope ps(want_align ? "lin_dp_dm" : "lin_dp_cost", st);
+      rc = launch_lin_team(DA, mode, team, team_words, tl.maxsum, st);
     }
-    // the larger matrix could not be had: the buffer of the other kernel again
-    dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)max_words);
-    if (!dm) return fail(POYD_ENOMEM, "direction matrix allocation (%lld bytes) failed",
-                         (long long)(max_words * 4));
+    if (rc) return rc;
+    CK(cudaGetLastError());
+    return POYD_OK;
   }
   if (diag) {
     LinDiagArgs GA = {};
