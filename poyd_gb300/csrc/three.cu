@@ -415,14 +415,17 @@ static int p3_run(int mode, int32_t n, const uint8_t *seq, const int64_t *const 
     int blocks = (int)fit(std::min<int64_t>(n, 2LL * sms), open_plane, open_dir);
     uint8_t *plane = (uint8_t *)ws_buffer(w, WS_P3_RING, (size_t)(open_plane * blocks));
     uint8_t *dirb = (uint8_t *)ws_buffer(w, WS_P3_DIR, (size_t)(open_dir * blocks));
-    if (!plane || !dirb) return fail(POYD_ENOMEM, "three-sequence workspace (%d blocks)", blocks);
-    // a sum of an opened value and a column cost may pass 16 bits: cut it off
-    const bool clamp = 48LL * go + 16LL * (2LL * mm + 3LL * ge) + 31 >= 0x4000;
-    int rc = launch_p3_open(A, clamp, longest, blocks, csize, plane, open_plane, dirb, open_dir, st);
-    if (rc) return rc;
-    bool redo = false;
-    rc = finish(&redo);
-    if (rc || !redo) return rc;
+    // Its strips of 32 want more memory than k_p3's cube (a sixteenth more, up to 32
+    // times for a b of one element): what that can hold is not refused.
+    if (plane && dirb) {
+      // a sum of an opened value and a column cost may pass 16 bits: cut it off
+      const bool clamp = 48LL * go + 16LL * (2LL * mm + 3LL * ge) + 31 >= 0x4000;
+      int rc = launch_p3_open(A, clamp, longest, blocks, csize, plane, open_plane, dirb, open_dir, st);
+      if (rc) return rc;
+      bool redo = false;
+      rc = finish(&redo);
+      if (rc || !redo) return rc;
+    }
   }
   const int64_t blocks = fit(std::min<int64_t>(n, 3LL * sms), ring_max * 4, dir_max * 8);
   A.ring = (int32_t *)ws_buffer(w, WS_P3_RING, (size_t)(ring_max * 4 * blocks));
