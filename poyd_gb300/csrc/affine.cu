@@ -1001,53 +1001,74 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   CKA(cudaGetDevice(&dev));
   CKA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const bool spread = want_align && n <= kDiagSpreadPerSm * sms;
-  std::vector<int32_t> order, rows_of, slots[kDiagClassN];
+  std::vector<int32_t> order, all;  // all: the tasks' pairs, then the rows kernels'
   longest_first(key, order);
-  for (int32_t id : order) {
-    const int c = (hwd[id] & kAffFits) ? aff_diag_class((hwd[id] & ~kAffFits) - 41, spread) : kDiagClassN;
-    if (c == kDiagClassN) rows_of.push_back(id);
-    else slots[c].push_back(id);
-  }
-  struct Task {
-    int cls, at;  // the class and the first of its pairs in slots[cls]
+  std::vector<int64_t> task_word, off, hw;
+  int diag = 0, rows = 0, maxwd = 1;
+  int64_t total = 0;  // direction words
+  auto divide = [&](bool by_diag) -> int {
+    std::vector<int32_t> rows_of, slots[kDiagClassN], torder;
+    for (int32_t id : order) {
+      const int c = by_diag && (hwd[id] & kAffFits) ? aff_diag_class((hwd[id] & ~kAffFits) - 41, spread)
+                                                    : kDiagClassN;
+      if (c == kDiagClassN) rows_of.push_back(id);
+      else slots[c].push_back(id);
+    }
+    struct Task {
+      int cls, at;  // the class and the first of its pairs in slots[cls]
+    };
+    std::vector<Task> tasks;
+    key.clear();
+    for (int c = 0; c < kDiagClassN; ++c) {
+      const int per = 32 / kDiagClasses[c].lanes;
+      for (int at = 0; at < (int)slots[c].size(); at += per) {
+        tasks.push_back({c, at});
+        key.push_back((int64_t)hwd[(size_t)n + slots[c][at]] * kDiagClasses[c].width << 3);
+      }
+    }
+    longest_first(key, torder);
+    task_word.clear();
+    all.clear();
+    total = 0;
+    for (int32_t q : torder) {
+      const Task t = tasks[q];
+      const AffDiagClass c = kDiagClasses[t.cls];
+      task_word.push_back(aff_diag_task(total, c));
+      if (want_align) total += aff_diag_words(c.width, hwd[(size_t)n + slots[t.cls][t.at]]);
+      for (int g = 0; g < kDiagTask; ++g) {
+        const bool in = g < 32 / c.lanes && t.at + g < (int)slots[t.cls].size();
+        all.push_back(in ? slots[t.cls][t.at + g] : -1);
+      }
+    }
+    diag = (int)all.size(), rows = (int)rows_of.size();
+    all.insert(all.end(), rows_of.begin(), rows_of.end());
+    if (rows) {
+      hw.resize((size_t)n);
+      CKA(cudaMemcpyAsync(hw.data(), dmw, sizeof(int64_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
+      CKA(cudaStreamSynchronize(st));
+      off.assign((size_t)n, 0);
+      for (int32_t id : rows_of) {
+        off[id] = total;
+        if (want_align) total += hw[id];
+        maxwd = std::max(maxwd, hwd[id] & ~kAffFits);
+      }
+    }
+    return POYD_OK;
   };
-  std::vector<Task> tasks;
-  key.clear();
-  for (int c = 0; c < kDiagClassN; ++c) {
-    const int per = 32 / kDiagClasses[c].lanes;
-    for (int at = 0; at < (int)slots[c].size(); at += per) {
-      tasks.push_back({c, at});
-      key.push_back((int64_t)hwd[(size_t)n + slots[c][at]] * kDiagClasses[c].width << 3);
+  if ((rc = divide(true))) return rc;
+  uint32_t *dm = nullptr;
+  if (want_align) {
+    auto matrix = [&]() {
+      dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)std::max<int64_t>(total, 1));
+    };
+    matrix();
+    if (!dm && diag) {
+      // k_aff_diag's matrix holds a band for each step of both sequences, the rows
+      // kernels' one for each row: far less where one sequence is much the shorter
+      if ((rc = divide(false))) return rc;
+      matrix();
     }
-  }
-  std::vector<int32_t> torder, all;
-  longest_first(key, torder);
-  std::vector<int64_t> task_word;
-  int64_t total = 0;
-  for (int32_t q : torder) {
-    const Task t = tasks[q];
-    const AffDiagClass c = kDiagClasses[t.cls];
-    task_word.push_back(aff_diag_task(total, c));
-    if (want_align) total += aff_diag_words(c.width, hwd[(size_t)n + slots[t.cls][t.at]]);
-    for (int g = 0; g < kDiagTask; ++g) {
-      const bool in = g < 32 / c.lanes && t.at + g < (int)slots[t.cls].size();
-      all.push_back(in ? slots[t.cls][t.at + g] : -1);
-    }
-  }
-  const int diag = (int)all.size(), rows = (int)rows_of.size();
-  all.insert(all.end(), rows_of.begin(), rows_of.end());
-  int maxwd = 1;
-  std::vector<int64_t> off, hw;
-  if (rows) {
-    hw.resize((size_t)n);
-    CKA(cudaMemcpyAsync(hw.data(), dmw, sizeof(int64_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
-    CKA(cudaStreamSynchronize(st));
-    off.assign((size_t)n, 0);
-    for (int32_t id : rows_of) {
-      off[id] = total;
-      if (want_align) total += hw[id];
-      maxwd = std::max(maxwd, hwd[id] & ~kAffFits);
-    }
+    if (!dm) return fail(POYD_ENOMEM, "affine direction matrix allocation failed");
   }
   // device lists: the order, then (8-byte aligned) the tasks' offsets
   const size_t list = (all.size() + 1) & ~(size_t)1;
@@ -1062,11 +1083,6 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   if (diag)
     CKA(cudaMemcpyAsync(dtask, task_word.data(), 8 * task_word.size(), cudaMemcpyHostToDevice, st));
   CKA(cudaMemsetAsync(counter, 0, 64, st));
-  uint32_t *dm = nullptr;
-  if (want_align) {
-    dm = (uint32_t *)ws_buffer(w, WS_DM, sizeof(uint32_t) * (size_t)std::max<int64_t>(total, 1));
-    if (!dm) return fail(POYD_ENOMEM, "affine direction matrix allocation failed");
-  }
   const char *name = want_align ? "aff_dp_dm" : "aff_dp_cost";
   AffDiagArgs GA = {};
   GA.seq = seq; GA.plans = plans; GA.order = dord; GA.tables = tabs; GA.go = cm->gap_open;
