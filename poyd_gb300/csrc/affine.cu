@@ -992,62 +992,75 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   if (herr & 2) return fail(POYD_ERANGE, "affine costs could reach the HIGH_NUM sentinel range");
   if (herr & 4) return fail(POYD_EINVAL, "sequence codes must be below 32 (5-bit element masks)");
 
-  // Longest first; the pairs whose values fit go to k_aff_diag (affine_diag.cu)
-  // in tasks of one class (lanes x diagonals a lane), longest task first; the
-  // others run in rows.
-  std::vector<int64_t> key((size_t)n);
-  for (int32_t t = 0; t < n; ++t) key[t] = (int64_t)hwd[(size_t)n + t] << 7;  // longest_first's unit
+  // The pairs whose values fit go to k_aff_diag (affine_diag.cu) in tasks of one
+  // class (lanes x diagonals a lane), the longest task first; the others run in
+  // rows, longest first.  One counting sort by class and steps (as fine as the batch
+  // is large) and a merge of the classes' tasks: the costs of 200,000 pairs of 5
+  // elements take 1.8 ms, 3.4 with two radix sorts and a list for each class.
   int dev = 0, sms = 1;
   CKA(cudaGetDevice(&dev));
   CKA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const bool spread = want_align && n <= kDiagSpreadPerSm * sms;
-  std::vector<int32_t> order, all;  // all: the tasks' pairs, then the rows kernels'
-  longest_first(key, order);
+  const int32_t *steps = hwd.data() + n;
+  const int most = *std::max_element(steps, steps + n);
+  int shift = 0;
+  while (most >> shift >= std::max(256, n)) ++shift;
+  const int bins = (most >> shift) + 1;  // of a class, longest first
+  constexpr int kWidest = 512;           // diagonals of the widest class
+  int8_t class_of[kWidest + 1];
+  for (int wd = 0; wd <= kWidest; ++wd) class_of[wd] = (int8_t)aff_diag_class(wd - 41, spread);
+  std::vector<int32_t> all;  // the tasks' pairs, then the rows kernels'
   std::vector<int64_t> task_word, off, hw;
   int diag = 0, rows = 0, maxwd = 1;
   int64_t total = 0;  // direction words
   auto divide = [&](bool by_diag) -> int {
-    std::vector<int32_t> rows_of, slots[kDiagClassN], torder;
-    for (int32_t id : order) {
-      const int c = by_diag && (hwd[id] & kAffFits) ? aff_diag_class((hwd[id] & ~kAffFits) - 41, spread)
-                                                    : kDiagClassN;
-      if (c == kDiagClassN) rows_of.push_back(id);
-      else slots[c].push_back(id);
-    }
-    struct Task {
-      int cls, at;  // the class and the first of its pairs in slots[cls]
+    auto bin_of = [&](int32_t id) {
+      const int wd = hwd[id] & ~kAffFits;
+      const int c = by_diag && (hwd[id] & kAffFits) && wd <= kWidest ? class_of[wd] : kDiagClassN;
+      return c * bins + ((most - steps[id]) >> shift);
     };
-    std::vector<Task> tasks;
-    key.clear();
+    std::vector<int32_t> first((size_t)(kDiagClassN + 1) * bins + 1, 0), sorted((size_t)n);
+    for (int32_t id = 0; id < n; ++id) ++first[bin_of(id) + 1];
+    int32_t at[kDiagClassN + 2];  // the first pair of each class in `sorted`
+    for (size_t b = 1; b < first.size(); ++b) first[b] += first[b - 1];
+    for (int c = 0; c <= kDiagClassN + 1; ++c) at[c] = first[(size_t)c * bins];
+    for (int32_t id = 0; id < n; ++id) sorted[first[bin_of(id)]++] = id;
+
+    int32_t next[kDiagClassN], tasks = 0;  // the classes' next tasks
+    int64_t work[kDiagClassN];
+    auto steps_at = [&](int c, int32_t p) { return (int64_t)steps[sorted[p]] * kDiagClasses[c].width; };
     for (int c = 0; c < kDiagClassN; ++c) {
       const int per = 32 / kDiagClasses[c].lanes;
-      for (int at = 0; at < (int)slots[c].size(); at += per) {
-        tasks.push_back({c, at});
-        key.push_back((int64_t)hwd[(size_t)n + slots[c][at]] * kDiagClasses[c].width << 3);
-      }
+      tasks += (at[c + 1] - at[c] + per - 1) / per;
+      next[c] = at[c];
+      work[c] = at[c] < at[c + 1] ? steps_at(c, at[c]) : -1;
     }
-    longest_first(key, torder);
-    task_word.clear();
-    all.clear();
+    diag = kDiagTask * tasks, rows = at[kDiagClassN + 1] - at[kDiagClassN];
+    all.assign((size_t)diag + rows, -1);
+    task_word.resize((size_t)tasks);
     total = 0;
-    for (int32_t q : torder) {
-      const Task t = tasks[q];
-      const AffDiagClass c = kDiagClasses[t.cls];
-      task_word.push_back(aff_diag_task(total, c));
-      if (want_align) total += aff_diag_words(c.width, hwd[(size_t)n + slots[t.cls][t.at]]);
-      for (int g = 0; g < kDiagTask; ++g) {
-        const bool in = g < 32 / c.lanes && t.at + g < (int)slots[t.cls].size();
-        all.push_back(in ? slots[t.cls][t.at + g] : -1);
+    for (int32_t t = 0; t < tasks; ++t) {
+      const int c = (int)(std::max_element(work, work + kDiagClassN) - work);
+      const int m = std::min(32 / kDiagClasses[c].lanes, at[c + 1] - next[c]);
+      int longest = 0;
+      for (int g = 0; g < m; ++g) {
+        const int32_t id = sorted[next[c] + g];
+        all[(size_t)kDiagTask * t + g] = id;
+        longest = std::max(longest, steps[id]);
       }
+      task_word[t] = aff_diag_task(total, kDiagClasses[c]);
+      if (want_align) total += aff_diag_words(kDiagClasses[c].width, longest);
+      next[c] += m;
+      work[c] = next[c] < at[c + 1] ? steps_at(c, next[c]) : -1;
     }
-    diag = (int)all.size(), rows = (int)rows_of.size();
-    all.insert(all.end(), rows_of.begin(), rows_of.end());
+    std::copy(sorted.begin() + at[kDiagClassN], sorted.end(), all.begin() + diag);
     if (rows) {
       hw.resize((size_t)n);
       CKA(cudaMemcpyAsync(hw.data(), dmw, sizeof(int64_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
       CKA(cudaStreamSynchronize(st));
       off.assign((size_t)n, 0);
-      for (int32_t id : rows_of) {
+      for (size_t p = diag; p < all.size(); ++p) {
+        const int32_t id = all[p];
         off[id] = total;
         if (want_align) total += hw[id];
         maxwd = std::max(maxwd, hwd[id] & ~kAffFits);
