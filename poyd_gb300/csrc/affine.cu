@@ -26,7 +26,6 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
-#include <numeric>
 #include <vector>
 #include "affine_diag.cuh"
 #include "affine_kernels.cuh"
@@ -68,13 +67,24 @@ struct AffPlanArgs {
   int scale, go;     // k_aff_diag's value scale (0: its 16 bits are out of the question)
   int maxsub, maxext;  // largest substitution and extension cost
   AffPlan *plans;
-  int64_t *dm_words;
-  int32_t *wd_out;   // band width; kAffFits when k_aff_diag's values fit
-  int32_t *steps;    // leni + lenj
+  int32_t *rows_out;  // leni; kAffFits when k_aff_diag's values fit
+  int32_t *cols_out;  // lenj
   int64_t *cells;
   int32_t *err;
 };
 constexpr int32_t kAffFits = 1 << 30;
+
+// Band of the pair: columns up to e0 past a row's own, kStart before it.
+__host__ __device__ inline int aff_e0(int leni, int lenj) {
+  const int e0 = lenj - leni + 8;
+  const int least = e0 < 40 ? 40 : e0;
+  return least < lenj ? least : lenj;
+}
+// The rows kernels' strips and the 4-step direction words of one.
+__host__ __device__ inline int aff_strips(int leni) { return (leni + kAffRows) / kAffRows; }
+__host__ __device__ inline int aff_strip_words(int wd) {
+  return (wd + 2 * (kAffRows - 1) + 15) / 16 * 4;  // whole 16-step half blocks
+}
 
 struct AffDpArgs {
   int n;
@@ -117,19 +127,15 @@ __global__ void __launch_bounds__(128) k_aff_plan(AffPlanArgs A) {
   const int swap = la > lb;  // rows = shorter (algn.c:2595-2617)
   const int li = swap ? lb : la, lj = swap ? la : lb;
   const int leni = li - 1, lenj = lj - 1;
-  int e0 = (lenj - leni) + 8;
-  if (e0 < 40) e0 = 40;
-  if (e0 > lenj) e0 = lenj;
+  const int e0 = aff_e0(leni, lenj);
   AffPlan P;
   P.si_off = swap ? bo : ao;
   P.sj_off = swap ? ao : bo;
   P.leni = leni; P.lenj = lenj; P.e0 = e0;
   P.wd = e0 - kDlo + 1;
   P.swap = swap;
-  P.nstrips = (leni + 1 + kAffRows - 1) / kAffRows;
-  const int S = P.wd + 2 * (kAffRows - 1);
-  const int Spad = (S + 15) / 16 * 16;  // whole 16-step half blocks
-  P.sblocks = Spad / 4;
+  P.nstrips = aff_strips(leni);
+  P.sblocks = aff_strip_words(P.wd);
   P.empty = 0;
   // codes: any above 31 (they index 32-entry table rows), gap-bearing ones past
   // position 0, all gaps
@@ -164,15 +170,14 @@ __global__ void __launch_bounds__(128) k_aff_plan(AffPlanArgs A) {
   if (lane != 0) return;
   for (int t = 0; t < 4; ++t) P.pad_[t] = 0;
   A.plans[id] = P;
-  A.dm_words[id] = (int64_t)P.nstrips * P.sblocks * kAffRows;
-  A.steps[id] = leni + lenj;
+  A.cols_out[id] = lenj;
   // k_aff_diag: a cell's value is at most that of the diagonal path and one gap
   // to it (and a state's, one more opening and step); infinities grow by at
   // most a band of extensions outside the matrix
   const long long ext = A.maxext + A.go + 1LL, step = A.maxsub + 2 * ext;
   const long long most = A.scale * ((long long)leni * A.maxsub + P.wd * ext + 4 * step);
   const bool fits = A.scale && most < 0xC000 && A.scale * (ext * (P.wd + 8) + 4 * step) < 0x3000;
-  A.wd_out[id] = P.wd | (fits ? kAffFits : 0);
+  A.rows_out[id] = leni | (fits ? kAffFits : 0);
   if (A.cells) A.cells[id] = cells + lenj + 1;
   int err = 0;
   if (la < 1 || lb < 1) err |= 1;
@@ -946,10 +951,9 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   int rc = upload_tables_ws(w, cm, &tabs, st);
   if (rc) return rc;
   AffPlan *plans = (AffPlan *)ws_buffer(w, WS_AFF, sizeof(AffPlan) * (size_t)n);
-  int64_t *dmw = (int64_t *)ws_buffer(w, WS_DMWORDS, sizeof(int64_t) * 2 * (size_t)n);
-  // band widths, steps and the error word, read back together
+  // rows, columns and the error word, read back together
   int32_t *wdb = (int32_t *)ws_buffer(w, WS_WD, sizeof(int32_t) * (2 * (size_t)n + 1) + 16);
-  if (!plans || !dmw || !wdb) return fail(POYD_ENOMEM, "plan allocation failed");
+  if (!plans || !wdb) return fail(POYD_ENOMEM, "plan allocation failed");
   int32_t *err = wdb + 2 * (size_t)n;
   CKA(cudaMemsetAsync(err, 0, 4, st));
   // The packed kernels run when one step's largest add stays far below their
@@ -977,17 +981,17 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   PA.scale = packed && !negative ? (want_align ? 4 : 1) : 0;
   PA.maxsub = maxsub; PA.maxext = maxext;
   PA.go = cm->gap_open;
-  PA.plans = plans; PA.dm_words = dmw; PA.wd_out = wdb; PA.steps = wdb + n; PA.cells = cells;
+  PA.plans = plans; PA.rows_out = wdb; PA.cols_out = wdb + n; PA.cells = cells;
   PA.err = err;
   {
     ProfScope ps("aff_plan", st);
     k_aff_plan<<<(unsigned)(((int64_t)n + 3) / 4), 128, 0, st>>>(PA);
   }
   CKA(cudaGetLastError());
-  std::vector<int32_t> hwd(2 * (size_t)n + 1);
-  CKA(cudaMemcpyAsync(hwd.data(), wdb, sizeof(int32_t) * hwd.size(), cudaMemcpyDeviceToHost, st));
+  std::vector<int32_t> hd(2 * (size_t)n + 1);
+  CKA(cudaMemcpyAsync(hd.data(), wdb, sizeof(int32_t) * hd.size(), cudaMemcpyDeviceToHost, st));
   CKA(cudaStreamSynchronize(st));
-  const int herr = hwd[2 * (size_t)n];
+  const int herr = hd[2 * (size_t)n];
   if (herr & 1) return fail(POYD_EINVAL, "sequences must have length >= 1 (the leading gap)");
   if (herr & 2) return fail(POYD_ERANGE, "affine costs could reach the HIGH_NUM sentinel range");
   if (herr & 4) return fail(POYD_EINVAL, "sequence codes must be below 32 (5-bit element masks)");
@@ -1001,39 +1005,78 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   CKA(cudaGetDevice(&dev));
   CKA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const bool spread = want_align && n <= kDiagSpreadPerSm * sms;
-  const int32_t *steps = hwd.data() + n;
-  const int most = *std::max_element(steps, steps + n);
+  const int32_t *rows_f = hd.data(), *cols = hd.data() + n;
+  auto leni_of = [&](int32_t id) { return rows_f[id] & ~kAffFits; };
+  auto steps_of = [&](int32_t id) { return leni_of(id) + cols[id]; };
+  int most = 0;
+  for (int32_t id = 0; id < n; ++id) most = std::max(most, steps_of(id));
   int shift = 0;
   while (most >> shift >= std::max(256, n)) ++shift;
   const int bins = (most >> shift) + 1;  // of a class, longest first
   constexpr int kWidest = 512;           // diagonals of the widest class
-  int8_t class_of[kWidest + 1];
-  for (int wd = 0; wd <= kWidest; ++wd) class_of[wd] = (int8_t)aff_diag_class(wd - 41, spread);
+  struct {
+    int32_t bin, slots, words;  // the class's first bin, its diagonals; a strip's direction words
+  } of[kWidest + 1];
+  for (int wd = 0; wd <= kWidest; ++wd) {
+    const int c = aff_diag_class(wd - 41, spread);
+    of[wd] = {c * bins, c < kDiagClassN ? kDiagClasses[c].lanes * kDiagClasses[c].width : 0, aff_strip_words(wd)};
+  }
+  const int32_t in_rows = kDiagClassN * bins;
+  // Pairs of few rows and many columns may be better off in rows: the rows kernels
+  // step along each strip's band, k_aff_diag along both sequences (r against d for
+  // a pair's share of a warp; less only where the band is wider than its least).
+  // They are once there are enough of them, for the rows kernels' own latency, which
+  // comes after k_aff_diag's batch, is the longer.  In microseconds: a step of the
+  // longest 0.4, of all the others 1.5e-5 and (k_aff_diag) 2.5e-5 each.  Costs of
+  // 16,384 pairs of 10 and 440 elements 0.67 ms in rows, 1.25 by antidiagonals; of 20
+  // and 300 0.71 and 0.86, of 20 and 200 0.59 and 0.44; of 5,200 of 10 and 440 0.54
+  // and 0.54; of 40,000 of 50 and 300 2.08 and 1.98.
+  std::vector<int32_t> bin((size_t)n);
+  int64_t r_all = 0, d_all = 0, r_most = 0;
+  auto uneven = [&](int32_t id, int wd, int64_t *r, int64_t *d) {
+    *r = (int64_t)aff_strips(leni_of(id)) * of[wd].words * 4;
+    *d = (int64_t)of[wd].slots * steps_of(id) / 64;
+    return *r < *d;
+  };
+  for (int32_t id = 0; id < n; ++id) {
+    const int wd = aff_e0(leni_of(id), cols[id]) - kDlo + 1;
+    const int at = (most - steps_of(id)) >> shift;
+    bin[id] = at + ((rows_f[id] & kAffFits) && wd <= kWidest ? of[wd].bin : in_rows);
+    int64_t r, d;
+    if (wd > 81 && bin[id] < in_rows && uneven(id, wd, &r, &d))
+      r_all += r, d_all += d, r_most = std::max(r_most, r);
+  }
+  if (2.5e-5 * (double)d_all - 1.5e-5 * (double)r_all > 0.4 * (double)r_most)
+    for (int32_t id = 0; id < n; ++id) {
+      const int wd = aff_e0(leni_of(id), cols[id]) - kDlo + 1;
+      int64_t r, d;
+      if (wd > 81 && bin[id] < in_rows && uneven(id, wd, &r, &d)) bin[id] = bin[id] % bins + in_rows;
+    }
   std::vector<int32_t> all;  // the tasks' pairs, then the rows kernels'
-  std::vector<int64_t> task_word, off, hw;
+  std::vector<int64_t> task_word, off;
   int diag = 0, rows = 0, maxwd = 1;
   int64_t total = 0;  // direction words
-  auto divide = [&](bool by_diag) -> int {
-    auto bin_of = [&](int32_t id) {
-      const int wd = hwd[id] & ~kAffFits;
-      const int c = by_diag && (hwd[id] & kAffFits) && wd <= kWidest ? class_of[wd] : kDiagClassN;
-      return c * bins + ((most - steps[id]) >> shift);
-    };
+  auto divide = [&](bool by_diag) -> void {
+    if (!by_diag)
+      for (int32_t id = 0; id < n; ++id) bin[id] = bin[id] % bins + in_rows;
     std::vector<int32_t> first((size_t)(kDiagClassN + 1) * bins + 1, 0), sorted((size_t)n);
-    for (int32_t id = 0; id < n; ++id) ++first[bin_of(id) + 1];
+    for (int32_t id = 0; id < n; ++id) ++first[bin[id] + 1];
     int32_t at[kDiagClassN + 2];  // the first pair of each class in `sorted`
     for (size_t b = 1; b < first.size(); ++b) first[b] += first[b - 1];
     for (int c = 0; c <= kDiagClassN + 1; ++c) at[c] = first[(size_t)c * bins];
-    for (int32_t id = 0; id < n; ++id) sorted[first[bin_of(id)]++] = id;
+    for (int32_t id = 0; id < n; ++id) sorted[first[bin[id]]++] = id;
 
     int32_t next[kDiagClassN], tasks = 0;  // the classes' next tasks
     int64_t work[kDiagClassN];
-    auto steps_at = [&](int c, int32_t p) { return (int64_t)steps[sorted[p]] * kDiagClasses[c].width; };
+    auto steps_at = [&](int32_t p) { return steps_of(sorted[p]); };
+    auto work_at = [&](int c) {
+      return next[c] < at[c + 1] ? (int64_t)steps_at(next[c]) * kDiagClasses[c].width : -1;
+    };
     for (int c = 0; c < kDiagClassN; ++c) {
       const int per = 32 / kDiagClasses[c].lanes;
       tasks += (at[c + 1] - at[c] + per - 1) / per;
       next[c] = at[c];
-      work[c] = at[c] < at[c + 1] ? steps_at(c, at[c]) : -1;
+      work[c] = work_at(c);
     }
     diag = kDiagTask * tasks, rows = at[kDiagClassN + 1] - at[kDiagClassN];
     all.assign((size_t)diag + rows, -1);
@@ -1044,31 +1087,25 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
       const int m = std::min(32 / kDiagClasses[c].lanes, at[c + 1] - next[c]);
       int longest = 0;
       for (int g = 0; g < m; ++g) {
-        const int32_t id = sorted[next[c] + g];
-        all[(size_t)kDiagTask * t + g] = id;
-        longest = std::max(longest, steps[id]);
+        all[(size_t)kDiagTask * t + g] = sorted[next[c] + g];
+        longest = std::max(longest, steps_at(next[c] + g));
       }
       task_word[t] = aff_diag_task(total, kDiagClasses[c]);
       if (want_align) total += aff_diag_words(kDiagClasses[c].width, longest);
       next[c] += m;
-      work[c] = next[c] < at[c + 1] ? steps_at(c, next[c]) : -1;
+      work[c] = work_at(c);
     }
     std::copy(sorted.begin() + at[kDiagClassN], sorted.end(), all.begin() + diag);
-    if (rows) {
-      hw.resize((size_t)n);
-      CKA(cudaMemcpyAsync(hw.data(), dmw, sizeof(int64_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
-      CKA(cudaStreamSynchronize(st));
-      off.assign((size_t)n, 0);
-      for (size_t p = diag; p < all.size(); ++p) {
-        const int32_t id = all[p];
-        off[id] = total;
-        if (want_align) total += hw[id];
-        maxwd = std::max(maxwd, hwd[id] & ~kAffFits);
-      }
+    if (rows && want_align) off.assign((size_t)n, 0);
+    for (size_t p = diag; p < all.size(); ++p) {
+      const int32_t id = all[p], wd = aff_e0(leni_of(id), cols[id]) - kDlo + 1;
+      maxwd = std::max(maxwd, wd);
+      if (!want_align) continue;
+      off[id] = total;
+      total += (int64_t)aff_strips(leni_of(id)) * aff_strip_words(wd) * kAffRows;
     }
-    return POYD_OK;
   };
-  if ((rc = divide(true))) return rc;
+  divide(true);
   uint32_t *dm = nullptr;
   if (want_align) {
     auto matrix = [&]() {
@@ -1078,14 +1115,13 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
     if (!dm && diag) {
       // k_aff_diag's matrix holds a band for each step of both sequences, the rows
       // kernels' one for each row: far less where one sequence is much the shorter
-      if ((rc = divide(false))) return rc;
+      divide(false);
       matrix();
     }
     if (!dm) return fail(POYD_ENOMEM, "affine direction matrix allocation failed");
   }
   // device lists: the order, then (8-byte aligned) the tasks' offsets
   const size_t list = (all.size() + 1) & ~(size_t)1;
-  int64_t *doff = dmw + n;
   int32_t *dord = (int32_t *)ws_buffer(w, WS_ORDER, 4 * list + 8 * task_word.size() + 16);
   int *counter = (int *)ws_buffer(w, WS_COUNTER, 64);
   AffWhere *where = want_align ? (AffWhere *)ws_buffer(w, WS_CELLS, sizeof(AffWhere) * (size_t)n) : nullptr;
@@ -1118,7 +1154,12 @@ int affine_batch(const poyd_cm *cm, int maxc, int32_t n, const uint8_t *seq,
   // The rows kernels, two pairs per lane group in 16-bit halves or (large
   // costs) one in 32 bits; a pair whose final cost is past the packed exact
   // range sends its batch to the 32-bit kernel afterwards.
-  CKA(cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, st));
+  int64_t *doff = nullptr;
+  if (want_align) {
+    doff = (int64_t *)ws_buffer(w, WS_DMWORDS, sizeof(int64_t) * (size_t)n);
+    if (!doff) return fail(POYD_ENOMEM, "order allocation failed");
+    CKA(cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, st));
+  }
   for (int attempt = 0; attempt < 2; ++attempt) {
     const int blocks = aff_blocks(want_align, packed);
     const int64_t slab = maxwd + 8;
