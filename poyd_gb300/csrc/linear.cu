@@ -719,52 +719,104 @@ __global__ void __launch_bounds__(kDpWarps * 32, 3) k_lin_dp(LinDpArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// Packing of batched align_2 results: a block per pair copies the used tail of
-// each of its four right-aligned slots back to back, 16 bytes a store.  A
-// store's source starts anywhere in a word: its five aligned words are
-// shifted together (only words that hold some of its bytes are read).
+// Packing of batched align_2 results: the used tail of each of a pair's four
+// right-aligned slots back to back, 16 bytes a store.  A store's source starts
+// anywhere in a word: its five aligned words are shifted together (only words that
+// hold some of its bytes are read).  A block takes a pair, or in large batches four:
+// a warp each, then the block together those longer than kPackWarpMost.
+// A warp copies short sequences by bytes, all loads before the stores.
 // Measured: 65,536 pairs of 100-5,000 bp (670 MB) took 785 us with a warp per
-// pair copying bytes; one pair of 1,000 bp 25 us.
+// pair copying bytes; one pair of 1,000 bp 25 us, 8 with a block.  200,000 pairs of 5,
+// 100 and 300 elements 39, 121 and 265 us with a warp each copying bytes, 204, 278
+// and 300 with a block each, 56, 80 and 209 now.
 // ---------------------------------------------------------------------------
-constexpr int kPackThreads = 128;
-__device__ __forceinline__ void pack_copy(uint8_t *d, const uint8_t *s, int64_t len) {
+constexpr int kPackThreads = 128, kPackWarpMost = 16384, kPackBytes = 4;
+// t: of T threads
+template <int T>
+__device__ __forceinline__ void pack_copy(uint8_t *d, const uint8_t *s, int64_t len, int t) {
   const int64_t head = min(len, (int64_t)(-(intptr_t)d & 15));
-  if (threadIdx.x < head) d[threadIdx.x] = s[threadIdx.x];
+  if (t < head) d[t] = s[t];
   d += head, s += head, len -= head;
   const int64_t full = len >> 4;
   const uint32_t *w = reinterpret_cast<const uint32_t *>((uintptr_t)s & ~(uintptr_t)3);
   const unsigned sh = 8u * (unsigned)((uintptr_t)s & 3);
-  for (int64_t x = threadIdx.x; x < full; x += kPackThreads) {
+#pragma unroll 2
+  for (int64_t x = t; x < full; x += T) {
     const uint32_t *p = w + 4 * x;
     const uint32_t a = p[0], b = p[1], c = p[2], e = p[3], f = sh ? p[4] : 0u;
     reinterpret_cast<uint4 *>(d)[x] =
         make_uint4(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh), __funnelshift_r(c, e, sh),
                    __funnelshift_r(e, f, sh));
   }
-  const int64_t at = (full << 4) + threadIdx.x;
-  if (threadIdx.x < 16 && at < len) d[at] = s[at];
+  const int64_t at = (full << 4) + t;
+  if (t < 16 && at < len) d[at] = s[at];
 }
 
-// cap: every slot's sequence capacity, or null: from the pair's lengths
-__global__ void __launch_bounds__(kPackThreads, 12) k_pack_alignments(
-    const uint8_t *out, const int64_t *out_off, const int32_t *a_len, const int32_t *b_len,
-    const int64_t *caps, const int32_t *out_len, uint8_t *packed, const int64_t *packed_off) {
-  const int64_t id = blockIdx.x;
-  const int64_t cap = caps ? caps[id] : slot_cap(a_len[id], b_len[id]);
-  const int64_t na = out_len[2 * id], nm = out_len[2 * id + 1];
-  const uint8_t *src = out + out_off[id];
-  uint8_t *dst = packed + packed_off[id];
+struct PackArgs {
+  int n;
+  const uint8_t *out;
+  const int64_t *out_off;
+  const int32_t *a_len, *b_len;
+  const int64_t *caps;  // every slot's sequence capacity, or null: from the pair's lengths
+  const int32_t *out_len;
+  uint8_t *packed;
+  const int64_t *packed_off;
+};
+template <int T>
+__device__ __forceinline__ void pack_pair(const PackArgs &A, int64_t id, int64_t na, int64_t nm, int t) {
+  const int64_t cap = A.caps ? A.caps[id] : slot_cap(A.a_len[id], A.b_len[id]);
+  const uint8_t *src = A.out + A.out_off[id];
+  uint8_t *dst = A.packed + A.packed_off[id];
+  if (T == 32 && max(na, nm) <= 32 * kPackBytes) {  // bytes, all loads before the stores
+    uint8_t v[4][kPackBytes];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int h = 0; h < kPackBytes; ++h) {
+        const int len = (int)(k < 3 ? na : nm), x = t + 32 * h;
+        v[k][h] = x < len ? src[(k + 1) * cap - len + x] : 0;
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int h = 0; h < kPackBytes; ++h)
+        if (t + 32 * h < (k < 3 ? na : nm)) dst[k * na + t + 32 * h] = v[k][h];
+    return;
+  }
 #pragma unroll 1
-  for (int k = 0; k < 3; ++k) pack_copy(dst + k * na, src + (k + 1) * cap - na, na);
-  pack_copy(dst + 3 * na, src + 4 * cap - nm, nm);
+  for (int k = 0; k < 3; ++k) pack_copy<T>(dst + k * na, src + (k + 1) * cap - na, na, t);
+  pack_copy<T>(dst + 3 * na, src + 4 * cap - nm, nm, t);
+}
+
+template <int PAIRS>  // of a block: 1 or its warps
+__global__ void __launch_bounds__(kPackThreads, 12) k_pack_alignments(const __grid_constant__ PackArgs A) {
+  if (PAIRS == 1) {
+    const int64_t id = blockIdx.x;
+    pack_pair<kPackThreads>(A, id, A.out_len[2 * id], A.out_len[2 * id + 1], threadIdx.x);
+    return;
+  }
+  static_assert(PAIRS == 1 || PAIRS == kPackThreads / 32, "a warp a pair");
+  const int64_t first = (int64_t)blockIdx.x * PAIRS, mine = first + (threadIdx.x >> 5);
+  if (mine < A.n) {
+    const int32_t na = A.out_len[2 * mine], nm = A.out_len[2 * mine + 1];
+    if (max(na, nm) <= kPackWarpMost) pack_pair<32>(A, mine, na, nm, threadIdx.x & 31);
+  }
+#pragma unroll 1
+  for (int64_t id = first; id < min(first + PAIRS, (int64_t)A.n); ++id) {
+    const int32_t na = A.out_len[2 * id], nm = A.out_len[2 * id + 1];
+    if (max(na, nm) > kPackWarpMost) pack_pair<kPackThreads>(A, id, na, nm, threadIdx.x);
+  }
 }
 
 void launch_pack_alignments(int n, const uint8_t *out, const int64_t *out_off,
                             const int32_t *a_len, const int32_t *b_len, const int64_t *caps,
                             const int32_t *out_len, uint8_t *packed,
                             const int64_t *packed_off, cudaStream_t st) {
-  k_pack_alignments<<<(unsigned)n, kPackThreads, 0, st>>>(out, out_off, a_len, b_len, caps,
-                                                          out_len, packed, packed_off);
+  const PackArgs A = {n, out, out_off, a_len, b_len, caps, out_len, packed, packed_off};
+  constexpr int kPairs = kPackThreads / 32;
+  // four pairs a block where that still makes some blocks for each SM
+  if (n > 4096) k_pack_alignments<kPairs><<<(unsigned)((n - 1) / kPairs + 1), kPackThreads, 0, st>>>(A);
+  else k_pack_alignments<1><<<(unsigned)n, kPackThreads, 0, st>>>(A);
 }
 
 // ---------------------------------------------------------------------------
