@@ -40,10 +40,14 @@ __device__ __forceinline__ uint32_t nzbits(uint32_t x) {
   return (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
 }
 
-// A lane's vectors are read four at a time and counted with one population count
-// each (a quarter-rate operation: one a word, and a read a round, took 60 us and not 51
-// for 154,296 pairs of 2,000 characters whose rows lie in L2).
-__global__ void k_fitch_distance(const uint8_t *nodes, int64_t stride, int len, int n,
+// A lane's vectors are read kBatch at a time (all of a row's, at most four) and
+// counted with one population count each (a quarter-rate operation: one a word, and
+// a read a round, took 60 us and not 51 for 154,296 pairs of 2,000 characters whose
+// rows lie in L2).  Rows of up to 512 characters, one vector a lane, are bound by
+// their latency and the warps on an SM: 100,000 pairs of 100 characters 16.5 us, 22.6
+// with room for four vectors a lane.  Of 800 characters 20.6 and 24.7.
+template <int kBatch>
+__global__ void __launch_bounds__(256) k_fitch_distance(const uint8_t *nodes, int64_t stride, int len, int n,
                                  const int32_t *ai, const int32_t *bi, int64_t *dist) {
   const int lane = threadIdx.x & 31;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -51,7 +55,6 @@ __global__ void k_fitch_distance(const uint8_t *nodes, int64_t stride, int len, 
   const uint4 *a = (const uint4 *)(nodes + (int64_t)ai[c] * stride);
   const uint4 *b = (const uint4 *)(nodes + (int64_t)bi[c] * stride);
   const int nv = (len + 15) >> 4;
-  constexpr int kBatch = 4;
   int cnt = 0;
   for (int base = 0; base < nv; base += 32 * kBatch) {
     uint4 x[kBatch], y[kBatch];
@@ -446,8 +449,11 @@ extern "C" int poyd_nonadd8_distance_batch(const uint8_t *nodes, int64_t stride,
   if (!a_idx || !b_idx || !dist) return fail(POYD_EINVAL, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope ps("fitch_distance", st);
-  k_fitch_distance<<<(unsigned)(((int64_t)n * 32 + 255) / 256), 256, 0, st>>>(
-      nodes, stride, len, n, a_idx, b_idx, dist);
+  const unsigned blocks = (unsigned)(((int64_t)n * 32 + 255) / 256);
+  const int per_lane = (len + 511) / 512;  // vectors
+  auto kern = per_lane <= 1 ? k_fitch_distance<1> : per_lane == 2 ? k_fitch_distance<2>
+              : per_lane == 3 ? k_fitch_distance<3> : k_fitch_distance<4>;
+  kern<<<blocks, 256, 0, st>>>(nodes, stride, len, n, a_idx, b_idx, dist);
   FS_CK(cudaGetLastError());
   return POYD_OK;
 }
