@@ -227,6 +227,17 @@ static int sm_count() {
 }
 
 constexpr int kTeamPairsPerSm = 3;
+// More than two pairs an SM run in two rounds of blocks with 16 diagonals a lane (512
+// in all) and in three with 32 (1,024), which pays while the band fills them.  Costs
+// of 456 pairs of 2,000 bp (band 302) 396 us and 326 with a warp per pair, of 3,000
+// (402) 576 and 561, of 3,500 (452) 667 and 717, of 310 pairs of 2,500 (352) 417 and
+// 450; 456 of 5,000 (602) 1,317 and 1,225, of 6,000 (702) 1,575 and 1,688; 400
+// alignments of 3,000-3,500 with a band of up to 560 1.33 and 1.26 ms, 456 of 5,000
+// 1.90 and 1.97.
+static int team_least_band(int width, bool align, int n) {
+  if (width == 32) return align ? 590 : 672;
+  return align ? 0 : 340 + 90 * (n - 2 * sm_count()) / sm_count();
+}
 // k_lin_diag's batches start where its throughput pays: below, a lone warp's steps
 // take longer than k_lin_dp4's.  Costs of 1,500 bp: 700 pairs 408 and 356 us,
 // 1,300 pairs 410 and 470; alignments of 100-1,500 bp: 1,300 pairs 849 and 796 us,
@@ -432,6 +443,7 @@ static int linear_batch(Workspace *w, const poyd_cm *cm, int maxc, int32_t n, co
   int team = packed && path && small && !host_waves && var.packed < 0 && var.blocks_per_sm == 0 &&
                      var.solo < 0 && n <= kTeamPairsPerSm * sm_count()
                  ? lin_team_width(maxwd, tl.maxsum) : 0;
+  if (team > 8 && n > 2 * sm_count() && maxwd < team_least_band(team, want_align, n)) team = 0;
   const int64_t team_words = team && want_align ? lin_team_words(team, tl.maxsum) : 0;
   // One allocation, of what the kernel at hand needs: a buffer that grows waits for
   // the device, other streams' work included.
