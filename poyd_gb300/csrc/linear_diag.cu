@@ -708,10 +708,11 @@ int diag_blocks() {
 }  // namespace
 
 // Fewer lanes a pair waste less of the band's width and of a double step's fixed
-// part; more, while warps would idle.
+// part; more, while warps would idle.  (Alignments come here from more pairs than
+// warps on: theirs take 32 lanes for bands that 16 do not hold alone.)
 int lin_diag_min_lanes(int n, int sms, bool bt) {
   const int warps = sms * (bt ? diag_warps<true>() : diag_warps<false>());
-  return n <= warps ? 32 : n <= 2 * warps ? 16 : 8;
+  return !bt && n <= warps ? 32 : n <= 2 * warps ? 16 : 8;
 }
 
 void launch_lin_diag_order(int n, int min_lanes, bool bt, const LinPlan *plans,
