@@ -89,7 +89,7 @@ size_t ws_size(const Workspace *w, int slot);  // bytes it holds now
 std::mutex &ws_layout_mutex(Workspace *w);     // held from a layout's launch to its read-back
 enum WsSlot {
   WS_TABLES = 0, WS_PLANS, WS_DMWORDS, WS_WD, WS_ORDER, WS_DM, WS_SCRATCH,
-  WS_COUNTER, WS_CELLS, WS_AFF, WS_ERR, WS_SEQ, WS_META, WS_OUT, WS_BATCH, WS_ORDSCR,
+  WS_COUNTER, WS_CELLS, WS_AFF, WS_SEQ, WS_META, WS_OUT, WS_BATCH, WS_ORDSCR,
   WS_LVL_NODES, WS_LVL_PAIRS, WS_P3_RING, WS_P3_DIR, WS_P3_META, WS_P3_IO, WS_P3_LENS,
   WS_LAYOUT, WS_NSLOTS
 };
