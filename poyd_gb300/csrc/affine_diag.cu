@@ -37,8 +37,8 @@
 //
 // Bound: integer issue (the ALU pipe 80 % busy).  Measured: 16,384 pairs of
 // 100-5,000 bp with directions 27.4 ms in k_aff_dp2 and 3.2 ms here, their
-// traceback 6.3 ms with a thread per pair and 0.8 ms with k_aff_walk; the costs
-// of 38,001 pairs of 1,000 bp with gap-bearing codes 6.5 and 2.5 ms.
+// traceback 6.3 ms with a thread per pair and 0.7 ms with k_aff_walk; the costs
+// of 38,001 pairs of 1,000 bp with gap-bearing codes 6.5 and 2.2 ms.
 #include <algorithm>
 #include <atomic>
 #include "affine_diag.cuh"

@@ -11,8 +11,8 @@
 //
 // Sankoff restates SankCS.elt_median / distance (sankCS.ml:302-377) with
 // int32 costs and the saturating infinity of sankCS.ml:34-67 mapped to
-// POYD_SANK_INF: one thread per (candidate, character), k <= 8 states,
-// tcm in shared memory.
+// POYD_SANK_INF, k <= 8 states, tcm in shared memory: medians a thread per
+// (candidate, character), distances a warp per candidate.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>

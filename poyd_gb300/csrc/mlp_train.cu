@@ -142,7 +142,8 @@ __device__ __forceinline__ void t_head_sums(const MlpBwdArgs &A, float *buf) {
 }
 
 // dZ3 = dy w4 masked, dZ2 = dZ3 W3^T masked, dZ1 = dZ2 W2^T masked, for 32
-// rows a block; the first block takes t_head_sums.
+// rows a block, whose activations are in shared memory and whose weights come from
+// L2; the first block takes t_head_sums.
 __global__ void __launch_bounds__(kTThreads) k_mlp_chain(const __grid_constant__ MlpBwdArgs A) {
   __shared__ __align__(16) __nv_bfloat16 z3[kTRows * (kTH3 + kTPad)];
   __shared__ __align__(16) __nv_bfloat16 z2[kTRows * (kTH2 + kTPad)];
