@@ -97,10 +97,17 @@ def _native_ok(dtype, *tensors) -> bool:
                t.device.index == torch.cuda.current_device() for t in tensors)
 
 
+def _torch_stream(stream):
+    """`stream`, which need only have a ``cuda_stream`` handle, as torch's own."""
+    if isinstance(stream, torch.cuda.Stream):
+        return stream
+    return torch.cuda.ExternalStream(stream.cuda_stream)
+
+
 def _order_after(stream):
     """What the current stream does next waits for what `stream` has been given."""
-    if stream is not None and stream != torch.cuda.current_stream():
-        torch.cuda.current_stream().wait_stream(stream)
+    if stream is not None and stream.cuda_stream != torch.cuda.current_stream().cuda_stream:
+        torch.cuda.current_stream().wait_stream(_torch_stream(stream))
 
 
 def _keep_for(stream, *temporaries):
@@ -108,7 +115,7 @@ def _keep_for(stream, *temporaries):
     if stream is not None:
         for t in temporaries:
             if t.numel():
-                t.record_stream(stream)
+                t.record_stream(_torch_stream(stream))
 
 
 def slot_layout(lens, extra: int, stream=None):
@@ -282,7 +289,7 @@ class AlignResult:
         a_len = (self.cap - 2).to(torch.int32)  # slot_cap(cap - 2, 0) == cap
         zeros = torch.zeros_like(a_len)
         if stream is not None:
-            stream.wait_stream(torch.cuda.current_stream())
+            _torch_stream(stream).wait_stream(torch.cuda.current_stream())
         check(lib().poyd_pack_alignments(
             n, self.out.data_ptr(), self.out_off.data_ptr(), a_len.data_ptr(), zeros.data_ptr(),
             self.out_len.data_ptr(), packed.data_ptr(), off.data_ptr(), _stream_handle(stream)))
